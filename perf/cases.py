@@ -128,7 +128,8 @@ def _points(gen, dist, dims, *counts):
     elif dist == "gauss_mix":  # 256 clusters, centres N(0, 1), sigma 0.3
         centres, sigma = torch.randn((256, dims), generator=gen, device=dev), 0.3
     else:                      # a 4-d linear subspace plus noise
-        basis = torch.linalg.qr(torch.randn((dims, 4), generator=gen, device=dev, dtype=torch.float64))[0].float()
+        basis = torch.randn((dims, 4), generator=gen, device=dev, dtype=torch.float64).cpu()
+        basis = torch.linalg.qr(basis)[0].float().to(dev)
         return [torch.randn((n, 4), generator=gen, device=dev) @ basis.T +
                 0.05 * torch.randn((n, dims), generator=gen, device=dev) for n in counts]
     out = []
