@@ -514,11 +514,9 @@ def measure(D, w, key, steps, warmup, plain_steps, world, rank, cpu=True):
     e2e_exact = float((oracle.row_keys(h_i.numpy()[sample], h_d.numpy()[sample]) == want).all(axis=1).mean())
 
     kernel_ms = float(np.median(chosen_kern))
-    kernel_name = {"kd": "kd_knn_kernel", "ball": "ball_knn_kernel", "bf": "bf_knn_kernel"}[w.structure]
-    if tuned_plan["traversal"] == "group":
-        kernel_name = "kd_group_kernel"
-    elif tuned_plan["traversal"] == "box":
-        kernel_name = "kd_box_knn_kernel"
+    kernel_name = {"kd": "kd_warp_query_kernel", "ball": "ball_knn_kernel", "bf": "bf_knn_kernel"}[w.structure]
+    if w.structure == "kd" and tuned_plan["traversal"] == "warp":
+        kernel_name = "kd_knn_warp_kernel"
     if tuned_plan["bf16_filter"]:
         # Tensor-core filter: the MMA work it issues, 2 x 128 queries x 256 rows x (16 per K step,
         # ceil(D/16) steps) per point tile scanned (device counter), against the dense 16-bit peak.

@@ -43,7 +43,7 @@ int query_structure(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaS
 
 namespace {
 
-// mode: 0 per-thread search, 1 warp-coherent, 2 box search (k-d only).
+// mode: 0 per-thread search, 1 warp-coherent, 2 a warp per query over the node boxes (k-d only).
 int batch_launch(int structure, uint32_t dp, const void* sets, uint32_t nsets, uint32_t total_queries,
                  uint32_t total_blocks, uint32_t kmax, uint32_t mode, uint32_t block, uint32_t* counter, uint32_t* keys,
                  uint32_t* vals, bool key_pass, cudaStream_t s) {
@@ -239,10 +239,15 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
             }
             continue;
         }
-        if (c.plan.box) {
-            // The box search reads each index's node boxes: build them now (capture cannot allocate).
-            for (uint32_t i : c.items)
-                if ((rc = knn::kd_box_prepare(items[i].index, s)) != KNN_OK) break;
+        if (c.structure == KNN_KD_TREE && !c.plan.warp) {
+            // A warp per query over each index's node boxes, built now (capture cannot allocate); the
+            // per-thread search where there is no memory for them.
+            c.plan.box = true;
+            for (uint32_t i : c.items) {
+                bool ready = false;
+                if ((rc = knn::kd_boxes_ready(items[i].index, s, &ready)) != KNN_OK) break;
+                c.plan.box = c.plan.box && ready;
+            }
             if (rc != KNN_OK) break;
         }
         const uint32_t block = c.plan.block;
@@ -252,7 +257,9 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
             first_block += knn::ceil_div(items[i].count, block);
         }
         c.total_blocks = first_block;
-        c.sort = (flags & KNN_QF_KEEP_ORDER) == 0;
+        // (A warp per query gains from the locality sort only beyond L2, where one graph of many small
+        // sets is not; the sort's launches would cost more than the searches.)
+        c.sort = (flags & KNN_QF_KEEP_ORDER) == 0 && !c.plan.box;
         uint32_t set_bits = 0;
         while ((1u << set_bits) < c.items.size()) ++set_bits;
         c.key_bits = 24 + set_bits;

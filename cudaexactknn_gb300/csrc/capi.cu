@@ -145,9 +145,28 @@ constexpr float kSeedGrowth = 16.0f;
 int seeded_query(knn_index* ix, const knn::QueryArgs& a, const knn::QueryPlan& plan, cudaStream_t s) {
     // The tensor-core filter tightens each query's bound from its own cell's points before it
     // skips tiles; a seed would only add retries, so it runs unseeded.
-    if (plan.bf16) return dispatch(ix, a, plan, s);
+    if (plan.bf16 || plan.unseeded) return dispatch(ix, a, plan, s);
     const knn::Range range("learned-radius search");
     const size_t n = a.count;
+    if (plan.group && (ix->dp > 16 || a.k > 32))
+        return fail(KNN_ERR_INVALID_ARGUMENT, "group search: dims above 16 or k above 32");
+    bool warp_query = false;
+    if (ix->structure == KNN_KD_TREE && !plan.warp) KNN_TRY(knn::kd_boxes_ready(ix, s, &warp_query));
+    if (warp_query) {
+        // The warp-per-query search starts each query from its seed and, where that held fewer than k
+        // points, searches it again within the caller's radius, all in one launch.  The seeds may be
+        // widened by a factor exp(widen * margin / 2) that the autotuner picks (traversal 2).
+        KNN_TRY(ix->seed_ws.reserve(n * sizeof(float)));
+        float* radii = ix->seed_ws.as<float>();
+        KNN_TRY(knn::model_predict(ix->model.as<float>(), ix->dims, a.queries, a.count, a.max_d2, a.radii, radii,
+                                   nullptr, s, true));
+        knn::QueryArgs seeded = a;
+        seeded.seeds = radii;
+        seeded.seed_scale = std::exp(0.5f * static_cast<float>(plan.widen) * ix->model_margin);
+        knn::QueryPlan p = plan;
+        p.group = false;
+        return dispatch(ix, seeded, p, s);
+    }
     KNN_TRY(ix->seed_ws.reserve(knn::carve_bytes({n * 4, n * 4, 256, knn::retry_scratch_bytes(a.count)})));
     knn::Carver c(ix->seed_ws.ptr);
     float* radii = c.take<float>(n);
@@ -164,18 +183,10 @@ int seeded_query(knn_index* ix, const knn::QueryArgs& a, const knn::QueryPlan& p
     KNN_TRY_CUDA(cudaEventRecord(ix->side.join, ix->side.stream));
     const uint32_t* order = nullptr;
     if (plan.reorder && a.count >= 4096) {
-        // (The group search takes its warps' queries from the order; 16 levels group them as well
-        // as 24 at two radix passes instead of three.)
-        if (ix->structure == KNN_KD_TREE) KNN_TRY(knn::kd_order(ix, a, s, &order, plan.group ? 16u : 24u));
+        if (ix->structure == KNN_KD_TREE) KNN_TRY(knn::kd_order(ix, a, s, &order));
         if (ix->structure == KNN_BALL_TREE) KNN_TRY(knn::ball_order(ix, a, s, &order));
     }
     KNN_TRY_CUDA(cudaStreamWaitEvent(s, ix->side.join, 0));
-    // The warp-group k-d search settles or hands on every query itself (no retry rounds).
-    // Its seeds may be widened by a factor exp(widen * margin / 2) that the autotuner picks: a
-    // miss costs the warp another walk, a wider seed only a few more candidates per query.
-    if (plan.group && ix->structure == KNN_KD_TREE)
-        return knn::kd_group_query(ix, a, plan, order, radii, list, list_count,
-                                   std::exp(0.5f * static_cast<float>(plan.widen) * ix->model_margin), s);
     knn::QueryArgs seeded = a;
     seeded.radii = radii;
     seeded.order = order;
@@ -311,8 +322,7 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
         // The tensor-core filter, for dims >= 16 (the form it is built for), on any structure.
         const bool try_tc = allow_tc && ix->dims >= 16 && knn::tc_supported(ix->dims, a.k);
         if (learned && ix->structure == KNN_KD_TREE && ix->dp <= 16 && a.k <= 32) {
-            // The warp-group search, seeded by the radius model (seeds from each query's own
-            // subtree are too loose to pay).
+            // The warp-per-query search from the radius model's seeds, by bucket size and widening.
             for (uint32_t leaf : {8u, 16u, 32u}) {
                 for (uint32_t widen : {0u, 1u, 2u}) {
                     knn::QueryPlan p;
@@ -326,6 +336,15 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             }
             if (rc != KNN_OK) break;
         }
+        if (learned && ix->structure == KNN_KD_TREE) {
+            // And without them: a warp's search finds a radius nearly as good in its first bucket, so
+            // where the model is not cheap against the search the seeds do not pay for it (4.19 M
+            // clustered 3-d points, 1,048,576 queries: 1.83 ms without, 2.0 with).
+            knn::QueryPlan p;
+            p.block = 128;
+            p.unseeded = true;
+            if ((rc = consider(p)) != KNN_OK) break;
+        }
         if (ix->structure != KNN_BRUTE_FORCE && try_tc) {
             // First, so that slow tree candidates are cut short against its time.
             knn::QueryPlan p;
@@ -333,24 +352,13 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             p.bf16 = true;
             if ((rc = consider(p)) != KNN_OK) break;
         }
-        if (ix->structure == KNN_KD_TREE && ix->dp <= 16) {
-            // The per-thread search over tight node boxes, by bucket size.
-            for (uint32_t leaf : {8u, 16u, 32u}) {
-                knn::QueryPlan p;
-                p.block = 128;
-                p.box = true;
-                p.leaf_scan = leaf;
-                if ((rc = consider(p)) != KNN_OK) break;
-            }
-            if (rc != KNN_OK) break;
-        }
         if (ix->structure != KNN_BRUTE_FORCE) {
             for (bool warp : {false, true}) {
                 for (uint32_t leaf : {0u, 4u, 8u, 16u, 32u, 64u}) {
                     if (leaf && leaf <= ix->leaf_slots) continue;
                     knn::QueryPlan p = best;
                     p.bf16 = false;
-                    p.group = p.box = false;
+                    p.group = p.unseeded = false;
                     p.widen = 0;
                     p.warp = warp;
                     p.leaf_scan = leaf;
@@ -368,15 +376,17 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             }
         }
         const knn::QueryPlan stage2 = best;
+        // Kernels of fixed shape: the filter, and the k-d trees' warp-per-query search.
+        const bool fixed = stage2.bf16 || (ix->structure == KNN_KD_TREE && !stage2.warp);
         for (uint32_t block : {32u, 64u, 256u}) {
-            if (stage2.bf16 || stage2.group || stage2.box) break;  // kernels of fixed shape
+            if (fixed) break;
             knn::QueryPlan p = stage2;
             p.block = block;
             if ((rc = consider(p)) != KNN_OK) break;
         }
         if (rc != KNN_OK) break;
         const knn::QueryPlan stage3 = best;
-        for (int v = 1; v < 8 && !stage3.bf16 && !stage3.group && !stage3.box; ++v) {
+        for (int v = 1; v < 8 && !fixed; ++v) {
             knn::QueryPlan p = stage3;
             p.heap = v & 1;
             p.sh_nn = (v >> 1) & 1;

@@ -20,10 +20,7 @@ int kd_query_dp(knn_index*, const QueryArgs&, const QueryPlan&, cudaStream_t);
 template <uint32_t DP>
 int kd_order_dp(knn_index*, const QueryArgs&, cudaStream_t, const uint32_t**, uint32_t);
 template <uint32_t DP>
-int kd_group_query_dp(knn_index*, const QueryArgs&, const QueryPlan&, const uint32_t*, float*, uint32_t*, uint32_t*,
-                      float, cudaStream_t);
-template <uint32_t DP>
-int kd_box_prepare_dp(knn_index*, cudaStream_t);
+int kd_boxes(knn_index*, cudaStream_t, bool*);
 
 namespace {
 
@@ -147,28 +144,18 @@ int kd_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t
     }
 }
 
-int kd_group_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, const uint32_t* order, float* seeds,
-                   uint32_t* fb_list, uint32_t* fb_count, float seed_scale, cudaStream_t s) {
+int kd_boxes_ready(knn_index* ix, cudaStream_t s, bool* ready) {
     switch (ix->dp) {
-        case 1: return kd_group_query_dp<1>(ix, a, p, order, seeds, fb_list, fb_count, seed_scale, s);
-        case 2: return kd_group_query_dp<2>(ix, a, p, order, seeds, fb_list, fb_count, seed_scale, s);
-        case 3: return kd_group_query_dp<3>(ix, a, p, order, seeds, fb_list, fb_count, seed_scale, s);
-        case 4: return kd_group_query_dp<4>(ix, a, p, order, seeds, fb_list, fb_count, seed_scale, s);
-        case 8: return kd_group_query_dp<8>(ix, a, p, order, seeds, fb_list, fb_count, seed_scale, s);
-        case 16: return kd_group_query_dp<16>(ix, a, p, order, seeds, fb_list, fb_count, seed_scale, s);
-        default: return fail(KNN_ERR_INVALID_ARGUMENT, "group search: dims above 16");
-    }
-}
-
-int kd_box_prepare(knn_index* ix, cudaStream_t s) {
-    switch (ix->dp) {
-        case 1: return kd_box_prepare_dp<1>(ix, s);
-        case 2: return kd_box_prepare_dp<2>(ix, s);
-        case 3: return kd_box_prepare_dp<3>(ix, s);
-        case 4: return kd_box_prepare_dp<4>(ix, s);
-        case 8: return kd_box_prepare_dp<8>(ix, s);
-        case 16: return kd_box_prepare_dp<16>(ix, s);
-        default: return fail(KNN_ERR_INVALID_ARGUMENT, "box search: dims above 16");
+        case 1: return kd_boxes<1>(ix, s, ready);
+        case 2: return kd_boxes<2>(ix, s, ready);
+        case 3: return kd_boxes<3>(ix, s, ready);
+        case 4: return kd_boxes<4>(ix, s, ready);
+        case 8: return kd_boxes<8>(ix, s, ready);
+        case 16: return kd_boxes<16>(ix, s, ready);
+        case 32: return kd_boxes<32>(ix, s, ready);
+        case 64: return kd_boxes<64>(ix, s, ready);
+        case 128: return kd_boxes<128>(ix, s, ready);
+        default: return fail(KNN_ERR_UNSUPPORTED, "dims %u", ix->dims);
     }
 }
 

@@ -10,17 +10,26 @@
 //     fused sum is non-negative), and nodes are pruned only when bound > k-th distance, so no
 //     point whose key could enter the top-k is skipped, ties included;
 //   * k-th key cached in a register; tracker/stack storage chosen by the plan.
+//
+// That per-thread search is what the engine runs where the tight node boxes are not to be had (a
+// query captured into a graph before any query built them, or no memory left for them).  Otherwise
+// each query gets a warp (kd_warp_query_kernel, warp_search.cuh), bounded by the boxes.
 
 #include <algorithm>
 #include <cstring>
 
 #include "tree_query.cuh"
+#include "warp_search.cuh"
 
 #ifndef KNN_DP
 #error "compile with -DKNN_DP=<padded dims>"
 #endif
 
 namespace knn {
+
+constexpr size_t kMaxBlockSmem = 232448;        // most shared memory a block can ask for
+constexpr size_t kL2Bytes = 128u << 20;         // this GPU's L2
+constexpr uint32_t kWarpOrderMin = 1u << 18;    // fewest queries worth an order on an index beyond L2
 
 struct KdParams {
     const float* split;
@@ -35,10 +44,14 @@ struct KdParams {
     uint32_t dims;
     uint32_t nq;
     const uint32_t* order;  // thread -> query, or null
-    const uint32_t* count_dev;
-    uint32_t order_base;  // subtracted from order entries (batched orders hold batch-wide ids)  // when set, *count_dev threads are live (nq is an upper bound)
+    const uint32_t* count_dev;  // when set, *count_dev threads are live (nq is an upper bound)
+    uint32_t order_base;  // subtracted from order entries (batched orders hold batch-wide ids)
     float max_d2;
     const float* radii;
+    const float* box;     // tight node boxes (warp-per-query search), per node lo[], hi[]
+    uint32_t box_stride;  // floats per box
+    const float* seeds;   // warp-per-query search: per query radius to start from (x seed_scale), or null
+    float seed_scale;
     uint32_t k;
     int32_t* out_idx;
     float* out_dist;
@@ -220,21 +233,15 @@ __global__ void kd_leaf_key_kernel(const float* __restrict__ split, uint32_t aux
     vals[t] = t;
 }
 
-template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
-static int launch_kd(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
-                     cudaStream_t s) {
-    const uint32_t block = plan.block ? plan.block : 128;
-    const size_t smem = tracker_smem_bytes(SHNN, KMAX, block) + stack_smem_bytes(SHST, block);
-    auto kern = plan.warp ? kd_knn_warp_kernel<DP, KMAX, HEAP, SHNN, SHST> : kd_knn_kernel<DP, KMAX, HEAP, SHNN, SHST>;
-    if (smem > 48 * 1024)
-        KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+// A query batch's search parameters: its tree, buckets of `bucket` slots (0 = the tree's leaves).
+inline KdParams kd_params(const knn_index* ix, const QueryArgs& a, const uint32_t* order, uint32_t bucket) {
     KdParams p{};
     p.split = ix->split.as<float>();
     p.leaf = ix->leaf.as<float>();
     p.leaf_stride = ix->leaf_stride;
     p.node_count = ix->node_count;
     p.node_depth = ix->node_depth;
-    p.stop_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, plan.leaf_scan);
+    p.stop_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, bucket);
     p.leaf_slots = ix->leaf_slots;
     p.aux = ix->aux_dims;
     p.queries = a.queries;
@@ -244,10 +251,33 @@ static int launch_kd(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, c
     p.count_dev = a.count_dev;
     p.max_d2 = a.max_d2;
     p.radii = a.radii;
+    p.seeds = a.seeds;
+    p.seed_scale = a.seed_scale;
     p.k = a.k;
     p.out_idx = a.out_idx;
     p.out_dist = a.out_dist;
     p.counters = a.counters;
+    return p;
+}
+
+// The same for a search over the node boxes.
+inline KdParams kd_box_params(const knn_index* ix, const QueryArgs& a, const uint32_t* order, uint32_t bucket) {
+    KdParams p = kd_params(ix, a, order, bucket);
+    p.stop_depth = std::min(p.stop_depth, ix->kd_box_depth);
+    p.box = ix->kd_box.as<float>();
+    p.box_stride = ix->kd_box_stride;
+    return p;
+}
+
+template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
+static int launch_kd(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
+                     cudaStream_t s) {
+    const uint32_t block = plan.block ? plan.block : 128;
+    const size_t smem = tracker_smem_bytes(SHNN, KMAX, block) + stack_smem_bytes(SHST, block);
+    auto kern = plan.warp ? kd_knn_warp_kernel<DP, KMAX, HEAP, SHNN, SHST> : kd_knn_kernel<DP, KMAX, HEAP, SHNN, SHST>;
+    if (smem > 48 * 1024)
+        KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    const KdParams p = kd_params(ix, a, order, plan.leaf_scan);
     if (plan.timing) KNN_TRY(ix->timing.begin(s));
     kern<<<ceil_div(a.count, block), block, smem, s>>>(p);
     KNN_LAUNCHED();
@@ -300,18 +330,37 @@ int kd_order_dp(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_
 }
 
 template <uint32_t DP>
-int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
-                      float* seeds, uint32_t* fb_list, uint32_t* fb_count, float seed_scale, cudaStream_t s);
+int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s);
 
 template <uint32_t DP>
-int kd_box_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s);
+int kd_boxes(knn_index* ix, cudaStream_t s, bool* ready);
+
+template <uint32_t DP>
+int kd_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s);
 
 template <uint32_t DP>
 int kd_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s) {
+    if (p.box && DP > 16) return fail(KNN_ERR_INVALID_ARGUMENT, "box search: dims above 16");
     const uint32_t* order = a.order;
+    if (!p.warp && !(p.group && !a.count_dev)) {
+        // A warp per query, where its node boxes are at hand.  The per-thread search's storage options
+        // do not matter to it, but sizes that search refuses stay refused (by the launch below).
+        const uint32_t block = p.block ? p.block : 128;
+        const bool fits = tracker_smem_bytes(p.sh_nn, k_class(a.k), block) + stack_smem_bytes(p.sh_stack, block) <= kMaxBlockSmem;
+        bool ready = false;
+        if (fits || p.box) KNN_TRY(kd_boxes<DP>(ix, s, &ready));
+        if (ready) {
+            // Neighbouring queries share the boxes and slots they read only through the caches: an
+            // order pays once the index outgrows L2 (16 M clustered 3-d points, 2 M queries: 3.74 ms
+            // sorted, 3.96 unsorted; 40 M and 4 M: 7.59 and 8.48) and costs before (4.19 M and 1 M:
+            // 1.92 and 1.83).
+            if (!order && p.reorder && a.count >= kWarpOrderMin && ix->leaf.bytes > kL2Bytes)
+                KNN_TRY(kd_order_dp<DP>(ix, a, s, &order, 24));
+            return kd_warp_query_dp<DP>(ix, a, p, order, s);
+        }
+    }
     if (!order && p.reorder && a.count >= 4096) KNN_TRY(kd_order_dp<DP>(ix, a, s, &order, 24));
-    if (p.group && !a.count_dev) return kd_group_query_dp<DP>(ix, a, p, order, nullptr, nullptr, nullptr, 1.0f, s);
-    if (p.box) return kd_box_query_dp<DP>(ix, a, p, order, s);
+    if (p.group && !a.count_dev) return kd_group_query_dp<DP>(ix, a, p, order, s);
     switch (k_class(a.k)) {
         case 8: return launch_kd_variant<DP, 8>(ix, a, p, order, s);
         case 16: return launch_kd_variant<DP, 16>(ix, a, p, order, s);
@@ -333,15 +382,14 @@ int kd_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStrea
 // query's radius is appended to that query's candidate list in shared memory; at the end each
 // lane sorts its query's list.  A query with fewer than k candidates inside a radius below the
 // caller's grows its radius by the density it saw and walks again; one whose list overflows, or
-// that is still short after a few rounds, goes to a list that the box-bounded per-thread search
-// answers.  Every
+// that is still short after a few rounds, goes to a list that the warp-per-query search answers.  Every
 // answer is exact: a bucket is skipped only when its box bound exceeds the radius, and the box
 // bound is a rigorous lower bound on the float distance of every point inside (below).
 constexpr uint32_t kGroupWarps = 4;
 constexpr uint32_t kGroupList = 64;   // bucket entries collected before they are scanned
 constexpr uint32_t kGroupFan = 3;     // levels the walk descends per step (up to 8 boxes tested at once)
 constexpr uint32_t kGroupStack = 96;  // node stack (at most 7 net entries per step, 11 steps deep)
-constexpr uint32_t kGroupRounds = 6;  // radius growth rounds before the per-thread fallback
+constexpr uint32_t kGroupRounds = 6;  // radius growth rounds before a query is left over
 
 __host__ __device__ constexpr uint32_t group_cap(int kmax) { return kmax <= 8 ? 32u : (kmax <= 16 ? 48u : 80u); }
 __host__ __device__ constexpr int box_qs(int dp) { return dp < 4 ? 4 : dp; }
@@ -362,13 +410,10 @@ constexpr size_t group_smem_bytes() { return kGroupWarps * sizeof(GroupWarpSmem<
 
 struct KdGroupParams {
     KdParams p;              // tree, queries, locality order, caller's radius (max_d2 / radii), outputs
-    const float* box;        // per node (depth <= box depth): lo[box_qs(DP)], hi[box_qs(DP)]
-    float* seeds;            // per query radius to start from (<= the caller's); fallback radius on exit
-    uint32_t* fb_list;       // queries left to the per-thread search
+    float* seeds;            // per query radius to start from (<= the caller's); leftover's radius on exit
+    uint32_t* fb_list;       // queries left to the warp-per-query search
     uint32_t* fb_count;
     uint32_t* group_counter; // next group of 32 queries (zero before the launch)
-    uint32_t box_stride;     // floats per box
-    float seed_scale;        // seeds are multiplied by this (capped by the caller's radius)
 };
 
 // Lower bound on the float dist2 from q to any point of the box (lo, hi): per dimension the gap
@@ -377,11 +422,8 @@ struct KdGroupParams {
 // fma(t, t, acc) is non-decreasing in |t| and acc >= 0, so the bound never exceeds dist2(q, p).
 // An empty box (lo = +inf, hi = -inf) gives +inf.
 template <int DP>
-__device__ __forceinline__ float box_bound(const float (&q)[DP], const float* __restrict__ box) {
-    constexpr int QS = box_qs(DP);
-    const float4* lo4 = reinterpret_cast<const float4*>(box);
-    const float4* hi4 = reinterpret_cast<const float4*>(box + QS);
-    float acc = 0.0f;
+__device__ __forceinline__ float box_bound(const float (&q)[DP], const float4* __restrict__ lo4,
+                                           const float4* __restrict__ hi4, float acc) {
 #pragma unroll
     for (int v = 0; v < (DP + 3) / 4; ++v) {
         const float4 lo = __ldg(lo4 + v), hi = __ldg(hi4 + v);
@@ -396,6 +438,11 @@ __device__ __forceinline__ float box_bound(const float (&q)[DP], const float* __
         }
     }
     return acc;
+}
+
+template <int DP>
+__device__ __forceinline__ float box_bound(const float (&q)[DP], const float* __restrict__ box) {
+    return box_bound<DP>(q, reinterpret_cast<const float4*>(box), reinterpret_cast<const float4*>(box + box_qs(DP)), 0.0f);
 }
 
 template <int DP, int KMAX>
@@ -427,7 +474,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGrou
 #pragma unroll
         for (int d = 0; d < QS; ++d) sm.qv[lane][d] = d < DP ? q[d] : 0.0f;
         const float R = active ? (p.radii ? p.radii[qi] : p.max_d2) : -1.0f;
-        float r = active ? gp.seeds[qi] * gp.seed_scale : -1.0f;
+        float r = active ? gp.seeds[qi] : -1.0f;
         if (!(r <= R)) r = R;  // a seed above the caller's radius (or NaN) starts at the caller's
         bool pending = active;
 
@@ -487,7 +534,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGrou
             sm.rad[lane] = rl;
             __syncwarp();
             uint32_t top = 0, nlist = 0;
-            const uint32_t m0 = __ballot_sync(FULL, box_bound<DP>(q, gp.box) <= rl);
+            const uint32_t m0 = __ballot_sync(FULL, box_bound<DP>(q, p.box) <= rl);
             if (m0) {
                 if (stop == 0) {
                     if (lane == 0) sm.list[0] = m0;
@@ -509,7 +556,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGrou
 #pragma unroll
                 for (uint32_t j = 0; j < (1u << kGroupFan); ++j) {
                     // (j < fan first: with an unbounded radius an infinite bound is still "within".)
-                    const bool in = j < fan && box_bound<DP>(q, gp.box + static_cast<size_t>(first + j) * gp.box_stride) <= rl;
+                    const bool in = j < fan && box_bound<DP>(q, p.box + static_cast<size_t>(first + j) * p.box_stride) <= rl;
                     want[j] = __ballot_sync(FULL, in);
                 }
                 ++nodes;
@@ -568,8 +615,8 @@ __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGrou
                 };
                 if (c > C) {
                     // More candidates than the list holds.  The k-th smallest distance among the C
-                    // kept bounds the k-th neighbour's (k real points lie within it): the
-                    // per-thread search starts from it.  (Walking again with a radius shrunk by the
+                    // kept bounds the k-th neighbour's (k real points lie within it): its
+                    // own search starts from it.  (Walking again with a radius shrunk by the
                     // density was tried: the extra rounds cost more than the searches they save.)
                     Tracker<KMAX, false, false> tr;
                     tr.init(p.k, r, nullptr, 0);
@@ -616,214 +663,106 @@ __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGrou
     }
 }
 
-// Per-thread search over the tight node boxes (traversal 3, and the group search's leftovers):
-// depth first, the closer child first, a node skipped when its box bound exceeds the current k-th
-// distance, buckets at depth `stop` scanned whole; from radius r2, results to the query's row.
-// Box bounds matter most far from the data, where a single splitting plane prunes little.
-template <int DP, int KMAX>
-__device__ __forceinline__ void kd_box_search(const KdParams& p, const float* __restrict__ box, uint32_t box_stride,
-                                              uint32_t stop, uint32_t qi, float r2) {
-    float q[DP];
-    load_query<DP>(p.queries, p.dims, qi, q);
-    Tracker<KMAX, false, false> tr;
-    tr.init(p.k, r2, nullptr, 0);
-    Stack<false> st;
-    st.init(nullptr, 0);
-    st.push(0, box_bound<DP>(q, box));
-    bool overflow = false;
-    LocalCounters lc;
-    while (st.top) {
-        uint32_t node;
-        float bound;
-        st.pop(&node, &bound);
-        if (bound > tr.radius()) continue;
-        if (heap_depth(node) == stop) {
-            const SlotRange sr = subtree_slots(node, stop, p.node_depth, p.node_count, p.leaf_slots);
-            const float* slot = p.leaf + sr.first * p.leaf_stride;
-            ++lc.leaves;
-            for (uint32_t s = 0; s < sr.count; ++s, slot += p.leaf_stride) {
-                int32_t id;
-                const float d2 = slot_dist<DP>(q, slot, &id);
-                if (id < 0) continue;
-                ++lc.points;
-                tr.offer(make_key(d2, id));
+// One query per warp (warp_search.cuh) against the tight node boxes: the default search, and the
+// group search's leftovers.  1,048,576 queries, k 16, on 4.19 M clustered 3-d points: 1.83 ms, 8.5
+// boxes of 32 tested and 7.5 buckets of 32 slots scanned per query; a thread per query took 3.2 ms
+// over the same boxes and 38 to 60 ms with splitting planes only (their bound prunes little in the
+// space between clusters).  10,000 uniform 11-d queries within a radius on 500,000 points: 2.0 ms
+// (28 and 145 ms).  Bound by the instructions of the top-k insertions and box tests at C2's shape,
+// by L2 reads of boxes and slots in more dimensions.
+template <int DP>
+struct KdWarpView {
+    static constexpr bool kKeys = false;      // the nearest box first
+    static constexpr bool kShared = DP > 32;  // wide queries are read from shared memory (broadcast)
+    float q[kShared ? 1 : DP];
+    const float4* sq;
+    const float* box;
+    uint32_t box_stride;
+    __device__ __forceinline__ void test(uint32_t node, float* bound, uint32_t*) const {
+        const float* b = box + static_cast<size_t>(node) * box_stride;
+        if constexpr (kShared) {
+            const float4* lo4 = reinterpret_cast<const float4*>(b);
+            const float4* hi4 = reinterpret_cast<const float4*>(b + DP);
+            float acc = 0.0f;
+#pragma unroll 4
+            for (int v = 0; v < DP / 4; ++v) {
+                const float4 a = sq[v];
+                const float qq[4] = {a.x, a.y, a.z, a.w};
+                acc = box_bound<4>(qq, lo4 + v, hi4 + v, acc);
             }
-            continue;
+            *bound = acc;
+        } else {
+            *bound = box_bound<DP>(q, b);
         }
-        ++lc.nodes;
-        const uint32_t l = 2 * node + 1;
-        const float bl = box_bound<DP>(q, box + static_cast<size_t>(l) * box_stride);
-        const float br = box_bound<DP>(q, box + static_cast<size_t>(l + 1) * box_stride);
-        const bool left_first = bl <= br;  // pushed last, popped first
-        const uint32_t far_node = left_first ? l + 1 : l, near_node = left_first ? l : l + 1;
-        const float far_b = left_first ? br : bl, near_b = left_first ? bl : br;
-        if (far_b <= tr.radius()) overflow |= !st.push(far_node, far_b);
-        if (near_b <= tr.radius()) overflow |= !st.push(near_node, near_b);
     }
-    tr.emit(p.k, p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
-    if (p.counters) {
-        lc.flush(p.counters);
-        if (overflow) atomicExch(&p.counters->error, 1);
+    __device__ __forceinline__ float dist(const float* slot, int32_t* id) const {
+        if constexpr (kShared) {
+            *id = __float_as_int(slot[DP]);
+            return dist2_shared<DP>(sq, reinterpret_cast<const float4*>(slot));
+        } else {
+            return slot_dist<DP>(q, slot, id);
+        }
     }
-}
-
-// The group search's leftovers, from each one's radius in `seeds`: one query per warp (lane 0),
-// warps striding over the list.  The leftovers lie scattered in space, so 32 of them in one warp
-// would take 32 different paths one after another; a warp each runs them side by side.
-template <int DP, int KMAX>
-__global__ void __launch_bounds__(128) kd_fallback_kernel(const KdGroupParams gp) {
-    if ((threadIdx.x & 31u) != 0) return;
-    const uint32_t n = *gp.fb_count;
-    const uint32_t warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t t = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; t < n; t += warps) {
-        const uint32_t qi = gp.fb_list[t];
-        kd_box_search<DP, KMAX>(gp.p, gp.box, gp.box_stride, gp.p.stop_depth, qi, gp.seeds[qi]);
-    }
-}
-
-// ---- one query per warp: the group search's leftovers -----------------------------------------
-// The leftovers are mostly queries far from the data (their k-th distance is large and the ball
-// brushes many buckets of a dense cluster) or queries whose seed held far more points than a
-// list: searched by one thread each they took up to ~0.6 ms apiece and set the length of the
-// whole pass.  Here a warp searches one of them: each step tests the up-to-32 descendants five
-// levels below a node, one per lane (the box bound against the current k-th distance), scans the
-// wanted buckets one per lane, and merges the candidates into a top-32 held across the warp
-// (lane i the i-th smallest key) by bitonic sorting networks over shuffles.  Exact as the other
-// searches: a subtree is skipped only when its box bound exceeds the current k-th distance.
-constexpr uint32_t kSoloFan = 5;     // levels per step: up to 32 descendants, one per lane
-constexpr uint32_t kSoloStack = 256; // at most 31 net entries per step, 7 steps deep
-constexpr uint32_t kSoloCand = 1024; // candidates of one step: 32 buckets of at most 32 slots
-
-struct SoloWarpSmem {
-    uint64_t cand[kSoloCand];
-    uint32_t stack[kSoloStack];
-    uint32_t ncand;
 };
 
-__device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, uint32_t m) {
-    const uint32_t lo = __shfl_xor_sync(0xFFFFFFFFu, static_cast<uint32_t>(v), m);
-    const uint32_t hi = __shfl_xor_sync(0xFFFFFFFFu, static_cast<uint32_t>(v >> 32), m);
-    return (static_cast<uint64_t>(hi) << 32) | lo;
-}
+constexpr uint32_t kWarpsPerBlock = 4;
 
-__device__ __forceinline__ uint64_t shfl64(uint64_t v, uint32_t src) {
-    const uint32_t lo = __shfl_sync(0xFFFFFFFFu, static_cast<uint32_t>(v), src);
-    const uint32_t hi = __shfl_sync(0xFFFFFFFFu, static_cast<uint32_t>(v >> 32), src);
-    return (static_cast<uint64_t>(hi) << 32) | lo;
-}
+template <int DP>
+struct KdWarpSmem {
+    WarpRows<false> rows;
+    float4 q[DP > 32 ? DP / 4 : 1];
+};
 
-// Ascending bitonic sort of 32 keys, one per lane.
-__device__ __forceinline__ uint64_t warp_sort64(uint64_t v, uint32_t lane) {
-#pragma unroll
-    for (uint32_t k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            const uint64_t o = shfl_xor64(v, j);
-            const bool up = (lane & k) == 0, lower = (lane & j) == 0;
-            v = (lower == up) ? (v < o ? v : o) : (v < o ? o : v);
-        }
-    }
-    return v;
-}
-
-// The 32 smallest of two ascending 32-key sequences (one key per lane each), ascending.
-__device__ __forceinline__ uint64_t warp_merge_low64(uint64_t a, uint64_t b, uint32_t lane) {
-    const uint64_t rb = shfl64(b, 31 - lane);
-    uint64_t v = a < rb ? a : rb;  // a bitonic sequence holding the 32 smallest
-#pragma unroll
-    for (uint32_t j = 16; j > 0; j >>= 1) {
-        const uint64_t o = shfl_xor64(v, j);
-        v = (lane & j) == 0 ? (v < o ? v : o) : (v < o ? o : v);
-    }
-    return v;
-}
-
-template <int DP, int KMAX>
-__global__ void __launch_bounds__(128) kd_solo_kernel(const KdGroupParams gp) {
-    static_assert(KMAX <= 32, "the top-k is held one key per lane");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SoloWarpSmem& sm = reinterpret_cast<SoloWarpSmem*>(smem_raw)[threadIdx.x >> 5];
-    const KdParams& p = gp.p;
+// One warp's search of query qi within r2; its row goes to the query's result slots.
+template <int DP, int KR, bool SEEDED>
+__device__ __forceinline__ void kd_warp_query(const KdParams& p, uint32_t qi, float r2, KdWarpSmem<DP>& sm) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t stop = p.stop_depth;
-    const uint32_t n = *gp.fb_count;
-    const uint32_t warps = gridDim.x * (blockDim.x / 32);
-    LocalCounters lc;
-    bool stack_error = false;
-    for (uint32_t t = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; t < n; t += warps) {
-        const uint32_t qi = gp.fb_list[t];
-        float q[DP];
-        load_query<DP>(p.queries, p.dims, qi, q);
-        const float r2 = gp.seeds[qi];
-        uint64_t top = make_key(r2, -1);  // lane i: the i-th smallest key so far
-        float kth = r2;
-        if (lane == 0) sm.stack[0] = 0;
-        uint32_t depth_n = 1;  // stack entries
-        while (depth_n) {
-            __syncwarp();
-            const uint32_t node = sm.stack[--depth_n];
-            const uint32_t levels = min(kSoloFan, stop - heap_depth(node));
-            const uint32_t fan = 1u << levels;
-            const uint32_t first = ((node + 1) << levels) - 1;
-            const bool want =
-                lane < fan && box_bound<DP>(q, gp.box + static_cast<size_t>(first + lane) * gp.box_stride) <= kth;
-            const uint32_t wm = __ballot_sync(0xFFFFFFFFu, want);
-            if (heap_depth(node) + levels == stop) {
-                if (lane == 0) sm.ncand = 0;
-                __syncwarp();
-                if (want) {
-                    const SlotRange sr = subtree_slots(first + lane, stop, p.node_depth, p.node_count, p.leaf_slots);
-                    const float* slot = p.leaf + sr.first * p.leaf_stride;
-                    ++lc.leaves;
-                    for (uint32_t s = 0; s < sr.count; ++s, slot += p.leaf_stride) {
-                        int32_t id;
-                        const float d2 = slot_dist<DP>(q, slot, &id);
-                        if (id < 0) continue;
-                        ++lc.points;
-                        if (d2 <= kth) {
-                            const uint32_t pos = atomicAdd(&sm.ncand, 1u);
-                            if (pos < kSoloCand) sm.cand[pos] = make_key(d2, id);
-                        }
-                    }
-                }
-                __syncwarp();
-                const uint32_t nc = min(sm.ncand, kSoloCand);  // at most 32 buckets of <= 32 slots
-                for (uint32_t base = 0; base < nc; base += 32) {
-                    const uint64_t x = base + lane < nc ? sm.cand[base + lane] : ~0ull;
-                    top = warp_merge_low64(top, warp_sort64(x, lane), lane);
-                }
-                kth = key_dist(shfl64(top, p.k - 1));
-            } else {
-                ++lc.nodes;
-                const uint32_t cnt = __popc(wm);
-                if (depth_n + cnt > kSoloStack) {  // cannot happen (see kSoloStack); recorded
-                    stack_error = true;
-                    continue;
-                }
-                // The lowest-numbered descendant ends on top (popped first).
-                if (want) sm.stack[depth_n + cnt - 1 - __popc(wm & ((1u << lane) - 1u))] = first + lane;
-                depth_n += cnt;
-            }
-        }
-        if (lane < p.k) {
-            p.out_idx[static_cast<size_t>(qi) * p.k + lane] = key_index(top);
-            p.out_dist[static_cast<size_t>(qi) * p.k + lane] = key_dist(top);
-        }
+    KdWarpView<DP> view;
+    if constexpr (DP > 32) {
+        stage_query<DP>(p.queries, p.dims, qi, lane, sm.q);
+        view.sq = sm.q;
+    } else {
+        load_query<DP>(p.queries, p.dims, qi, view.q);
     }
-    if (p.counters) {
+    view.box = p.box;
+    view.box_stride = p.box_stride;
+    const WarpTree t{p.leaf, p.leaf_stride, p.leaf_slots << (p.node_depth - p.stop_depth), p.stop_depth};
+    WarpTopK<KR> top;
+    LocalCounters lc;
+    bool missed = false;
+    top.init(p.k, r2, lane);
+    if constexpr (SEEDED) {
+        const float r = p.seeds[qi] * p.seed_scale;
+        missed = warp_search<KdWarpView<DP>, KR, true>(view, t, sm.rows, top, lc, r < r2 ? r : r2, r2);
+    } else {
+        warp_search<KdWarpView<DP>, KR, false>(view, t, sm.rows, top, lc, r2, r2);
+    }
+    top.emit(p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
+    if (p.counters && lane == 0) {
         lc.flush(p.counters);
-        if (stack_error) atomicExch(&p.counters->error, 1);
+        if (missed) atomicAdd(&p.counters->fallback, 1ull);
     }
 }
 
-// Traversal 3: one box-bounded search per thread, in the batch's locality order.
-template <int DP, int KMAX>
-__global__ void __launch_bounds__(128) kd_box_knn_kernel(const KdParams p, const float* __restrict__ box,
-                                                         uint32_t box_stride) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (p.count_dev ? *p.count_dev : p.nq)) return;
-    const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
-    kd_box_search<DP, KMAX>(p, box, box_stride, p.stop_depth, qi, p.radii ? p.radii[qi] : p.max_d2);
+template <int DP, int KR, bool SEEDED>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) kd_warp_query_kernel(const KdParams p) {
+    __shared__ KdWarpSmem<DP> sm[kWarpsPerBlock];
+    const uint32_t w = threadIdx.x >> 5, t = blockIdx.x * kWarpsPerBlock + w;
+    if (t >= (p.count_dev ? *p.count_dev : p.nq)) return;  // no block-wide barriers
+    const uint32_t qi = p.order ? p.order[t] : t;
+    kd_warp_query<DP, KR, SEEDED>(p, qi, p.radii ? p.radii[qi] : p.max_d2, sm[w]);
+}
+
+// The group search's leftovers, each within its radius in `seeds`; warps stride over the list.
+template <int DP>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) kd_leftover_kernel(const KdGroupParams gp) {
+    __shared__ KdWarpSmem<DP> sm[kWarpsPerBlock];
+    const uint32_t w = threadIdx.x >> 5, n = *gp.fb_count;
+    for (uint32_t t = blockIdx.x * kWarpsPerBlock + w; t < n; t += gridDim.x * kWarpsPerBlock) {
+        const uint32_t qi = gp.fb_list[t];
+        kd_warp_query<DP, 1, false>(gp.p, qi, gp.seeds[qi], sm[w]);
+        __syncwarp();
+    }
 }
 
 // Self seeds: each query's k-th distance among the points of the subtree of at least
@@ -888,82 +827,81 @@ __global__ void kd_box_bottom_kernel(const float* __restrict__ leaf, uint32_t le
     }
 }
 
+// Nodes whose boxes one block of kd_box_up_kernel folds (a power of two; 32 KB of shared memory at most).
+constexpr uint32_t box_up_nodes(uint32_t qs) { return qs <= 16 ? 256u : 4096u / qs; }
+
+// Boxes of up to log2(T) levels above `depth`: a block loads the boxes of T neighbouring nodes there
+// and folds them pairwise in shared memory (one launch instead of one per level, whose tiny grids
+// near the root each cost a launch).
 template <int QS>
-__global__ void kd_box_up_kernel(float* __restrict__ box, uint32_t depth) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (1u << depth)) return;
-    const uint32_t node = (1u << depth) - 1u + i;
-    const float* a = box + static_cast<size_t>(2 * node + 1) * (2 * QS);
-    const float* b = a + 2 * QS;
-    float* out = box + static_cast<size_t>(node) * (2 * QS);
-#pragma unroll
-    for (int d = 0; d < QS; ++d) {
-        out[d] = fminf(a[d], b[d]);
-        out[QS + d] = fmaxf(a[QS + d], b[QS + d]);
+__global__ void kd_box_up_kernel(float* __restrict__ box, uint32_t depth, uint32_t levels) {
+    constexpr uint32_t T = box_up_nodes(QS);
+    __shared__ float sb[T][2 * QS];
+    const uint32_t t = threadIdx.x, first = blockIdx.x * T;
+    uint32_t nodes = min(T, (1u << depth) - first);
+    if (t < nodes) {
+        const float* in = box + ((1u << depth) - 1u + first + t) * static_cast<size_t>(2 * QS);
+#pragma unroll 8
+        for (int d = 0; d < 2 * QS; ++d) sb[t][d] = in[d];
+    }
+    for (uint32_t l = 1; l <= levels; ++l) {
+        nodes >>= 1;
+        for (int d = 0; d < QS; ++d) {
+            __syncthreads();
+            float lo = 0.0f, hi = 0.0f;
+            if (t < nodes) {
+                lo = fminf(sb[2 * t][d], sb[2 * t + 1][d]);
+                hi = fmaxf(sb[2 * t][QS + d], sb[2 * t + 1][QS + d]);
+            }
+            __syncthreads();
+            if (t < nodes) {
+                sb[t][d] = lo;
+                sb[t][QS + d] = hi;
+                float* out = box + ((1u << (depth - l)) - 1u + (first >> l) + t) * static_cast<size_t>(2 * QS);
+                out[d] = lo;
+                out[QS + d] = hi;
+            }
+        }
     }
 }
 
 template <uint32_t DP>
 int kd_box_build_dp(knn_index* ix, cudaStream_t s) {
-    constexpr uint32_t QS = box_qs(DP);
-    const uint32_t depth = ix->kd_box_depth;
+    constexpr uint32_t QS = box_qs(DP), T = box_up_nodes(QS);
+    uint32_t depth = ix->kd_box_depth;
     const size_t nodes = (static_cast<size_t>(2) << depth) - 1;
     ix->kd_box_stride = 2 * QS;
     KNN_TRY(ix->kd_box.alloc(nodes * ix->kd_box_stride * sizeof(float)));
-    kd_box_bottom_kernel<DP><<<ceil_div(1u << depth, 256), 256, 0, s>>>(
+    kd_box_bottom_kernel<DP><<<ceil_div(1u << depth, 128), 128, 0, s>>>(
         ix->leaf.as<float>(), ix->leaf_stride, depth, ix->node_depth, ix->node_count, ix->leaf_slots,
         ix->kd_box.as<float>(), ix->kd_box_stride);
     KNN_LAUNCHED();
-    for (uint32_t d = depth; d-- > 0;) {
-        kd_box_up_kernel<QS><<<ceil_div(1u << d, 256), 256, 0, s>>>(ix->kd_box.as<float>(), d);
+    while (depth) {
+        uint32_t levels = 0;
+        while (levels < depth && (2u << levels) <= T) ++levels;
+        kd_box_up_kernel<QS><<<ceil_div(1u << depth, T), T, 0, s>>>(ix->kd_box.as<float>(), depth, levels);
         KNN_LAUNCHED();
+        depth -= levels;
     }
     return KNN_OK;
 }
 
-inline uint32_t bucket_slots_of(const KdParams& p) { return p.leaf_slots << (p.node_depth - p.stop_depth); }
-
 template <int DP, int KMAX>
 static int launch_kd_group(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
-                           float* seeds, bool self_seed, uint32_t* fb_list, uint32_t* fb_count, float seed_scale,
-                           cudaStream_t s) {
+                           float* seeds, uint32_t* fb_list, uint32_t* fb_count, cudaStream_t s) {
     KdGroupParams gp{};
-    KdParams& p = gp.p;
-    p.split = ix->split.as<float>();
-    p.leaf = ix->leaf.as<float>();
-    p.leaf_stride = ix->leaf_stride;
-    p.node_count = ix->node_count;
-    p.node_depth = ix->node_depth;
-    p.stop_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, plan.leaf_scan ? plan.leaf_scan : 8u);
-    if (p.stop_depth > ix->kd_box_depth) p.stop_depth = ix->kd_box_depth;
-    p.leaf_slots = ix->leaf_slots;
-    p.aux = ix->aux_dims;
-    p.queries = a.queries;
-    p.dims = ix->dims;
-    p.nq = a.count;
-    p.order = order;
-    p.max_d2 = a.max_d2;
-    p.radii = a.radii;
-    p.k = a.k;
-    p.out_idx = a.out_idx;
-    p.out_dist = a.out_dist;
-    p.counters = a.counters;
-    gp.box = ix->kd_box.as<float>();
-    gp.box_stride = ix->kd_box_stride;
+    gp.p = kd_box_params(ix, a, order, plan.leaf_scan ? plan.leaf_scan : 8u);
     gp.seeds = seeds;
-    gp.seed_scale = seed_scale;
     gp.fb_list = fb_list;
     gp.fb_count = fb_count;
     gp.group_counter = fb_count + 1;  // the count's scratch slot holds 256 bytes
     KNN_TRY_CUDA(cudaMemsetAsync(fb_count, 0, 2 * sizeof(uint32_t), s));
-    if (self_seed) {
-        // Subtree of at least max(4k, 32) slots.
-        const uint32_t want = std::max<uint32_t>(32u, 4u * a.k);
-        uint32_t sd = ix->node_depth;
-        while (sd > 0 && (static_cast<uint64_t>(ix->leaf_slots) << (ix->node_depth - sd)) < want) --sd;
-        kd_self_seed_kernel<DP, KMAX><<<ceil_div(a.count, 128), 128, 0, s>>>(p, sd, seeds);
-        KNN_LAUNCHED();
-    }
+    // Self seeds from a subtree of at least max(4k, 32) slots.
+    const uint32_t want = std::max<uint32_t>(32u, 4u * a.k);
+    uint32_t sd = ix->node_depth;
+    while (sd > 0 && (static_cast<uint64_t>(ix->leaf_slots) << (ix->node_depth - sd)) < want) --sd;
+    kd_self_seed_kernel<DP, KMAX><<<ceil_div(a.count, 128), 128, 0, s>>>(gp.p, sd, seeds);
+    KNN_LAUNCHED();
     constexpr size_t smem = group_smem_bytes<DP, KMAX>();
     auto kern = kd_group_kernel<DP, KMAX>;
     KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
@@ -974,110 +912,81 @@ static int launch_kd_group(knn_index* ix, const QueryArgs& a, const QueryPlan& p
                                              static_cast<uint32_t>(std::max(per_sm, 1) * sm_count()));
     kern<<<grid, 32 * kGroupWarps, smem, s>>>(gp);
     KNN_LAUNCHED();
-    if (bucket_slots_of(p) <= 32) {
-        constexpr size_t solo_smem = 4 * sizeof(SoloWarpSmem);
-        KNN_TRY_CUDA(cudaFuncSetAttribute(kd_solo_kernel<DP, KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(solo_smem)));
-        kd_solo_kernel<DP, KMAX><<<8 * static_cast<uint32_t>(sm_count()), 128, solo_smem, s>>>(gp);
-    } else {
-        kd_fallback_kernel<DP, KMAX><<<8 * static_cast<uint32_t>(sm_count()), 128, 0, s>>>(gp);
-    }
+    kd_leftover_kernel<DP><<<8 * static_cast<uint32_t>(sm_count()), 32 * kWarpsPerBlock, 0, s>>>(gp);
     KNN_LAUNCHED();
     if (plan.timing) KNN_TRY(ix->timing.end(s));
     return KNN_OK;
 }
 
-template <uint32_t DP>
-int kd_box_prepare_dp(knn_index* ix, cudaStream_t s);
-
-// Builds the node boxes on first use (down to subtrees of at most 4 slots).
+// Builds the node boxes on first use, down to subtrees of at most 4 slots (16 slots beyond 16 dims,
+// where a box is as large as several slots).
 template <uint32_t DP>
 int kd_box_ensure(knn_index* ix, cudaStream_t s) {
     if (ix->kd_box.ptr) return KNN_OK;
-    ix->kd_box_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, 4);
+    ix->kd_box_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, DP <= 16 ? 4 : 16);
     return kd_box_build_dp<DP>(ix, s);
 }
 
-// Traversal 3 (plan.box): per-thread box-bounded search, buckets of plan.leaf_scan slots (0 = 8).
+// The boxes for a search that can do without them: *ready is false where they are missing and cannot
+// be built now (the stream is being captured, or no memory is left for them).
 template <uint32_t DP>
-int kd_box_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s) {
-    if constexpr (DP > 16) {
-        return fail(KNN_ERR_INVALID_ARGUMENT, "box search: dims above 16");
-    } else {
-        KNN_TRY(kd_box_ensure<DP>(ix, s));
-        KdParams p{};
-        p.split = ix->split.as<float>();
-        p.leaf = ix->leaf.as<float>();
-        p.leaf_stride = ix->leaf_stride;
-        p.node_count = ix->node_count;
-        p.node_depth = ix->node_depth;
-        p.stop_depth = std::min(scan_depth_for(ix->node_depth, ix->leaf_slots, plan.leaf_scan ? plan.leaf_scan : 8u),
-                                ix->kd_box_depth);
-        p.leaf_slots = ix->leaf_slots;
-        p.aux = ix->aux_dims;
-        p.queries = a.queries;
-        p.dims = ix->dims;
-        p.nq = a.count;
-        p.order = order;
-        p.count_dev = a.count_dev;
-        p.max_d2 = a.max_d2;
-        p.radii = a.radii;
-        p.k = a.k;
-        p.out_idx = a.out_idx;
-        p.out_dist = a.out_dist;
-        p.counters = a.counters;
-        const uint32_t grid = ceil_div(a.count, 128);
-        if (plan.timing) KNN_TRY(ix->timing.begin(s));
-        switch (k_class(a.k)) {
-            case 8: kd_box_knn_kernel<DP, 8><<<grid, 128, 0, s>>>(p, ix->kd_box.as<float>(), ix->kd_box_stride); break;
-            case 16: kd_box_knn_kernel<DP, 16><<<grid, 128, 0, s>>>(p, ix->kd_box.as<float>(), ix->kd_box_stride); break;
-            case 32: kd_box_knn_kernel<DP, 32><<<grid, 128, 0, s>>>(p, ix->kd_box.as<float>(), ix->kd_box_stride); break;
-            case 64: kd_box_knn_kernel<DP, 64><<<grid, 128, 0, s>>>(p, ix->kd_box.as<float>(), ix->kd_box_stride); break;
-            default: kd_box_knn_kernel<DP, 128><<<grid, 128, 0, s>>>(p, ix->kd_box.as<float>(), ix->kd_box_stride); break;
-        }
-        KNN_LAUNCHED();
-        if (plan.timing) KNN_TRY(ix->timing.end(s));
-        return KNN_OK;
-    }
+int kd_boxes(knn_index* ix, cudaStream_t s, bool* ready) {
+    *ready = ix->kd_box.ptr != nullptr;
+    if (*ready) return KNN_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    KNN_TRY_CUDA(cudaStreamIsCapturing(s, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return KNN_OK;
+    const int rc = kd_box_ensure<DP>(ix, s);
+    *ready = rc == KNN_OK;
+    return rc == KNN_ERR_OUT_OF_MEMORY ? KNN_OK : rc;
 }
 
-// Warp-group search (plan.group) with per-query seeds (or self seeds when `seeds` holds none):
-// boxes built on first use, locality order, the group kernel and the fallback list.  Scratch
-// (seeds when self-seeded, the fallback list) comes from the index workspace after the order.
+// Bucket slots at least (plans may ask for more).  A warp scans 32 slots at once, and the fewer, larger buckets of 32 are
+// the cheapest in few dimensions (4.19 M 3-d points: 1.83 ms, 1.99 with 8); in more the boxes of
+// smaller ones prune more (11 dims: 1.92 ms with 16, 2.3 with 32).
+inline uint32_t kd_warp_bucket(uint32_t dims) { return dims <= 8 ? 32u : 16u; }
+
 template <uint32_t DP>
-int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
-                      float* seeds, uint32_t* fb_list, uint32_t* fb_count, float seed_scale, cudaStream_t s) {
+int kd_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s) {
+    const KdParams p = kd_box_params(ix, a, order, std::max(plan.leaf_scan, kd_warp_bucket(ix->dims)));
+    const uint32_t grid = ceil_div(a.count, kWarpsPerBlock), threads = 32 * kWarpsPerBlock;
+    void (*kern)(const KdParams) = nullptr;
+    if (p.seeds)
+        kern = a.k <= 32 ? kd_warp_query_kernel<DP, 1, true> : a.k <= 64 ? kd_warp_query_kernel<DP, 2, true> : kd_warp_query_kernel<DP, 4, true>;
+    else
+        kern = a.k <= 32 ? kd_warp_query_kernel<DP, 1, false> : a.k <= 64 ? kd_warp_query_kernel<DP, 2, false> : kd_warp_query_kernel<DP, 4, false>;
+    if (plan.timing) KNN_TRY(ix->timing.begin(s));
+    kern<<<grid, threads, 0, s>>>(p);
+    KNN_LAUNCHED();
+    if (plan.timing) KNN_TRY(ix->timing.end(s));
+    return KNN_OK;
+}
+
+// Warp-group search (plan.group) from each query's own subtree: boxes built on first use, the group
+// kernel in the batch's locality order, then the leftovers.
+template <uint32_t DP>
+int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s) {
     if constexpr (DP > 16) {
         return fail(KNN_ERR_INVALID_ARGUMENT, "group search: dims above 16");
     } else {
         if (a.k > 32) return fail(KNN_ERR_INVALID_ARGUMENT, "group search: k above 32");
         KNN_TRY(kd_box_ensure<DP>(ix, s));
-        const bool self_seed = seeds == nullptr;
         const size_t n = a.count;
-        if (self_seed) {
-            KNN_TRY(ix->group_ws.reserve(carve_bytes({n * 4, n * 4, 256})));
-            Carver c(ix->group_ws.ptr);
-            seeds = c.take<float>(n);
-            fb_list = c.take<uint32_t>(n);
-            fb_count = c.take<uint32_t>(1);
-        }
+        KNN_TRY(ix->group_ws.reserve(carve_bytes({n * 4, n * 4, 256})));
+        Carver c(ix->group_ws.ptr);
+        float* seeds = c.take<float>(n);
+        uint32_t* fb_list = c.take<uint32_t>(n);
+        uint32_t* fb_count = c.take<uint32_t>(1);
         switch (k_class(a.k)) {
-            case 8: return launch_kd_group<DP, 8>(ix, a, plan, order, seeds, self_seed, fb_list, fb_count, seed_scale, s);
-            case 16: return launch_kd_group<DP, 16>(ix, a, plan, order, seeds, self_seed, fb_list, fb_count, seed_scale, s);
-            default: return launch_kd_group<DP, 32>(ix, a, plan, order, seeds, self_seed, fb_list, fb_count, seed_scale, s);
+            case 8: return launch_kd_group<DP, 8>(ix, a, plan, order, seeds, fb_list, fb_count, s);
+            case 16: return launch_kd_group<DP, 16>(ix, a, plan, order, seeds, fb_list, fb_count, s);
+            default: return launch_kd_group<DP, 32>(ix, a, plan, order, seeds, fb_list, fb_count, s);
         }
     }
 }
 
 template int kd_query_dp<KNN_DP>(knn_index*, const QueryArgs&, const QueryPlan&, cudaStream_t);
-template int kd_box_query_dp<KNN_DP>(knn_index*, const QueryArgs&, const QueryPlan&, const uint32_t*, cudaStream_t);
-template <>
-int kd_box_prepare_dp<KNN_DP>(knn_index* ix, cudaStream_t s) {
-    if constexpr (KNN_DP > 16) return fail(KNN_ERR_INVALID_ARGUMENT, "box search: dims above 16");
-    else return kd_box_ensure<KNN_DP>(ix, s);
-}
-template int kd_group_query_dp<KNN_DP>(knn_index*, const QueryArgs&, const QueryPlan&, const uint32_t*, float*,
-                                        uint32_t*, uint32_t*, float, cudaStream_t);
+template int kd_boxes<KNN_DP>(knn_index*, cudaStream_t, bool*);
 template int kd_order_dp<KNN_DP>(knn_index*, const QueryArgs&, cudaStream_t, const uint32_t**, uint32_t);
 
 
@@ -1087,8 +996,6 @@ struct KdBatchSet {
     uint32_t first_block;  // first work block of this set in the class
     uint32_t query_offset; // first query of this set in the class-wide numbering
     uint32_t levels;       // descent depth of the locality key
-    const float* box;      // the index's node boxes (box-search classes), or null
-    uint32_t box_stride;
 };
 
 __device__ __forceinline__ uint32_t kd_find_set(const KdBatchSet* sets, uint32_t nsets, uint32_t item, bool by_query) {
@@ -1123,7 +1030,7 @@ __global__ void kd_batch_key_kernel(const KdBatchSet* __restrict__ sets, uint32_
 
 // Persistent kernel: blocks take work blocks (blockDim queries of one set) from a shared counter
 // until the class is done; sets of very different sizes share the GPU without a launch each.
-// MODE: 0 per-thread search, 1 warp-coherent search, 2 per-thread box search (dims <= 16).
+// MODE: 0 per-thread search, 1 warp-coherent search.
 template <int DP, int KMAX, int MODE>
 __global__ void __launch_bounds__(256) kd_batch_kernel(const KdBatchSet* __restrict__ sets, uint32_t nsets,
                                                         uint32_t total_blocks, uint32_t* __restrict__ counter) {
@@ -1140,15 +1047,29 @@ __global__ void __launch_bounds__(256) kd_batch_kernel(const KdBatchSet* __restr
         const uint32_t t = (item - sets[si].first_block) * blockDim.x + threadIdx.x;
         if constexpr (MODE == 1) {
             kd_search_warp<DP, KMAX, false, false, false>(p, t, p.nq, smem);
-        } else if constexpr (MODE == 2 && DP <= 16) {
-            if (t < p.nq) {
-                const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
-                kd_box_search<DP, KMAX>(p, sets[si].box, sets[si].box_stride, p.stop_depth, qi,
-                                        p.radii ? p.radii[qi] : p.max_d2);
-            }
         } else {
             if (t < p.nq) kd_search_thread<DP, KMAX, false, false, false>(p, t, smem);
         }
+    }
+}
+
+// A warp per query over the sets' node boxes: persistent warps take the class's queries one by one.
+template <int DP, int KR>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) kd_batch_warp_kernel(const KdBatchSet* __restrict__ sets,
+                                                                           uint32_t nsets, uint32_t total_queries,
+                                                                           uint32_t* __restrict__ counter) {
+    __shared__ KdWarpSmem<DP> sm[kWarpsPerBlock];
+    for (;;) {
+        uint32_t g = 0;
+        if ((threadIdx.x & 31u) == 0) g = atomicAdd(counter, 1u);
+        g = __shfl_sync(kFullMask, g, 0);
+        if (g >= total_queries) break;  // no block-wide barriers
+        const uint32_t si = kd_find_set(sets, nsets, g, true);
+        const KdParams& p = sets[si].p;
+        const uint32_t t = g - sets[si].query_offset;
+        const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
+        kd_warp_query<DP, KR, false>(p, qi, p.max_d2, sm[threadIdx.x >> 5]);
+        __syncwarp();
     }
 }
 
@@ -1175,45 +1096,33 @@ int kd_batch_launch(const void* sets, uint32_t nsets, uint32_t total_queries, ui
     }
     KNN_BATCH(8, 0) KNN_BATCH(16, 0) KNN_BATCH(32, 0) KNN_BATCH(64, 0) KNN_BATCH(128, 0)
     KNN_BATCH(8, 1) KNN_BATCH(16, 1) KNN_BATCH(32, 1) KNN_BATCH(64, 1) KNN_BATCH(128, 1)
-    KNN_BATCH(8, 2) KNN_BATCH(16, 2) KNN_BATCH(32, 2) KNN_BATCH(64, 2) KNN_BATCH(128, 2)
 #undef KNN_BATCH
+    if (mode == 2) {
+        auto kern = kmax <= 32 ? kd_batch_warp_kernel<DP, 1> : kmax <= 64 ? kd_batch_warp_kernel<DP, 2> : kd_batch_warp_kernel<DP, 4>;
+        int per_sm = 0;
+        KNN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarpsPerBlock, 0));
+        const uint32_t grid = std::max(1, per_sm) * static_cast<uint32_t>(sm_count());
+        kern<<<std::min(grid, ceil_div(total_queries, kWarpsPerBlock)), 32 * kWarpsPerBlock, 0, s>>>(d_sets, nsets, total_queries, counter);
+        KNN_LAUNCHED();
+        return KNN_OK;
+    }
     return fail(KNN_ERR_INVALID_ARGUMENT, "batch class k %u", kmax);
 }
 
 #if KNN_DP == 1
-// Fills the search parameters of one batch set from its index and item.
+// Fills the search parameters of one batch set from its index and item (plan.box: a warp per query).
 size_t kd_batch_set_bytes() { return sizeof(KdBatchSet); }
 
 void kd_batch_set_fill(void* out, const knn_index* ix, const QueryArgs& a, const QueryPlan& plan,
                         const uint32_t* order, uint32_t order_base, uint32_t first_block, uint32_t query_offset) {
     KdBatchSet bs{};
-    KdParams& p = bs.p;
-    p.split = ix->split.as<float>();
-    p.aux = ix->aux_dims;
-    p.leaf = ix->leaf.as<float>();
-    p.leaf_stride = ix->leaf_stride;
-    p.node_count = ix->node_count;
-    p.node_depth = ix->node_depth;
-    p.stop_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, plan.leaf_scan);
-    p.leaf_slots = ix->leaf_slots;
-    p.queries = a.queries;
-    p.dims = ix->dims;
-    p.nq = a.count;
-    p.order = order;
-    p.order_base = order_base;
-    p.max_d2 = a.max_d2;
-    p.k = a.k;
-    p.out_idx = a.out_idx;
-    p.out_dist = a.out_dist;
+    // (A class of warp-per-query searches has every index's boxes built before the batch is captured.)
+    bs.p = plan.box ? kd_box_params(ix, a, order, std::max(plan.leaf_scan, kd_warp_bucket(ix->dims)))
+                    : kd_params(ix, a, order, plan.leaf_scan);
+    bs.p.order_base = order_base;
     bs.first_block = first_block;
     bs.query_offset = query_offset;
     bs.levels = std::min<uint32_t>(ix->node_depth, 24);
-    if (plan.box && ix->kd_box.ptr) {  // prepared by kd_box_prepare before the batch is captured
-        bs.box = ix->kd_box.as<float>();
-        bs.box_stride = ix->kd_box_stride;
-        p.stop_depth = std::min(scan_depth_for(ix->node_depth, ix->leaf_slots, plan.leaf_scan ? plan.leaf_scan : 8u),
-                                ix->kd_box_depth);
-    }
     std::memcpy(out, &bs, sizeof(bs));
 }
 #endif

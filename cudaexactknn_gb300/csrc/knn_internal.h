@@ -163,8 +163,9 @@ struct QueryPlan {
     bool timing = false;     // record events around the main search kernel
     bool warp = false;       // trees: warp-coherent traversal instead of one search per thread
     bool group = false;      // k-d tree: warp-group search from per-query radii (traversal 2)
-    bool box = false;        // k-d tree: per-thread search over tight node boxes (traversal 3)
-    uint32_t widen = 0;      // group search: learned seeds x exp(widen * margin / 2) (fewer retries)
+    bool box = false;        // k-d tree: warp-per-query search over tight node boxes, or nothing (traversal 3)
+    bool unseeded = false;   // learned-radius query without the seeds (the autotuner found them slower)
+    uint32_t widen = 0;      // learned seeds x exp(widen * margin / 2) (fewer retries)
     bool bf16 = false;       // brute force: BF16 tensor-core filter + FP32 rescoring
     uint32_t tc_cap = 0;     // candidates kept per query by the filter (0 = default)
     uint32_t leaf_scan = 0;  // 0 = tree leaves
@@ -324,9 +325,9 @@ struct knn_index {
 
     // k-d tree: split value per internal node (implicit heap, children 2i+1, 2i+2).
     knn::DevBuf split;
-    // k-d tree, warp-group search (built on first use): the tight bounding box of the points
-    // under every node down to depth kd_box_depth (subtrees of at most 4 slots), per node
-    // lo[q], hi[q] with q = max(4, padded dims) floats each; and the search's own scratch.
+    // k-d tree (built on first use): the tight bounding box of the points under every node down to
+    // depth kd_box_depth (subtrees of at most 4 slots, 16 beyond 16 dims), per node lo[q], hi[q] with
+    // q = max(4, padded dims) floats each; and the warp-group search's scratch.
     knn::DevBuf kd_box;
     uint32_t kd_box_depth = 0, kd_box_stride = 0;
     knn::DevBuf group_ws;
@@ -407,6 +408,8 @@ struct QueryArgs {
     DevCounters* counters;    // null unless instrumented
     const uint32_t* order = nullptr;      // explicit thread -> query list (no reordering)
     const uint32_t* count_dev = nullptr;  // device-side count bounding `order` (count is then an upper bound)
+    const float* seeds = nullptr;         // warp-per-query searches: radius to try first, per query (x seed_scale)
+    float seed_scale = 1.0f;
 };
 
 // Learned radius model (radius_model.cu).
@@ -439,12 +442,9 @@ int tc_selftest(uint32_t dims, float* max_rel_err, uint32_t* bad);
 int kd_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order, uint32_t max_levels = 24);
 int ball_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order);
 int kd_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s);
-// Warp-group k-d search from per-query seed radii (kd_kernels.cu); queries it cannot settle go to
-// fb_list / fb_count and are answered by the per-thread search in the same call.
-// The k-d node boxes the box and group searches read, built if missing (dims <= 16).
-int kd_box_prepare(knn_index* ix, cudaStream_t s);
-int kd_group_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, const uint32_t* order, float* seeds,
-                   uint32_t* fb_list, uint32_t* fb_count, float seed_scale, cudaStream_t s);
+// Whether queries can search the k-d node boxes (built here if missing): not where the stream is being
+// captured before they were built, nor where no memory is left for them.
+int kd_boxes_ready(knn_index* ix, cudaStream_t s, bool* ready);
 int ball_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s);
 
 // Rows of unfilled results (index -1, distance = radius) for an empty point set.

@@ -114,6 +114,35 @@ __device__ __forceinline__ void load_query(const float* __restrict__ queries, ui
     for (int d = 0; d < DP; ++d) q[d] = static_cast<uint32_t>(d) < dims ? src[d] : 0.0f;
 }
 
+// The same into shared memory, by a warp (a wide query that every lane then reads by broadcast).
+template <int DP>
+__device__ __forceinline__ void stage_query(const float* __restrict__ queries, uint32_t dims, uint32_t qi, uint32_t lane,
+                                            float4* sq) {
+    float* out = reinterpret_cast<float*>(sq);
+    for (uint32_t d = lane; d < static_cast<uint32_t>(DP); d += 32)
+        out[d] = d < dims ? queries[static_cast<size_t>(qi) * dims + d] : 0.0f;
+    __syncwarp();
+}
+
+// dist2_vec4 with the query in shared memory: the same sequential fused sum.
+template <int DP>
+__device__ __forceinline__ float dist2_shared(const float4* sq, const float4* __restrict__ p4) {
+    float acc = 0.0f;
+#pragma unroll 8
+    for (int v = 0; v < DP / 4; ++v) {
+        const float4 a = sq[v], x = p4[v];
+        float t = __fsub_rn(a.x, x.x);
+        acc = __fmaf_rn(t, t, acc);
+        t = __fsub_rn(a.y, x.y);
+        acc = __fmaf_rn(t, t, acc);
+        t = __fsub_rn(a.z, x.z);
+        acc = __fmaf_rn(t, t, acc);
+        t = __fsub_rn(a.w, x.w);
+        acc = __fmaf_rn(t, t, acc);
+    }
+    return acc;
+}
+
 // Per-thread counters flushed once per thread (instrumented runs only).
 struct LocalCounters {
     uint32_t nodes = 0, leaves = 0, points = 0;

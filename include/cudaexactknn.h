@@ -108,15 +108,20 @@ typedef struct knn_query_opts {
     uint32_t shmem_stack;
     uint32_t flags;
     uint32_t leaf_scan;     /* trees: scan whole subtrees of at most this many points as one
-                               leaf (0 = the tree's own leaves) */
-    uint32_t traversal;     /* trees: 0 = one depth-first search per thread (the reference's
-                               scheme), 1 = warp-coherent search (a warp's queries walk together);
+                               leaf (0 = the engine's choice, or the tree's own leaves; the
+                               warp-per-query search takes values below its own choice as that) */
+    uint32_t traversal;     /* trees: 0 = one depth-first search per query (the reference's scheme);
+                               k-d trees run it with a warp per query, bounded by tight node boxes
+                               that the first query builds (a thread per query, bounded by the
+                               splitting planes, where they cannot be built: inside a stream
+                               capture, or out of memory; the storage options above apply to that
+                               search), 1 = warp-coherent search (a warp's queries walk together);
                                k-d trees of at most 16 dims, k <= 32: 2 = warp-group search (a
-                               warp's 32 queries walk the tree once against tight node boxes from
-                               per-query radii -- the radius model's seeds, or each query's own
-                               subtree -- and share out their (bucket, query) scans; leaf_scan =
-                               points per bucket, 0 = 8); 3 = one search per thread bounded by
-                               the same tight node boxes instead of splitting planes */
+                               warp's 32 queries walk the tree once against the node boxes from
+                               their own subtrees' radii and share out their (bucket, query) scans;
+                               leaf_scan = points per bucket, 0 = 8; with KNN_QF_LEARNED_RADIUS the
+                               warp-per-query search from the model's seeds); of at most 16 dims:
+                               3 = 0 */
     uint32_t reserved;      /* KNN_QF_BF16_FILTER: candidates kept per query (0 = the engine's
                                default, min(4096, max(1024, 16 k))); for
                                knn_tuned_plan, the number of candidate plans timed */
@@ -124,7 +129,8 @@ typedef struct knn_query_opts {
 
 /* Per-query statistics written by knn_query_stats (summed over the batch). */
 typedef struct knn_query_counters {
-    uint64_t nodes_visited;    /* internal nodes whose bound was evaluated */
+    uint64_t nodes_visited;    /* nodes whose bound was evaluated (warp-per-query search: and found
+                                  within the radius) */
     uint64_t leaves_visited;   /* leaves scanned */
     uint64_t points_scanned;   /* leaf slots whose distance was computed */
     uint64_t fallback_queries; /* queries the fast form handed to the plain search: learned-
