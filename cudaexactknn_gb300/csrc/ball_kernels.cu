@@ -1,9 +1,10 @@
 // Ball tree query kernels, one translation unit per padded dimension count (KNN_DP).
 //
-// Replaces BallTreeKernels::knnDevice and its four storage variants (src/BallTreeGpu.cuh:36-200).
-// Same depth-first search: at each internal node measure the query's distance to both child
-// balls, descend into the closer one, push the farther one when it can still hold a neighbour,
-// stop the descent when even the closer ball is out of range (src/BallTreeGpu.cuh:82-92).
+// Replaces BallTreeKernels::knnDevice and its four storage variants (src/BallTreeGpu.cuh:36-200),
+// a depth-first search per thread: at each internal node the distance to both child balls, the closer
+// one entered, the farther one pushed when it can still hold a neighbour (src/BallTreeGpu.cuh:82-92).
+// Here each query gets a warp (ball_warp_query_kernel, warp_search.cuh); traversal 1 walks 32
+// neighbouring queries together.
 // The reference's border distance sqrt(d2) - r (with -use_fast_math's approximate sqrt) can
 // round above a point's own float distance and prune a true neighbour; here knn::ball_bound
 // uses directed rounding and relative margins so it never exceeds the float dist2 of any point
@@ -13,6 +14,7 @@
 #include <cstring>
 
 #include "tree_query.cuh"
+#include "warp_search.cuh"
 
 #ifndef KNN_DP
 #error "compile with -DKNN_DP=<padded dims>"
@@ -38,6 +40,8 @@ struct BallParams {
     uint32_t order_base;  // subtracted from order entries (batched orders hold batch-wide ids)
     float max_d2;
     const float* radii;
+    const float* seeds;   // warp-per-query search: per query radius to start from (x seed_scale), or null
+    float seed_scale;
     uint32_t k;
     int32_t* out_idx;
     float* out_dist;
@@ -62,87 +66,6 @@ __device__ __forceinline__ float centre_dist(const float (&q)[DP], const float* 
         *r = b[DP];
         return dist2_vec4<DP>(q, reinterpret_cast<const float4*>(b));
     }
-}
-
-// One thread's search: query slot t of the batch (its query is p.order[t] - p.order_base, or t).
-template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
-__device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t t, unsigned char* smem) {
-    uint64_t* sh_nn = reinterpret_cast<uint64_t*>(smem);
-    uint32_t* sh_st = reinterpret_cast<uint32_t*>(smem + tracker_smem_bytes(SHNN, KMAX, blockDim.x));
-
-    const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
-    float q[DP];
-    load_query<DP>(p.queries, p.dims, qi, q);
-    const float r2 = p.radii ? p.radii[qi] : p.max_d2;
-
-    Tracker<KMAX, HEAP, SHNN> tr;
-    tr.init(p.k, r2, sh_nn + threadIdx.x, blockDim.x);
-    Stack<SHST> st;
-    st.init(sh_st, blockDim.x);
-    st.push(0, 0.0f);
-    LocalCounters lc;
-    bool overflow = false;
-
-    while (st.top) {
-        uint32_t node;
-        float bound;
-        st.pop(&node, &bound);
-        if (bound > tr.radius()) continue;
-        bool pruned = false;
-        uint32_t depth = heap_depth(node);
-        while (depth < p.stop_depth) {
-            const uint32_t l = 2 * node + 1;
-            float rl, rr;
-            const float sl = centre_dist<DP>(q, p.ball + static_cast<size_t>(l) * p.ball_stride, &rl);
-            const float sr = centre_dist<DP>(q, p.ball + static_cast<size_t>(l + 1) * p.ball_stride, &rr);
-            const float bl = ball_bound(sl, rl, p.margin);
-            const float br = ball_bound(sr, rr, p.margin);
-            ++lc.nodes;
-            // Visit order only (not a bound): the nearer border first.
-            const bool left_first = sqrtf(sl) - rl < sqrtf(sr) - rr;
-            const uint32_t close_child = left_first ? l : l + 1;
-            const float close_b = left_first ? bl : br;
-            const float far_b = left_first ? br : bl;
-            if (close_b > tr.radius()) {
-                // The farther ball's bound is at least as large in the common case, but the
-                // order above is approximate, so it is checked on its own.
-                if (far_b <= tr.radius()) {
-                    node = left_first ? l + 1 : l;
-                    ++depth;
-                    continue;
-                }
-                pruned = true;
-                break;
-            }
-            if (far_b <= tr.radius()) overflow |= !st.push(left_first ? l + 1 : l, far_b);
-            node = close_child;
-            ++depth;
-        }
-        if (pruned) continue;
-        const SlotRange r = subtree_slots(node, depth, p.node_depth, p.node_count, p.leaf_slots);
-        const float* slot = p.leaf + r.first * p.leaf_stride;
-        ++lc.leaves;
-        for (uint32_t s = 0; s < r.count; ++s, slot += p.leaf_stride) {
-            int32_t id;
-            const float d2 = slot_dist<DP>(q, slot, &id);
-            if (id < 0) continue;
-            ++lc.points;
-            tr.offer(make_key(d2, id));
-        }
-    }
-    tr.emit(p.k, p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
-    if (p.counters) {
-        lc.flush(p.counters);
-        if (overflow) atomicExch(&p.counters->error, 1);
-    }
-}
-
-template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
-__global__ void __launch_bounds__(256) ball_knn_kernel(const BallParams p) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (p.count_dev ? *p.count_dev : p.nq)) return;  // no block-wide barriers below
-    ball_search_thread<DP, KMAX, HEAP, SHNN, SHST>(p, t, smem);
 }
 
 // Warp-coherent variant (see kd_knn_warp_kernel): the warp's queries walk the tree together,
@@ -231,6 +154,89 @@ __global__ void __launch_bounds__(256) ball_knn_warp_kernel(const BallParams p) 
     ball_search_warp<DP, KMAX, HEAP, SHNN, SHST>(p, t, live, smem);
 }
 
+// One query per warp (warp_search.cuh) over the balls: a node's bound is its ball's, the visit order
+// the distance to the ball's border (overlapping balls have equal bounds of zero).  65,536 queries, k
+// 32, on 262,144 points near a 4-d subspace of 16 dims: 4.2 ms (a thread per query with its stack and
+// top-k in local memory: 15.6; 4,000 uniform 32-d queries, k 64, on 30,000: 3.4 and 177).  Bound by the
+// L2 reads of balls and slots, about 10,000 rows of 80 bytes per query there.
+template <int DP>
+struct BallWarpView {
+    static constexpr bool kKeys = true;
+    static constexpr bool kShared = DP > 32;  // wide queries are read from shared memory (broadcast)
+    float q[kShared ? 1 : DP];
+    const float4* sq;
+    const float* ball;
+    uint32_t ball_stride;
+    float margin;
+    __device__ __forceinline__ float dist2_to(const float* row, float* last) const {
+        if constexpr (kShared) {
+            *last = row[DP];
+            return dist2_shared<DP>(sq, reinterpret_cast<const float4*>(row));
+        } else {
+            return centre_dist<DP>(q, row, last);
+        }
+    }
+    __device__ __forceinline__ void test(uint32_t node, float* bound, uint32_t* key) const {
+        float r;
+        const float s = dist2_to(ball + static_cast<size_t>(node) * ball_stride, &r);
+        *bound = ball_bound(s, r, margin);
+        *key = min(orderable(sqrtf(s) - r), 0xFFFFFFFEu);
+    }
+    __device__ __forceinline__ float dist(const float* slot, int32_t* id) const {
+        float last;
+        const float d2 = dist2_to(slot, &last);
+        *id = __float_as_int(last);
+        return d2;
+    }
+};
+
+template <int DP>
+struct BallWarpSmem {
+    WarpRows<true> rows;
+    float4 q[DP > 32 ? DP / 4 : 1];
+};
+
+// One warp's search of query qi within r2; its row goes to the query's result slots.
+template <int DP, int KR, bool SEEDED>
+__device__ __forceinline__ void ball_warp_query(const BallParams& p, uint32_t qi, float r2, BallWarpSmem<DP>& sm) {
+    const uint32_t lane = threadIdx.x & 31u;
+    BallWarpView<DP> view;
+    if constexpr (DP > 32) {
+        stage_query<DP>(p.queries, p.dims, qi, lane, sm.q);
+        view.sq = sm.q;
+    } else {
+        load_query<DP>(p.queries, p.dims, qi, view.q);
+    }
+    view.ball = p.ball;
+    view.ball_stride = p.ball_stride;
+    view.margin = p.margin;
+    const WarpTree t{p.leaf, p.leaf_stride, p.leaf_slots << (p.node_depth - p.stop_depth), p.stop_depth};
+    WarpTopK<KR> top;
+    LocalCounters lc;
+    bool missed = false;
+    top.init(p.k, r2, lane);
+    if constexpr (SEEDED) {
+        const float r = p.seeds[qi] * p.seed_scale;
+        missed = warp_search<BallWarpView<DP>, KR, true>(view, t, sm.rows, top, lc, r < r2 ? r : r2, r2);
+    } else {
+        warp_search<BallWarpView<DP>, KR, false>(view, t, sm.rows, top, lc, r2, r2);
+    }
+    top.emit(p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
+    if (p.counters && lane == 0) {
+        lc.flush(p.counters);
+        if (missed) atomicAdd(&p.counters->fallback, 1ull);
+    }
+}
+
+template <int DP, int KR, bool SEEDED>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) ball_warp_query_kernel(const BallParams p) {
+    __shared__ BallWarpSmem<DP> sm[kWarpsPerBlock];
+    const uint32_t w = threadIdx.x >> 5, t = blockIdx.x * kWarpsPerBlock + w;
+    if (t >= (p.count_dev ? *p.count_dev : p.nq)) return;  // no block-wide barriers
+    const uint32_t qi = p.order ? p.order[t] : t;
+    ball_warp_query<DP, KR, SEEDED>(p, qi, p.radii ? p.radii[qi] : p.max_d2, sm[w]);
+}
+
 // Sort key of a query: the node reached after `levels` steps towards the nearer child centre.
 template <int DP>
 __global__ void ball_leaf_key_kernel(const float* __restrict__ ball, uint32_t ball_stride, uint32_t levels,
@@ -252,14 +258,8 @@ __global__ void ball_leaf_key_kernel(const float* __restrict__ ball, uint32_t ba
     vals[t] = t;
 }
 
-template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
-static int launch_ball(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
-                       cudaStream_t s) {
-    const uint32_t block = plan.block ? plan.block : 128;
-    const size_t smem = tracker_smem_bytes(SHNN, KMAX, block) + stack_smem_bytes(SHST, block);
-    auto kern = plan.warp ? ball_knn_warp_kernel<DP, KMAX, HEAP, SHNN, SHST> : ball_knn_kernel<DP, KMAX, HEAP, SHNN, SHST>;
-    if (smem > 48 * 1024)
-        KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+// A query batch's search parameters: its tree, buckets of `bucket` slots (0 = the tree's leaves).
+inline BallParams ball_params(const knn_index* ix, const QueryArgs& a, const uint32_t* order, uint32_t bucket) {
     BallParams p{};
     p.ball = ix->ball.as<float>();
     p.ball_stride = ix->ball_stride;
@@ -267,7 +267,7 @@ static int launch_ball(knn_index* ix, const QueryArgs& a, const QueryPlan& plan,
     p.leaf_stride = ix->leaf_stride;
     p.node_count = ix->node_count;
     p.node_depth = ix->node_depth;
-    p.stop_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, plan.leaf_scan);
+    p.stop_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, bucket);
     p.leaf_slots = ix->leaf_slots;
     p.margin = rel_margin(ix->dims);
     p.queries = a.queries;
@@ -277,10 +277,25 @@ static int launch_ball(knn_index* ix, const QueryArgs& a, const QueryPlan& plan,
     p.count_dev = a.count_dev;
     p.max_d2 = a.max_d2;
     p.radii = a.radii;
+    p.seeds = a.seeds;
+    p.seed_scale = a.seed_scale;
     p.k = a.k;
     p.out_idx = a.out_idx;
     p.out_dist = a.out_dist;
     p.counters = a.counters;
+    return p;
+}
+
+// Warp-coherent search (traversal 1).
+template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
+static int launch_ball(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
+                       cudaStream_t s) {
+    const uint32_t block = plan.block ? plan.block : 128;
+    const size_t smem = tracker_smem_bytes(SHNN, KMAX, block) + stack_smem_bytes(SHST, block);
+    auto kern = ball_knn_warp_kernel<DP, KMAX, HEAP, SHNN, SHST>;
+    if (smem > 48 * 1024)
+        KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    const BallParams p = ball_params(ix, a, order, plan.leaf_scan);
     if (plan.timing) KNN_TRY(ix->timing.begin(s));
     kern<<<ceil_div(a.count, block), block, smem, s>>>(p);
     KNN_LAUNCHED();
@@ -332,9 +347,45 @@ int ball_order_dp(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint3
     return KNN_OK;
 }
 
+// Bucket slots at least (plans may ask for more): 16 up to 16 dims (16 dims, 262,144 points: 4.16 to
+// 4.39 ms with 8, 16 and 32), 8 beyond, where smaller balls prune more than larger scans save (24
+// dims: 3.06 ms with 8, 3.46 with 32; 100 dims: 4.7 and 6.4).
+inline uint32_t ball_warp_bucket(uint32_t dims) { return dims <= 16 ? 16u : 8u; }
+
+// A warp per query over the balls (traversal 0).
+template <uint32_t DP>
+int ball_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s) {
+    const BallParams p = ball_params(ix, a, order, std::max(plan.leaf_scan, ball_warp_bucket(ix->dims)));
+    const uint32_t grid = ceil_div(a.count, kWarpsPerBlock), threads = 32 * kWarpsPerBlock;
+    void (*kern)(const BallParams) = nullptr;
+    if (p.seeds)
+        kern = a.k <= 32 ? ball_warp_query_kernel<DP, 1, true> : a.k <= 64 ? ball_warp_query_kernel<DP, 2, true> : ball_warp_query_kernel<DP, 4, true>;
+    else
+        kern = a.k <= 32 ? ball_warp_query_kernel<DP, 1, false> : a.k <= 64 ? ball_warp_query_kernel<DP, 2, false> : ball_warp_query_kernel<DP, 4, false>;
+    if (plan.timing) KNN_TRY(ix->timing.begin(s));
+    kern<<<grid, threads, 0, s>>>(p);
+    KNN_LAUNCHED();
+    if (plan.timing) KNN_TRY(ix->timing.end(s));
+    return KNN_OK;
+}
+
 template <uint32_t DP>
 int ball_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s) {
     const uint32_t* order = a.order;
+    if (!p.warp) {
+        // The storage options do not matter to a warp's search; sizes no block can hold stay refused.
+        const uint32_t block = p.block ? p.block : 128;
+        const size_t storage = tracker_smem_bytes(p.sh_nn, k_class(a.k), block) + stack_smem_bytes(p.sh_stack, block);
+        if (storage > kMaxBlockSmem)
+            return fail(KNN_ERR_CUDA, "storage options: %zu bytes of shared memory per block of %u", storage, block);
+        // Neighbouring queries share the rows they read through the caches: an order pays where rows are
+        // wide (the search then lives on L2 reads; 16 dims, 65,536 queries on 262,144 points: 4.14 ms
+        // sorted, 4.39 not) or the index outgrows L2, and costs otherwise (3 dims, 25,000 queries on
+        // 200,000: 0.25 and 0.17).
+        const bool wide = DP >= 16 && a.count >= 16384, large = a.count >= kWarpOrderMin && ix->leaf.bytes > kL2Bytes;
+        if (!order && p.reorder && (wide || large)) KNN_TRY(ball_order_dp<DP>(ix, a, s, &order));
+        return ball_warp_query_dp<DP>(ix, a, p, order, s);
+    }
     if (!order && p.reorder && a.count >= 4096) KNN_TRY(ball_order_dp<DP>(ix, a, s, &order));
     switch (k_class(a.k)) {
         case 8: return launch_ball_variant<DP, 8>(ix, a, p, order, s);
@@ -390,9 +441,9 @@ __global__ void ball_batch_key_kernel(const BallBatchSet* __restrict__ sets, uin
     vals[g] = g;
 }
 
-// Persistent kernel: blocks take work blocks (blockDim queries of one set) from a shared counter
+// Warp-coherent search: blocks take work blocks (blockDim queries of one set) from a shared counter
 // until the class is done; sets of very different sizes share the GPU without a launch each.
-template <int DP, int KMAX, bool WARP>
+template <int DP, int KMAX>
 __global__ void __launch_bounds__(256) ball_batch_kernel(const BallBatchSet* __restrict__ sets, uint32_t nsets,
                                                         uint32_t total_blocks, uint32_t* __restrict__ counter) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -406,17 +457,33 @@ __global__ void __launch_bounds__(256) ball_batch_kernel(const BallBatchSet* __r
         const uint32_t si = ball_find_set(sets, nsets, item, false);
         const BallParams& p = sets[si].p;
         const uint32_t t = (item - sets[si].first_block) * blockDim.x + threadIdx.x;
-        if constexpr (WARP) {
-            ball_search_warp<DP, KMAX, false, false, false>(p, t, p.nq, smem);
-        } else {
-            if (t < p.nq) ball_search_thread<DP, KMAX, false, false, false>(p, t, smem);
-        }
+        ball_search_warp<DP, KMAX, false, false, false>(p, t, p.nq, smem);
+    }
+}
+
+// A warp per query: persistent warps take the class's queries one by one.
+template <int DP, int KR>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) ball_batch_warp_kernel(const BallBatchSet* __restrict__ sets,
+                                                                             uint32_t nsets, uint32_t total_queries,
+                                                                             uint32_t* __restrict__ counter) {
+    __shared__ BallWarpSmem<DP> sm[kWarpsPerBlock];
+    for (;;) {
+        uint32_t g = 0;
+        if ((threadIdx.x & 31u) == 0) g = atomicAdd(counter, 1u);
+        g = __shfl_sync(kFullMask, g, 0);
+        if (g >= total_queries) break;  // no block-wide barriers
+        const uint32_t si = ball_find_set(sets, nsets, g, true);
+        const BallParams& p = sets[si].p;
+        const uint32_t t = g - sets[si].query_offset;
+        const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
+        ball_warp_query<DP, KR, false>(p, qi, p.max_d2, sm[threadIdx.x >> 5]);
+        __syncwarp();
     }
 }
 
 template <uint32_t DP>
 int ball_batch_launch(const void* sets, uint32_t nsets, uint32_t total_queries, uint32_t total_blocks, uint32_t kmax,
-                       bool warp, uint32_t block, uint32_t* counter, uint32_t* keys, uint32_t* vals, bool key_pass,
+                       uint32_t mode, uint32_t block, uint32_t* counter, uint32_t* keys, uint32_t* vals, bool key_pass,
                        cudaStream_t s) {
     using Set = BallBatchSet;
     const Set* d_sets = static_cast<const Set*>(sets);
@@ -425,9 +492,9 @@ int ball_batch_launch(const void* sets, uint32_t nsets, uint32_t total_queries, 
         KNN_LAUNCHED();
         return KNN_OK;
     }
-#define KNN_BATCH(KM, W)                                                                              \
-    if (kmax == KM && warp == W) {                                                                    \
-        auto kern = ball_batch_kernel<DP, KM, W>;                                                    \
+#define KNN_BATCH(KM)                                                                                 \
+    if (kmax == KM && mode == 1) {                                                                    \
+        auto kern = ball_batch_kernel<DP, KM>;                                                       \
         int per_sm = 0;                                                                               \
         KNN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0));         \
         const uint32_t grid = std::max(1, per_sm) * static_cast<uint32_t>(sm_count());                \
@@ -435,9 +502,17 @@ int ball_batch_launch(const void* sets, uint32_t nsets, uint32_t total_queries, 
         KNN_LAUNCHED();                                                                               \
         return KNN_OK;                                                                                \
     }
-    KNN_BATCH(8, false) KNN_BATCH(16, false) KNN_BATCH(32, false) KNN_BATCH(64, false) KNN_BATCH(128, false)
-    KNN_BATCH(8, true) KNN_BATCH(16, true) KNN_BATCH(32, true) KNN_BATCH(64, true) KNN_BATCH(128, true)
+    KNN_BATCH(8) KNN_BATCH(16) KNN_BATCH(32) KNN_BATCH(64) KNN_BATCH(128)
 #undef KNN_BATCH
+    if (mode == 2) {
+        auto kern = kmax <= 32 ? ball_batch_warp_kernel<DP, 1> : kmax <= 64 ? ball_batch_warp_kernel<DP, 2> : ball_batch_warp_kernel<DP, 4>;
+        int per_sm = 0;
+        KNN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarpsPerBlock, 0));
+        const uint32_t grid = std::max(1, per_sm) * static_cast<uint32_t>(sm_count());
+        kern<<<std::min(grid, ceil_div(total_queries, kWarpsPerBlock)), 32 * kWarpsPerBlock, 0, s>>>(d_sets, nsets, total_queries, counter);
+        KNN_LAUNCHED();
+        return KNN_OK;
+    }
     return fail(KNN_ERR_INVALID_ARGUMENT, "batch class k %u", kmax);
 }
 
@@ -448,25 +523,8 @@ size_t ball_batch_set_bytes() { return sizeof(BallBatchSet); }
 void ball_batch_set_fill(void* out, const knn_index* ix, const QueryArgs& a, const QueryPlan& plan,
                         const uint32_t* order, uint32_t order_base, uint32_t first_block, uint32_t query_offset) {
     BallBatchSet bs{};
-    BallParams& p = bs.p;
-    p.ball = ix->ball.as<float>();
-    p.ball_stride = ix->ball_stride;
-    p.margin = rel_margin(ix->dims);
-    p.leaf = ix->leaf.as<float>();
-    p.leaf_stride = ix->leaf_stride;
-    p.node_count = ix->node_count;
-    p.node_depth = ix->node_depth;
-    p.stop_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, plan.leaf_scan);
-    p.leaf_slots = ix->leaf_slots;
-    p.queries = a.queries;
-    p.dims = ix->dims;
-    p.nq = a.count;
-    p.order = order;
-    p.order_base = order_base;
-    p.max_d2 = a.max_d2;
-    p.k = a.k;
-    p.out_idx = a.out_idx;
-    p.out_dist = a.out_dist;
+    bs.p = ball_params(ix, a, order, plan.warp ? plan.leaf_scan : std::max(plan.leaf_scan, ball_warp_bucket(ix->dims)));
+    bs.p.order_base = order_base;
     bs.first_block = first_block;
     bs.query_offset = query_offset;
     bs.levels = std::min<uint32_t>(ix->node_depth, 24);
@@ -474,7 +532,7 @@ void ball_batch_set_fill(void* out, const knn_index* ix, const QueryArgs& a, con
 }
 #endif
 
-template int ball_batch_launch<KNN_DP>(const void*, uint32_t, uint32_t, uint32_t, uint32_t, bool, uint32_t, uint32_t*,
+template int ball_batch_launch<KNN_DP>(const void*, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t*,
                                       uint32_t*, uint32_t*, bool, cudaStream_t);
 
 }  // namespace knn

@@ -30,7 +30,7 @@ template <uint32_t DP>
 int kd_batch_launch(const void*, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t*, uint32_t*,
                     uint32_t*, bool, cudaStream_t);
 template <uint32_t DP>
-int ball_batch_launch(const void*, uint32_t, uint32_t, uint32_t, uint32_t, bool, uint32_t, uint32_t*, uint32_t*,
+int ball_batch_launch(const void*, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t*, uint32_t*,
                       uint32_t*, bool, cudaStream_t);
 size_t kd_batch_set_bytes();
 size_t ball_batch_set_bytes();
@@ -43,7 +43,7 @@ int query_structure(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaS
 
 namespace {
 
-// mode: 0 per-thread search, 1 warp-coherent, 2 a warp per query over the node boxes (k-d only).
+// mode: 0 per-thread search, 1 warp-coherent, 2 a warp per query (k-d: over the node boxes).
 int batch_launch(int structure, uint32_t dp, const void* sets, uint32_t nsets, uint32_t total_queries,
                  uint32_t total_blocks, uint32_t kmax, uint32_t mode, uint32_t block, uint32_t* counter, uint32_t* keys,
                  uint32_t* vals, bool key_pass, cudaStream_t s) {
@@ -52,8 +52,8 @@ int batch_launch(int structure, uint32_t dp, const void* sets, uint32_t nsets, u
         return structure == KNN_KD_TREE                                                                             \
                    ? kd_batch_launch<D_>(sets, nsets, total_queries, total_blocks, kmax, mode, block, counter, keys, \
                                          vals, key_pass, s)                                                         \
-                   : ball_batch_launch<D_>(sets, nsets, total_queries, total_blocks, kmax, mode == 1, block, counter, \
-                                           keys, vals, key_pass, s);
+                   : ball_batch_launch<D_>(sets, nsets, total_queries, total_blocks, kmax, mode, block, counter, keys, \
+                                           vals, key_pass, s);
     switch (dp) {
         KNN_BL(1) KNN_BL(2) KNN_BL(3) KNN_BL(4) KNN_BL(8) KNN_BL(16) KNN_BL(32) KNN_BL(64) KNN_BL(128)
         default: return fail(KNN_ERR_UNSUPPORTED, "dims");
@@ -239,11 +239,12 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
             }
             continue;
         }
-        if (c.structure == KNN_KD_TREE && !c.plan.warp) {
-            // A warp per query over each index's node boxes, built now (capture cannot allocate); the
-            // per-thread search where there is no memory for them.
+        if (!c.plan.warp) {
+            // A warp per query; k-d trees over each index's node boxes, built now (capture cannot
+            // allocate), or the per-thread search where there is no memory for them.
             c.plan.box = true;
             for (uint32_t i : c.items) {
+                if (c.structure != KNN_KD_TREE) break;
                 bool ready = false;
                 if ((rc = knn::kd_boxes_ready(items[i].index, s, &ready)) != KNN_OK) break;
                 c.plan.box = c.plan.box && ready;
@@ -257,9 +258,9 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
             first_block += knn::ceil_div(items[i].count, block);
         }
         c.total_blocks = first_block;
-        // (A warp per query gains from the locality sort only beyond L2, where one graph of many small
-        // sets is not; the sort's launches would cost more than the searches.)
-        c.sort = (flags & KNN_QF_KEEP_ORDER) == 0 && !c.plan.box;
+        // A warp per query gains from the locality sort where rows are wide, as in a single query (ball
+        // trees of 16 dims and more); elsewhere its launches would cost more than the searches.
+        c.sort = (flags & KNN_QF_KEEP_ORDER) == 0 && (!c.plan.box || (c.structure == KNN_BALL_TREE && c.dp >= 16));
         uint32_t set_bits = 0;
         while ((1u << set_bits) < c.items.size()) ++set_bits;
         c.key_bits = 24 + set_bits;

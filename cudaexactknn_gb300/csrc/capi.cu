@@ -150,7 +150,7 @@ int seeded_query(knn_index* ix, const knn::QueryArgs& a, const knn::QueryPlan& p
     const size_t n = a.count;
     if (plan.group && (ix->dp > 16 || a.k > 32))
         return fail(KNN_ERR_INVALID_ARGUMENT, "group search: dims above 16 or k above 32");
-    bool warp_query = false;
+    bool warp_query = ix->structure == KNN_BALL_TREE && !plan.warp;
     if (ix->structure == KNN_KD_TREE && !plan.warp) KNN_TRY(knn::kd_boxes_ready(ix, s, &warp_query));
     if (warp_query) {
         // The warp-per-query search starts each query from its seed and, where that held fewer than k
@@ -336,7 +336,7 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             }
             if (rc != KNN_OK) break;
         }
-        if (learned && ix->structure == KNN_KD_TREE) {
+        if (learned && ix->structure != KNN_BRUTE_FORCE) {
             // And without them: a warp's search finds a radius nearly as good in its first bucket, so
             // where the model is not cheap against the search the seeds do not pay for it (4.19 M
             // clustered 3-d points, 1,048,576 queries: 1.83 ms without, 2.0 with).
@@ -376,8 +376,8 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             }
         }
         const knn::QueryPlan stage2 = best;
-        // Kernels of fixed shape: the filter, and the k-d trees' warp-per-query search.
-        const bool fixed = stage2.bf16 || (ix->structure == KNN_KD_TREE && !stage2.warp);
+        // Kernels of fixed shape: the filter, and the trees' warp-per-query search.
+        const bool fixed = stage2.bf16 || (ix->structure != KNN_BRUTE_FORCE && !stage2.warp);
         for (uint32_t block : {32u, 64u, 256u}) {
             if (fixed) break;
             knn::QueryPlan p = stage2;

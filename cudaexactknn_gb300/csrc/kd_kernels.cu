@@ -27,10 +27,6 @@
 
 namespace knn {
 
-constexpr size_t kMaxBlockSmem = 232448;        // most shared memory a block can ask for
-constexpr size_t kL2Bytes = 128u << 20;         // this GPU's L2
-constexpr uint32_t kWarpOrderMin = 1u << 18;    // fewest queries worth an order on an index beyond L2
-
 struct KdParams {
     const float* split;
     const float* leaf;
@@ -704,8 +700,6 @@ struct KdWarpView {
         }
     }
 };
-
-constexpr uint32_t kWarpsPerBlock = 4;
 
 template <int DP>
 struct KdWarpSmem {

@@ -24,6 +24,10 @@ namespace knn {
 constexpr uint32_t kWarpFan = 5;    // levels per step: up to 32 descendants, one per lane
 constexpr uint32_t kWarpRows = 7;   // steps of a tree of at most 32 levels
 constexpr uint32_t kFullMask = 0xFFFFFFFFu;
+constexpr uint32_t kWarpsPerBlock = 2;  // queries of a block (4: 2% slower, 8: 5%, as a block waits for its slowest)
+constexpr size_t kMaxBlockSmem = 232448;      // most shared memory a block can ask for
+constexpr size_t kL2Bytes = 128u << 20;       // this GPU's L2
+constexpr uint32_t kWarpOrderMin = 1u << 18;  // fewest queries worth an order on an index beyond L2
 
 __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, uint32_t m) {
     const uint32_t lo = __shfl_xor_sync(kFullMask, static_cast<uint32_t>(v), m);
@@ -74,6 +78,7 @@ __device__ __forceinline__ uint64_t warp_merge_low64(uint64_t a, uint64_t b, uin
 }
 
 // The k smallest keys seen, ascending over (register, lane): rank r is register r / 32 of lane r % 32.
+// KR = 1 takes k <= 32, 2 k in (32, 64], 4 k in (64, 128].
 template <int KR>
 struct WarpTopK {
     uint64_t v[KR];
@@ -91,10 +96,8 @@ struct WarpTopK {
     }
     __device__ __forceinline__ float radius() const { return key_dist(kth); }
     __device__ __forceinline__ void refresh() {
-        uint64_t s = v[0];
-#pragma unroll
-        for (int j = 1; j < KR; ++j) s = (k - 1) / 32 == static_cast<uint32_t>(j) ? v[j] : s;
-        kth = shfl64(s, (k - 1) & 31u);
+        // (Rank k - 1 is in the last register, or with four in the third: k > 16 KR beyond 32.)
+        kth = shfl64(KR == 4 && k <= 96 ? v[KR - 2 + (KR == 1)] : v[KR - 1], (k - 1) & 31u);
     }
     // Inserts a key every lane holds.
     __device__ __forceinline__ void insert(uint64_t x) {
@@ -147,12 +150,13 @@ struct WarpTopK {
     }
 };
 
-// Shared memory of one warp: the waiting rows (bounds, and where the tree's visit order is not the
-// bound's, order keys).
+// Shared memory of one warp: the waiting rows (bounds; where the tree's visit order is not the
+// bound's, order keys; and for a seeded search over balls the bounds as they were tested).
 template <bool KEYS>
 struct WarpRows {
     float bound[kWarpRows][32];
     uint32_t key[KEYS ? kWarpRows : 1][32];
+    float tested[KEYS ? kWarpRows : 1][32];
 };
 
 struct WarpTree {
@@ -168,7 +172,8 @@ struct WarpTree {
 // SEEDED: subtrees are first entered only within r < r2 as well (scanned slots are offered all the
 // same).  A row left behind keeps its least remaining bound in its parent's, so that a seed that held
 // fewer than k points costs no second search: r goes to r2 and the search goes on from there, past the
-// buckets it has scanned.  Returns whether it had to.
+// buckets it has scanned.  (A ball's bound can be below its parent's: which buckets were scanned is
+// told by the largest bound on their path, `tested`.)  Returns whether it had to.
 template <class View, int KR, bool SEEDED>
 __device__ __forceinline__ bool warp_search(const View& view, const WarpTree& t, WarpRows<View::kKeys>& sm,
                                             WarpTopK<KR>& top, LocalCounters& lc, float r, float r2) {
@@ -178,11 +183,15 @@ __device__ __forceinline__ bool warp_search(const View& view, const WarpTree& t,
     uint32_t row = 0, par = 0, depth = lv0, lv = lv0;      // par: index, within its depth, of the row's parent
     float bound = __int_as_float(0x7fc00000);              // NaN: never within a radius (absent, or taken)
     uint32_t key = 0;
+    constexpr bool kTrack = SEEDED && View::kKeys;
+    float tested = 0.0f, above = 0.0f;                     // kTrack: this lane's path bound, the row's parent's
     float scanned = -1.0f;                                 // SEEDED: buckets within this are done
     auto radius = [&]() { return SEEDED ? fminf(r, top.radius()) : top.radius(); };
     auto expand = [&]() {
         bound = __int_as_float(0x7fc00000);
         if (lane < (1u << lv)) view.test((1u << depth) - 1u + (par << lv) + lane, &bound, &key);
+        if (kTrack && bound < above) bound = above;
+        tested = bound;
         if (SEEDED && row + 1 == steps && bound <= scanned) bound = __int_as_float(0x7fc00000);
         lc.nodes += __popc(__ballot_sync(kFullMask, bound <= radius()));
     };
@@ -197,6 +206,7 @@ __device__ __forceinline__ bool warp_search(const View& view, const WarpTree& t,
             m = __ballot_sync(kFullMask, want && k == best);
         }
         const uint32_t src = static_cast<uint32_t>(__ffs(m) - 1);
+        if constexpr (kTrack) above = __shfl_sync(kFullMask, tested, src);
         if (lane == src) bound = __int_as_float(0x7fc00000);
         *child = (par << lv) + src;
         return true;
@@ -221,11 +231,13 @@ __device__ __forceinline__ bool warp_search(const View& view, const WarpTree& t,
             bound = sm.bound[row][lane];
             if (SEEDED && lane == src) bound = __uint_as_float(rest);
             if constexpr (View::kKeys) key = sm.key[row][lane];
+            if constexpr (kTrack) tested = sm.tested[row][lane];
             continue;
         }
         if (row + 1 < steps) {
             sm.bound[row][lane] = bound;
             if constexpr (View::kKeys) sm.key[row][lane] = key;
+            if constexpr (kTrack) sm.tested[row][lane] = tested;
             ++row;
             par = child;
             lv = kWarpFan;

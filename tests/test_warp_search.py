@@ -120,7 +120,7 @@ def _want(pts, qs, k, r2=INF):
 # 32-slot buckets: 1 to 3 of them, one step's 32 (1,024 slots) and one more, two steps and one more.
 @gpu
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 65, 1024, 1025, 32768, 32769])
-@pytest.mark.parametrize("structure", ["kd"])
+@pytest.mark.parametrize("structure", ["kd", "ball"])
 def test_steps_and_buckets(structure, n):
     gu = _gu()
     rng = np.random.default_rng(n)
@@ -139,7 +139,7 @@ def test_steps_and_buckets(structure, n):
 
 @gpu
 @pytest.mark.parametrize("dims", [1, 4, 5, 16, 17, 33, 65, 128])
-@pytest.mark.parametrize("structure", ["kd"])
+@pytest.mark.parametrize("structure", ["kd", "ball"])
 def test_dims_seeds_and_resumption(structure, dims):
     """Learned seeds, good, and (margin forced low) too short for every query."""
     from cudaexactknn_gb300 import _lib, knn
@@ -162,7 +162,7 @@ def test_dims_seeds_and_resumption(structure, dims):
 
 
 @gpu
-@pytest.mark.parametrize("structure", ["kd"])
+@pytest.mark.parametrize("structure", ["kd", "ball"])
 def test_captured_queries(structure):
     """A first query inside a stream capture, before anything is built for the index, and a later one."""
     import torch
@@ -193,7 +193,8 @@ def test_batch_classes_take_a_warp_per_query():
     rng = np.random.default_rng(6)
     items, data = [], []
     for structure, dims, n, nq, k in [("kd", 3, 5, 3, 4), ("kd", 3, 40000, 1000, 4), ("kd", 3, 700, 1, 8), ("kd", 8, 3000, 90, 64),
-                                      ("kd", 20, 2000, 33, 100), ("kd", 2, 1, 2, 1)]:
+                                      ("kd", 20, 2000, 33, 100), ("kd", 2, 1, 2, 1), ("ball", 3, 40000, 1000, 4),
+                                      ("ball", 3, 9, 2, 8), ("ball", 16, 3000, 90, 64), ("ball", 100, 500, 33, 100)]:
         pts, qs = W.uniform(rng, n, dims), W.uniform(rng, nq, dims)
         data.append((pts, qs, k))
         items.append((gu.make_index(structure, pts, 1), gu.to_dev(qs), k, INF))
