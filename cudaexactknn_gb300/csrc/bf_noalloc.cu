@@ -55,25 +55,10 @@ int scratch_address(uint64_t** out) {
     return KNN_OK;
 }
 
-template <int DP, int KMAX>
+template <int DP, int KR>
 int run(const float* points, uint32_t n, uint32_t dims, const float* queries, uint32_t count, float max_d2,
         uint32_t k, int32_t* idx, float* dist, uint64_t* scratch, cudaStream_t s) {
-    constexpr int PS = (DP + 3) / 4 * 4;
-    constexpr uint32_t block = 128;
-    const uint32_t tile = std::max(32u, 8192u / PS);
-    const size_t smem = static_cast<size_t>(tile) * PS * sizeof(float);
-    auto kern = bf_knn_kernel<DP, KMAX, false, false, true>;
-    KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    int per_sm = 0;
-    KNN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
-    const uint32_t qblocks = ceil_div(count, block);
-    // As many point-range splits as fill the GPU about four times over, limited by the scratch.
-    const uint64_t want = 4ull * sm_count() * std::max(per_sm, 1);
-    uint32_t splits = static_cast<uint32_t>(std::min<uint64_t>(ceil_div(static_cast<uint32_t>(std::min<uint64_t>(want, 0xFFFFFFFFu)), qblocks), 0xFFFFu));
-    splits = std::min<uint64_t>(splits, kScratchKeys / (static_cast<uint64_t>(count) * k));
-    splits = std::max(2u, std::min(splits, ceil_div(n, tile)));
-    const uint32_t chunk = ceil_div(ceil_div(n, splits), tile) * tile;
-    splits = ceil_div(n, chunk);
+    const BfShape shape = bf_shape<DP, KR>(n, count, kScratchKeys / (static_cast<uint64_t>(count) * k));
     BfParams p{};
     p.points = points;
     p.n = n;
@@ -82,31 +67,19 @@ int run(const float* points, uint32_t n, uint32_t dims, const float* queries, ui
     p.nq = count;
     p.max_d2 = max_d2;
     p.k = k;
-    p.chunk = chunk;
-    p.tile = tile;
     p.out_idx = idx;
     p.out_dist = dist;
-    p.partial = splits > 1 ? scratch : nullptr;
-    kern<<<dim3(qblocks, splits), block, smem, s>>>(p);
-    KNN_LAUNCHED();
-    if (splits > 1) {
-        bf_merge_kernel<KMAX><<<ceil_div(count, 128), 128, 0, s>>>(scratch, splits, count, k, max_d2, nullptr, nullptr,
-                                                                    nullptr, idx, dist);
-        KNN_LAUNCHED();
-    }
-    return KNN_OK;
+    p.partial = scratch;
+    KNN_TRY((bf_launch<DP, KR, true>(p, shape, s)));
+    return shape.splits > 1 ? bf_launch_merge<KR>(p, shape.splits, s) : KNN_OK;
 }
 
 template <int DP>
 int run_k(const float* points, uint32_t n, uint32_t dims, const float* queries, uint32_t count, float max_d2,
           uint32_t k, int32_t* idx, float* dist, uint64_t* scratch, cudaStream_t s) {
-    switch (k_class(k)) {
-        case 8: return run<DP, 8>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
-        case 16: return run<DP, 16>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
-        case 32: return run<DP, 32>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
-        case 64: return run<DP, 64>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
-        default: return run<DP, 128>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
-    }
+    if (k <= 32) return run<DP, 1>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
+    if (k <= 64) return run<DP, 2>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
+    return run<DP, 4>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
 }
 
 }  // namespace

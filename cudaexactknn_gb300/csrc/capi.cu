@@ -374,10 +374,18 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
                 p.bf16 = true;
                 if ((rc = consider(p)) != KNN_OK) break;
             }
+            // More or fewer warps sharing each query's points (see bf_shape).
+            for (uint32_t warps : {16u, 64u}) {
+                if (best.bf16) break;
+                knn::QueryPlan p = best;
+                p.bf_warps = warps;
+                if ((rc = consider(p)) != KNN_OK) break;
+            }
+            break;
         }
         const knn::QueryPlan stage2 = best;
         // Kernels of fixed shape: the filter, and the trees' warp-per-query search.
-        const bool fixed = stage2.bf16 || (ix->structure != KNN_BRUTE_FORCE && !stage2.warp);
+        const bool fixed = stage2.bf16 || !stage2.warp;
         for (uint32_t block : {32u, 64u, 256u}) {
             if (fixed) break;
             knn::QueryPlan p = stage2;
@@ -391,7 +399,6 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             p.heap = v & 1;
             p.sh_nn = (v >> 1) & 1;
             p.sh_stack = (v >> 2) & 1;
-            if (ix->structure == KNN_BRUTE_FORCE && p.sh_stack) continue;
             if ((rc = consider(p)) != KNN_OK) break;
         }
     } while (false);

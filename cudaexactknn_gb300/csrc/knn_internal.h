@@ -169,6 +169,7 @@ struct QueryPlan {
     bool bf16 = false;       // brute force: BF16 tensor-core filter + FP32 rescoring
     uint32_t tc_cap = 0;     // candidates kept per query by the filter (0 = default)
     uint32_t leaf_scan = 0;  // 0 = tree leaves
+    uint32_t bf_warps = 0;   // brute force: warps per SM the points are shared out over (0 = 32)
     bool test_give_up = false;  // tensor-core filter blocks give up after their first copy (tests)
 };
 

@@ -138,6 +138,11 @@ struct WarpTopK {
         empty = false;
         refresh();
     }
+    __device__ __forceinline__ void emit_keys(uint64_t* __restrict__ out) const {
+#pragma unroll
+        for (int j = 0; j < KR; ++j)
+            if (32u * j + lane < k) out[32u * j + lane] = v[j];
+    }
     __device__ __forceinline__ void emit(int32_t* __restrict__ idx, float* __restrict__ dist) const {
 #pragma unroll
         for (int j = 0; j < KR; ++j) {

@@ -115,7 +115,8 @@ typedef struct knn_query_opts {
                                that the first query builds (a thread per query, bounded by the
                                splitting planes, where they cannot be built: inside a stream
                                capture, or out of memory; the storage options above apply to that
-                               search), 1 = warp-coherent search (a warp's queries walk together);
+                               search and to traversal 1), ball trees always, over their balls;
+                               1 = warp-coherent search (a warp's queries walk together);
                                k-d trees of at most 16 dims, k <= 32: 2 = warp-group search (a
                                warp's 32 queries walk the tree once against the node boxes from
                                their own subtrees' radii and share out their (bucket, query) scans;
