@@ -74,94 +74,221 @@ __device__ __forceinline__ void encode(const float* __restrict__ prm, const Mode
 
 namespace {
 
-// Forward (and, with targets, backward) of one sample per thread.  Stores the activations and
-// the back-propagated deltas for the gradient reductions.
-__global__ void mlp_fwd_bwd_kernel(const float* __restrict__ prm, uint32_t dims, const float* __restrict__ x,
-                                   const float* __restrict__ target, const uint32_t* __restrict__ rows,
-                                   uint32_t batch, float* __restrict__ xn_out, float* __restrict__ h1_out,
-                                   float* __restrict__ h2_out, float* __restrict__ d1_out,
-                                   float* __restrict__ d2_out, float* __restrict__ dy_out,
-                                   float* __restrict__ loss_out) {
-    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= batch) return;
+// Forward and backward of a batch: 64 threads per sample, one per hidden unit (each its own fixed-order
+// sums), kFwdSamples samples per block, the weights staged in shared memory transposed (row stride 65:
+// no bank conflicts in either direction).  Stores the activations and the back-propagated deltas for the
+// gradient reductions.  A step of 1,024 samples (this kernel and the next) takes 35 us; a
+// thread per sample, 8 blocks of dependent global loads, and a thread per parameter reading the batch
+// from global memory took 0.30 ms.  Bound by the
+// latency of four chains of 64 to 67 fused multiply-adds.
+constexpr uint32_t kFwdSamples = 8;
+constexpr uint32_t kFwdPad = kHidden + 1;
+
+constexpr size_t fwd_smem(uint32_t feats) {
+    return 4ull * (feats * kFwdPad + kHidden * kFwdPad + kHidden + kFwdSamples * (feats + 3 * kHidden));
+}
+
+__device__ __forceinline__ void copy_async4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
+
+__global__ void __launch_bounds__(kFwdSamples * kHidden) mlp_fwd_bwd_kernel(
+    const float* __restrict__ prm, uint32_t dims, const float* __restrict__ x, const float* __restrict__ target,
+    const uint32_t* __restrict__ rows, uint32_t batch, float* __restrict__ xn_out, float* __restrict__ h1_out,
+    float* __restrict__ h2_out, float* __restrict__ d1_out, float* __restrict__ d2_out, float* __restrict__ dy_out,
+    float* __restrict__ loss_out) {
+    extern __shared__ float fsm[];
     const ModelLayout L(dims);
-    const uint32_t r = rows ? rows[b] : b;
-    float* xn = xn_out + static_cast<size_t>(b) * L.feats;  // the sample's features
-    encode(prm, L, x + static_cast<size_t>(r) * dims, xn);
-    float h1[kHidden], h2[kHidden];
-    for (uint32_t i = 0; i < kHidden; ++i) {
-        float a = prm[L.b1 + i];
-        for (uint32_t d = 0; d < L.feats; ++d) a = fmaf(prm[L.w1 + i * L.feats + d], xn[d], a);
-        h1[i] = fmaxf(a, 0.0f);
-        h1_out[static_cast<size_t>(b) * kHidden + i] = h1[i];
-    }
-    float y = prm[L.b3];
-    for (uint32_t i = 0; i < kHidden; ++i) {
-        float a = prm[L.b2 + i];
-        for (uint32_t j = 0; j < kHidden; ++j) a = fmaf(prm[L.w2 + i * kHidden + j], h1[j], a);
-        h2[i] = fmaxf(a, 0.0f);
-        h2_out[static_cast<size_t>(b) * kHidden + i] = h2[i];
-        y = fmaf(prm[L.w3 + i], h2[i], y);
-    }
-    // Mean squared error on the log distance: loss = mean (y - t)^2.
-    const float err = y - target[r];
-    const float dy = 2.0f * err / static_cast<float>(batch);
-    dy_out[b] = dy;
-    loss_out[b] = err * err / static_cast<float>(batch);
-    float d2[kHidden];
-    for (uint32_t i = 0; i < kHidden; ++i) {
-        d2[i] = h2[i] > 0.0f ? dy * prm[L.w3 + i] : 0.0f;
-        d2_out[static_cast<size_t>(b) * kHidden + i] = d2[i];
-    }
-    for (uint32_t j = 0; j < kHidden; ++j) {
+    float* w1t = fsm;                                // [feature][hidden]
+    float* w2t = w1t + L.feats * kFwdPad;            // [input][output]
+    float* w3 = w2t + kHidden * kFwdPad;
+    float* act = w3 + kHidden;                       // per sample: features, h1, h2, d2
+    const uint32_t i = threadIdx.x % kHidden, sample = threadIdx.x / kHidden;
+    const uint32_t b = blockIdx.x * kFwdSamples + sample;
+    const bool live = b < batch;
+    const uint32_t r = live ? (rows ? rows[b] : b) : 0u;
+    // (The copies are in flight while the features are computed.)
+    for (uint32_t e = threadIdx.x; e < kHidden * L.feats; e += blockDim.x)
+        copy_async4(w1t + (e % L.feats) * kFwdPad + e / L.feats, prm + L.w1 + e);
+    for (uint32_t e = threadIdx.x; e < kHidden * kHidden; e += blockDim.x)
+        copy_async4(w2t + (e % kHidden) * kFwdPad + e / kHidden, prm + L.w2 + e);
+    if (threadIdx.x < kHidden) copy_async4(w3 + threadIdx.x, prm + L.w3 + threadIdx.x);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    float* xn = act + sample * (L.feats + 3 * kHidden);
+    float *sh1 = xn + L.feats, *sh2 = sh1 + kHidden, *sd2 = sh2 + kHidden;
+    const float* xr = x + static_cast<size_t>(r) * dims;
+    if (live)
+        for (uint32_t d = i; d < dims; d += kHidden) xn[d] = (xr[d] - prm[L.lo + d]) * prm[L.inv_range + d];
+    __syncthreads();
+    if (live && i < kFourier) {
         float a = 0.0f;
-        for (uint32_t i = 0; i < kHidden; ++i) a = fmaf(prm[L.w2 + i * kHidden + j], d2[i], a);
-        d1_out[static_cast<size_t>(b) * kHidden + j] = h1[j] > 0.0f ? a : 0.0f;
+        for (uint32_t d = 0; d < dims; ++d) a = fmaf(xn[d], prm[L.proj + d * kFourier + i], a);
+        float sv, cv;
+        sincospif(2.0f * a, &sv, &cv);  // sin and cos of 2 pi a
+        xn[dims + i] = sv;
+        xn[dims + kFourier + i] = cv;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float h1 = 0.0f, h2 = 0.0f, dy = 0.0f;
+    if (live) {
+        for (uint32_t d = i; d < L.feats; d += kHidden) xn_out[static_cast<size_t>(b) * L.feats + d] = xn[d];
+        float a = prm[L.b1 + i];
+#pragma unroll 8
+        for (uint32_t d = 0; d < L.feats; ++d) a = fmaf(w1t[d * kFwdPad + i], xn[d], a);
+        h1 = fmaxf(a, 0.0f);
+        sh1[i] = h1;
+        h1_out[static_cast<size_t>(b) * kHidden + i] = h1;
+    }
+    __syncthreads();
+    if (live) {
+        float a = prm[L.b2 + i];
+#pragma unroll 8
+        for (uint32_t j = 0; j < kHidden; ++j) a = fmaf(w2t[j * kFwdPad + i], sh1[j], a);
+        h2 = fmaxf(a, 0.0f);
+        sh2[i] = h2;
+        h2_out[static_cast<size_t>(b) * kHidden + i] = h2;
+    }
+    __syncthreads();
+    if (live) {
+        float y = prm[L.b3];
+#pragma unroll 8
+        for (uint32_t j = 0; j < kHidden; ++j) y = fmaf(w3[j], sh2[j], y);
+        // Mean squared error on the log distance: loss = mean (y - t)^2.
+        const float err = y - target[r];
+        dy = 2.0f * err / static_cast<float>(batch);
+        if (i == 0) {
+            dy_out[b] = dy;
+            loss_out[b] = err * err / static_cast<float>(batch);
+        }
+        const float d2 = h2 > 0.0f ? dy * w3[i] : 0.0f;
+        sd2[i] = d2;
+        d2_out[static_cast<size_t>(b) * kHidden + i] = d2;
+    }
+    __syncthreads();
+    if (live) {
+        float a = 0.0f;
+#pragma unroll 8
+        for (uint32_t j = 0; j < kHidden; ++j) a = fmaf(w2t[i * kFwdPad + j], sd2[j], a);
+        d1_out[static_cast<size_t>(b) * kHidden + i] = h1 > 0.0f ? a : 0.0f;
     }
 }
 
-// One thread per trainable parameter: its gradient summed over the batch in sample order.
-__global__ void mlp_grad_kernel(uint32_t dims, uint32_t batch, const float* __restrict__ xn,
-                                const float* __restrict__ h1, const float* __restrict__ h2,
-                                const float* __restrict__ d1, const float* __restrict__ d2,
-                                const float* __restrict__ dy, float* __restrict__ grad) {
+// One step of Adam (Kingma & Ba, 2015) with bias correction.
+struct AdamStep {
+    float *prm, *m, *v;  // prm null: gradients only
+    float lr, beta1, beta2, eps, corr1, corr2;
+};
+
+// Every trainable parameter's gradient, summed over the batch in sample order by one thread, and Adam's
+// update of it.  A block takes kGradUnits units of a layer (threads: an input column each, with the units'
+// chains side by side, then the units' biases) or the output layer, and stages tiles of the batch in
+// shared memory (the layer's inputs and the units' deltas), two tiles ahead of the one that is
+// summed.  Bound by the chains of 1,024 fused multiply-adds.
+constexpr uint32_t kGradThreads = 256;
+constexpr uint32_t kGradTile = 64;   // samples per staged tile
+constexpr uint32_t kGradStages = 3;  // tiles in flight or being summed: one tile is summed faster than the next arrives
+constexpr uint32_t kGradUnits = 4;
+static_assert((kMaxDims + 2 * kFourier + 31) / 32 * 32 + kGradUnits <= kGradThreads, "a thread per input column and bias");
+
+constexpr size_t grad_smem(uint32_t feats) { return 4ull * kGradStages * kGradTile * (feats + kGradUnits); }
+constexpr uint32_t kGradBlocks = 2 * kHidden / kGradUnits + 1;
+
+__global__ void __launch_bounds__(kGradThreads) mlp_grad_kernel(uint32_t dims, uint32_t batch, const float* __restrict__ xn,
+                                                                const float* __restrict__ h1, const float* __restrict__ h2,
+                                                                const float* __restrict__ d1, const float* __restrict__ d2,
+                                                                const float* __restrict__ dy, float* __restrict__ grad,
+                                                                const AdamStep adam) {
+    extern __shared__ __align__(16) float gsm[];
     const ModelLayout L(dims);
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= L.trainable) return;
-    float g = 0.0f;
-    if (p < L.b1) {
-        const uint32_t i = p / L.feats, d = p % L.feats;
-        for (uint32_t b = 0; b < batch; ++b) g = fmaf(d1[b * kHidden + i], xn[b * L.feats + d], g);
-    } else if (p < L.w2) {
-        const uint32_t i = p - L.b1;
-        for (uint32_t b = 0; b < batch; ++b) g += d1[b * kHidden + i];
-    } else if (p < L.b2) {
-        const uint32_t i = (p - L.w2) / kHidden, j = (p - L.w2) % kHidden;
-        for (uint32_t b = 0; b < batch; ++b) g = fmaf(d2[b * kHidden + i], h1[b * kHidden + j], g);
-    } else if (p < L.w3) {
-        const uint32_t i = p - L.b2;
-        for (uint32_t b = 0; b < batch; ++b) g += d2[b * kHidden + i];
-    } else if (p < L.b3) {
-        const uint32_t j = p - L.w3;
-        for (uint32_t b = 0; b < batch; ++b) g = fmaf(dy[b], h2[b * kHidden + j], g);
-    } else {
-        for (uint32_t b = 0; b < batch; ++b) g += dy[b];
+    constexpr uint32_t U = kGradUnits;
+    const uint32_t layer = blockIdx.x / (kHidden / U), unit = blockIdx.x % (kHidden / U) * U;  // layer 2: the output
+    const uint32_t cols = layer == 0 ? L.feats : kHidden;                                      // the layer's inputs
+    const float* in = layer == 0 ? xn : layer == 1 ? h1 : h2;
+    const float* delta = layer == 0 ? d1 : d2;
+    const uint32_t c = threadIdx.x, tile_floats = kGradTile * (cols + U);
+    const uint32_t bias = c - (cols + 31) / 32 * 32;  // the units' biases, in a warp of their own (none: wraps)
+    float g[U] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto stage = [&](uint32_t t, uint32_t buf) {
+        const uint32_t rows = min(kGradTile, batch - t * kGradTile), n = rows * cols;
+        float* si = gsm + buf * tile_floats;
+        float* sd = si + kGradTile * cols;
+        const float* gi = in + static_cast<size_t>(t) * kGradTile * cols;  // 16-byte aligned: whole tiles before it
+        for (uint32_t k = 4 * c; k + 3 < n; k += 4 * kGradThreads) copy_async16(si + k, gi + k);
+        if (c < n % 4) copy_async4(si + n / 4 * 4 + c, gi + n / 4 * 4 + c);
+        if (c < rows) {
+            const size_t b = static_cast<size_t>(t) * kGradTile + c;
+            if (layer < 2) copy_async16(sd + c * U, delta + b * kHidden + unit);
+            else copy_async4(sd + c * U, dy + b);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto sum = [](uint32_t rows, auto&& left, auto&& right, auto&& add) {
+        uint32_t b = 0;
+        for (; b + 8 <= rows; b += 8) {
+            decltype(left(0u)) x[8];
+            decltype(right(0u)) d[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) {
+                x[k] = left(b + k);
+                d[k] = right(b + k);
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) add(x[k], d[k]);
+        }
+        for (; b < rows; ++b) add(left(b), right(b));
+    };
+    const uint32_t tiles = (batch + kGradTile - 1) / kGradTile;
+    static_assert(kGradStages == 3, "two tiles ahead");
+    stage(0, 0);
+    if (tiles > 1) stage(1, 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    for (uint32_t t = 0; t < tiles; ++t) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // tile t has landed for every thread, and tile t - 1 is read to the end
+        if (t + 2 < tiles) stage(t + 2, (t + 2) % kGradStages);
+        else asm volatile("cp.async.commit_group;" ::: "memory");  // (an empty group: the wait counts groups)
+        const uint32_t rows = min(kGradTile, batch - t * kGradTile);
+        const float* si = gsm + t % kGradStages * tile_floats;
+        const float* sd = si + kGradTile * cols;
+        // (Eight samples' values are read before they are summed, so that only the sums form a chain.)
+        if (c < cols && layer < 2) {
+            sum(rows, [&](uint32_t b) { return si[b * cols + c]; }, [&](uint32_t b) { return *reinterpret_cast<const float4*>(sd + b * U); },
+                [&](float x, const float4& d) {
+                    g[0] = fmaf(d.x, x, g[0]);
+                    g[1] = fmaf(d.y, x, g[1]);
+                    g[2] = fmaf(d.z, x, g[2]);
+                    g[3] = fmaf(d.w, x, g[3]);
+                });
+        } else if (c < cols) {
+            sum(rows, [&](uint32_t b) { return si[b * cols + c]; }, [&](uint32_t b) { return sd[b * U]; },
+                [&](float x, float d) { g[0] = fmaf(d, x, g[0]); });
+        } else if (bias < (layer < 2 ? U : 1u)) {
+            sum(rows, [&](uint32_t b) { return sd[b * U + bias]; }, [&](uint32_t) { return 0.0f; }, [&](float d, float) { g[0] += d; });
+        }
     }
-    grad[p] = g;
-}
-
-// Adam (Kingma & Ba, 2015) with bias correction.
-__global__ void adam_kernel(float* __restrict__ prm, const float* __restrict__ grad, float* __restrict__ m,
-                            float* __restrict__ v, uint32_t n, float lr, float beta1, float beta2, float eps,
-                            float corr1, float corr2) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const float g = grad[p];
-    const float mp = beta1 * m[p] + (1.0f - beta1) * g;
-    const float vp = beta2 * v[p] + (1.0f - beta2) * g * g;
-    m[p] = mp;
-    v[p] = vp;
-    prm[p] -= lr * (mp / corr1) / (sqrtf(vp / corr2) + eps);
+    auto update = [&](uint32_t p, float gp) {
+        if (grad) grad[p] = gp;
+        if (adam.prm) {
+            const float mp = adam.beta1 * adam.m[p] + (1.0f - adam.beta1) * gp;
+            const float vp = adam.beta2 * adam.v[p] + (1.0f - adam.beta2) * gp * gp;
+            adam.m[p] = mp;
+            adam.v[p] = vp;
+            adam.prm[p] -= adam.lr * (mp / adam.corr1) / (sqrtf(vp / adam.corr2) + adam.eps);
+        }
+    };
+    if (layer == 2) {
+        if (c < cols) update(L.w3 + c, g[0]);
+        else if (bias == 0) update(L.b3, g[0]);
+    } else if (c < cols) {
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) update((layer == 0 ? L.w1 : L.w2) + (unit + u) * cols + c, g[u]);
+    } else if (bias < U) {
+        update((layer == 0 ? L.b1 : L.b2) + unit + bias, g[0]);
+    }
 }
 
 // Seeded radius of each query, specialised on the padded input width: the parameters are
@@ -346,28 +473,37 @@ __global__ void kth_log_kernel(const float* __restrict__ dist, const int32_t* __
 
 size_t model_floats(uint32_t dims) { return ModelLayout(dims).total; }
 
-// Forward + backward for `batch` samples with the given parameters; writes gradients and the
-// summed loss (used by training and by the gradient check).
-int model_gradients(const float* d_prm, uint32_t dims, const float* d_x, const float* d_t, const uint32_t* d_rows,
-                    uint32_t batch, float* d_grad, float* d_loss_rows, DevBuf& scratch, cudaStream_t s) {
-    const ModelLayout LL(dims);
-    const size_t need = carve_bytes({static_cast<size_t>(batch) * LL.feats * 4, static_cast<size_t>(batch) * kHidden * 4,
+// Forward + backward for `batch` samples with the given parameters: gradients (d_grad, may be null) and
+// per-sample losses, and with `adam` one step on the parameters (training; the gradient check has none).
+// d_prm and adam->prm are the same array: the second kernel, which updates it, does not read it.
+int gradients(const float* d_prm, uint32_t dims, const float* d_x, const float* d_t, const uint32_t* d_rows,
+              uint32_t batch, float* d_grad, float* d_loss_rows, const AdamStep& adam, DevBuf& scratch, cudaStream_t s) {
+    const ModelLayout L(dims);
+    const size_t need = carve_bytes({static_cast<size_t>(batch) * L.feats * 4, static_cast<size_t>(batch) * kHidden * 4,
                                      static_cast<size_t>(batch) * kHidden * 4, static_cast<size_t>(batch) * kHidden * 4,
                                      static_cast<size_t>(batch) * kHidden * 4, static_cast<size_t>(batch) * 4});
     KNN_TRY(scratch.reserve(need));
     Carver c(scratch.ptr);
-    float* xn = c.take<float>(static_cast<size_t>(batch) * LL.feats);
+    float* xn = c.take<float>(static_cast<size_t>(batch) * L.feats);
     float* h1 = c.take<float>(static_cast<size_t>(batch) * kHidden);
     float* h2 = c.take<float>(static_cast<size_t>(batch) * kHidden);
     float* d1 = c.take<float>(static_cast<size_t>(batch) * kHidden);
     float* d2 = c.take<float>(static_cast<size_t>(batch) * kHidden);
     float* dy = c.take<float>(batch);
-    mlp_fwd_bwd_kernel<<<ceil_div(batch, 128), 128, 0, s>>>(d_prm, dims, d_x, d_t, d_rows, batch, xn, h1, h2, d1,
-                                                            d2, dy, d_loss_rows);
-    const ModelLayout L(dims);
-    mlp_grad_kernel<<<ceil_div(L.trainable, 128), 128, 0, s>>>(dims, batch, xn, h1, h2, d1, d2, dy, d_grad);
+    const size_t fs = fwd_smem(L.feats), gs = grad_smem(L.feats);
+    KNN_TRY_CUDA(cudaFuncSetAttribute(mlp_fwd_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(fs)));
+    KNN_TRY_CUDA(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(gs)));
+    mlp_fwd_bwd_kernel<<<ceil_div(batch, kFwdSamples), kFwdSamples * kHidden, fs, s>>>(d_prm, dims, d_x, d_t, d_rows, batch, xn,
+                                                                                       h1, h2, d1, d2, dy, d_loss_rows);
+    mlp_grad_kernel<<<kGradBlocks, kGradThreads, gs, s>>>(
+        dims, batch, xn, h1, h2, d1, d2, dy, d_grad, adam);
     KNN_LAUNCHED_N(2);
     return KNN_OK;
+}
+
+int model_gradients(const float* d_prm, uint32_t dims, const float* d_x, const float* d_t, const uint32_t* d_rows,
+                    uint32_t batch, float* d_grad, float* d_loss_rows, DevBuf& scratch, cudaStream_t s) {
+    return gradients(d_prm, dims, d_x, d_t, d_rows, batch, d_grad, d_loss_rows, AdamStep{}, scratch, s);
 }
 
 // ---- inference on the tensor cores ----------------------------------------------------------------
@@ -624,14 +760,13 @@ int model_train(knn_index* ix, const float* d_samples, uint32_t count, uint32_t 
     const size_t ck = static_cast<size_t>(count) * k;
     const size_t pb = static_cast<size_t>(L.total) * 4;
     KNN_TRY(buf.alloc(carve_bytes({ck * 4, ck * 4, static_cast<size_t>(count) * 4, static_cast<size_t>(count) * 4,
-                                   pb, pb, pb, pb, static_cast<size_t>(o.batch) * 4})));
+                                   pb, pb, pb, static_cast<size_t>(o.batch) * 4})));
     Carver c(buf.ptr);
     int32_t* idx = c.take<int32_t>(ck);
     float* dist = c.take<float>(ck);
     float* target = c.take<float>(count);
     uint32_t* rows = c.take<uint32_t>(count);
     float* prm = c.take<float>(L.total);
-    float* grad = c.take<float>(L.total);
     float* m = c.take<float>(L.total);
     float* v = c.take<float>(L.total);
     float* loss_rows = c.take<float>(o.batch);
@@ -686,13 +821,11 @@ int model_train(knn_index* ix, const float* d_samples, uint32_t count, uint32_t 
     uint32_t offset = 0;
     for (uint32_t step = 0; step < o.steps; ++step) {
         if (offset + batch > count) offset = 0;
-        KNN_TRY(model_gradients(prm, dims, d_samples, target, rows + offset, batch, grad, loss_rows, scratch, s));
         c1 *= b1;
         c2 *= b2;
         const float lr = o.lr * 0.5f * (1.0f + std::cos(3.14159265f * static_cast<float>(step) / o.steps));
-        adam_kernel<<<ceil_div(L.trainable, 256), 256, 0, s>>>(prm, grad, m, v, L.trainable, lr, b1, b2, 1e-8f,
-                                                              1.0f - c1, 1.0f - c2);
-        KNN_LAUNCHED();
+        const AdamStep adam{prm, m, v, lr, b1, b2, 1e-8f, 1.0f - c1, 1.0f - c2};
+        KNN_TRY(gradients(prm, dims, d_samples, target, rows + offset, batch, nullptr, loss_rows, adam, scratch, s));
         offset += batch;
     }
     std::vector<float> hl(batch);
