@@ -65,6 +65,150 @@ __global__ void init_root_kernel(uint32_t* off, uint32_t* size, uint32_t n, uint
     if (p < count) node_of[p] = 0;
 }
 
+// ---- the lower levels: whole subtrees in shared memory -----------------------------------------------
+// Once a node holds at most `cap` points (4,096 up to 16 orders), one block takes it and splits it down to
+// the leaves: its segment of every order is read once, as local indices (16 bits) into its points, and
+// every further level partitions the orders in shared memory.  A level over all n points in global
+// memory took six launches and about 195 us at 4.19 M 3-d points, most of it streaming and gathering ids;
+// twelve of its 22 levels run here instead (see kd_build for the figures).  Bound by the barriers of two block scans a level.
+constexpr uint32_t kSubItems = 8;      // positions per thread
+constexpr uint32_t kSubCap = 4096;     // most points of a subtree
+
+struct SubtreeParams {
+    const uint32_t* ord[kMaxDims];  // the level's orders; ord[0] is rewritten in leaf order into out0
+    uint32_t orders;                // orders in use
+    uint32_t aux;                   // split dimension = depth % aux
+    uint32_t level, depth;          // the subtrees' roots, the leaves
+    uint32_t cap;
+    const uint32_t* off;            // per root: first position, points
+    const uint32_t* size;
+    const float* pts;
+    uint32_t dims;
+    uint32_t* local;                // per point: its index within its subtree (scratch)
+    float* split;
+    uint32_t* out0;
+    uint32_t* leaf_off;             // per leaf (leaf_size zero before the launch: an empty leaf is not written)
+    uint32_t* leaf_size;
+};
+
+inline size_t subtree_smem(uint32_t cap, uint32_t orders) {
+    return static_cast<size_t>(cap) * (2 * orders + 2 + 2 + 4 + 1) + 128;
+}
+
+__global__ void __launch_bounds__(kSubCap / kSubItems) kd_subtree_kernel(const SubtreeParams t) {
+    extern __shared__ __align__(16) unsigned char sub_smem[];
+    __shared__ uint32_t warp_sum[kSubCap / kSubItems / 32];
+    const uint32_t cap = t.cap, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    uint32_t* gid = reinterpret_cast<uint32_t*>(sub_smem);           // global id of each local index
+    uint16_t* ord = reinterpret_cast<uint16_t*>(gid + cap);          // [orders][cap]
+    uint16_t* next = ord + static_cast<size_t>(t.orders) * cap;
+    uint16_t* pre = next + cap;                                      // left flags before each position
+    uint8_t* right = reinterpret_cast<uint8_t*>(pre + cap);          // side of each local index
+    const uint32_t base = t.off[blockIdx.x], m = t.size[blockIdx.x];
+    for (uint32_t p = tid; p < m; p += blockDim.x) {
+        const uint32_t id = t.ord[0][base + p];
+        gid[p] = id;
+        t.local[id] = p;
+        ord[p] = static_cast<uint16_t>(p);
+    }
+    __threadfence();  // (they are read back past L1, below)
+    __syncthreads();
+    // (Past L1: a line there may hold another subtree's entries from before this block wrote its own.)
+    for (uint32_t a = 1; a < t.orders; ++a)
+        for (uint32_t p = tid; p < m; p += blockDim.x)
+            ord[a * cap + p] = static_cast<uint16_t>(__ldcg(t.local + t.ord[a][base + p]));
+    // This thread's positions and, for each, its node: first position, points, index within the level.
+    uint32_t off[kSubItems], size[kSubItems], node[kSubItems];
+    const uint32_t p0 = tid * kSubItems;
+#pragma unroll
+    for (uint32_t i = 0; i < kSubItems; ++i) {
+        off[i] = 0;
+        size[i] = m;
+        node[i] = blockIdx.x;
+    }
+    for (uint32_t d = t.level; d < t.depth; ++d) {
+        const uint32_t dim = d % t.aux;
+        const uint16_t* by = ord + static_cast<size_t>(dim) * cap;
+        __syncthreads();  // the orders are complete
+#pragma unroll
+        for (uint32_t i = 0; i < kSubItems; ++i) {
+            const uint32_t p = p0 + i;
+            if (p >= m) continue;
+            const uint32_t left = (size[i] + 1) / 2, id = by[p];
+            right[id] = p - off[i] >= left ? 1 : 0;
+            if (p - off[i] + 1 == left)
+                t.split[(1u << d) - 1u + node[i]] = t.pts[static_cast<size_t>(gid[id]) * t.dims + dim];
+        }
+        __syncthreads();
+        for (uint32_t a = 0; a < t.orders; ++a) {
+            // An order that no level below splits by is not needed (the first one: the leaves).
+            if (a == dim) continue;
+            uint32_t again = d + 1 + (a + t.aux - (d + 1) % t.aux) % t.aux;
+            if (a && again >= t.depth) continue;
+            uint16_t* o = ord + static_cast<size_t>(a) * cap;
+            uint32_t id[kSubItems], f = 0, c = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < kSubItems; ++i) {
+                const bool in = p0 + i < m;
+                id[i] = in ? o[p0 + i] : 0u;
+                const uint32_t l = in && right[id[i]] == 0 ? 1u : 0u;
+                f |= l << i;
+                c += l;
+            }
+            uint32_t incl = c;
+#pragma unroll
+            for (uint32_t s = 1; s < 32; s <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, s);
+                if (lane >= s) incl += v;
+            }
+            if (lane == 31) warp_sum[warp] = incl;
+            __syncthreads();
+            uint32_t run = incl - c;
+            for (uint32_t w = 0; w < warp; ++w) run += warp_sum[w];
+            uint32_t mine[kSubItems];
+#pragma unroll
+            for (uint32_t i = 0; i < kSubItems; ++i) {
+                mine[i] = run;
+                if (p0 + i < m) pre[p0 + i] = static_cast<uint16_t>(run);
+                run += f >> i & 1u;
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t i = 0; i < kSubItems; ++i) {
+                const uint32_t p = p0 + i;
+                if (p >= m) continue;
+                const uint32_t lr = mine[i] - pre[off[i]];  // left entries of its node before it
+                const uint32_t dst = f >> i & 1u ? off[i] + lr : off[i] + (size[i] + 1) / 2 + (p - off[i] - lr);
+                next[dst] = static_cast<uint16_t>(id[i]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t i = 0; i < kSubItems; ++i)
+                if (p0 + i < m) o[p0 + i] = next[p0 + i];
+            // (The next writes to warp_sum and pre come after a barrier that follows this copy.)
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kSubItems; ++i) {
+            const uint32_t left = (size[i] + 1) / 2;
+            const bool r = p0 + i - off[i] >= left;
+            off[i] += r ? left : 0u;
+            size[i] = r ? size[i] - left : left;
+            node[i] = 2 * node[i] + (r ? 1u : 0u);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < kSubItems; ++i) {
+        const uint32_t p = p0 + i;
+        if (p >= m) continue;
+        t.out0[base + p] = gid[ord[p]];
+        if (p == off[i]) {
+            t.leaf_off[node[i]] = base + p;
+            t.leaf_size[node[i]] = size[i];
+        }
+    }
+}
+
 }  // namespace
 
 // Leaf slot stride (floats) and position of the index within a slot.
@@ -86,18 +230,25 @@ int kd_build(knn_index* ix, const float* d_points, uint32_t, cudaStream_t s) {
     KNN_TRY(ix->leaf.alloc(sizeof(float) * static_cast<size_t>(leaves) * ix->leaf_slots * ix->leaf_stride));
     ix->device_bytes = ix->split.bytes + ix->leaf.bytes;
 
+    // Orders are needed for the dimensions that some level splits by (and the first, the leaves' order).
+    const uint32_t used = std::max(1u, std::min(A, nd));
     DevBuf scratch_buf;
-    KNN_TRY(scratch_buf.alloc(build::scratch_bytes(n, A, leaves)));
+    KNN_TRY(scratch_buf.alloc(build::scratch_bytes(n, used, leaves)));
     build::Scratch sc{};
-    build::carve_scratch(sc, scratch_buf.ptr, n, A, leaves);
+    build::carve_scratch(sc, scratch_buf.ptr, n, used, leaves);
 
-    for (uint32_t a = 0; a < A; ++a) KNN_TRY(build::sort_dimension(sc, d_points, n, ix->dims, a, a, s));
+    for (uint32_t a = 0; a < used; ++a) KNN_TRY(build::sort_dimension(sc, d_points, n, ix->dims, a, a, s));
 
     init_root_kernel<<<ceil_div(n, 256), 256, 0, s>>>(sc.off[0], sc.size[0], n, sc.node_of[0], n);
     KNN_LAUNCHED();
+    // Levels over all points until a node fits a block, then whole subtrees.
+    uint32_t cap = kSubCap;
+    while (cap * used > kSubCap * 16) cap /= 2;
+    uint32_t top = 0;
+    while (top < nd && (static_cast<uint64_t>(n) + (1u << top) - 1) >> top > cap) ++top;
     int cur = 0, tab = 0, nof = 0;
     std::vector<uint32_t> others;
-    for (uint32_t level = 0; level < nd; ++level) {
+    for (uint32_t level = 0; level < top; ++level) {
         const uint32_t count = 1u << level;
         const uint32_t dim = level % A;
         kd_split_kernel<<<ceil_div(n, 256), 256, 0, s>>>(sc.ord[cur][dim], d_points, n, ix->dims, dim,
@@ -105,7 +256,7 @@ int kd_build(knn_index* ix, const float* d_points, uint32_t, cudaStream_t s) {
                                                          ix->split.as<float>() + (count - 1), sc.side);
         KNN_LAUNCHED();
         others.clear();
-        for (uint32_t b = 0; b < A; ++b)
+        for (uint32_t b = 0; b < used; ++b)
             if (b != dim) others.push_back(b);
         KNN_TRY(build::partition_orders(sc, others.data(), static_cast<uint32_t>(others.size()), cur,
                                         sc.node_of[nof], sc.off[tab], sc.size[tab], n, s));
@@ -120,9 +271,35 @@ int kd_build(knn_index* ix, const float* d_points, uint32_t, cudaStream_t s) {
         tab ^= 1;
         nof ^= 1;
     }
+    const uint32_t* leaf_order = sc.ord[cur][0];
+    if (top < nd) {
+        SubtreeParams t{};
+        for (uint32_t a = 0; a < used; ++a) t.ord[a] = sc.ord[cur][a];
+        t.orders = used;
+        t.aux = A;
+        t.level = top;
+        t.depth = nd;
+        t.cap = cap;
+        t.off = sc.off[tab];
+        t.size = sc.size[tab];
+        t.pts = d_points;
+        t.dims = ix->dims;
+        t.local = sc.node_of[nof ^ 1];
+        t.split = ix->split.as<float>();
+        t.out0 = sc.ord[cur ^ 1][0];
+        t.leaf_off = sc.off[tab ^ 1];
+        t.leaf_size = sc.size[tab ^ 1];
+        KNN_TRY_CUDA(cudaMemsetAsync(t.leaf_size, 0, leaves * sizeof(uint32_t), s));
+        const size_t smem = subtree_smem(cap, used);
+        KNN_TRY_CUDA(cudaFuncSetAttribute(kd_subtree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        kd_subtree_kernel<<<1u << top, cap / kSubItems, smem, s>>>(t);
+        KNN_LAUNCHED();
+        leaf_order = t.out0;
+        tab ^= 1;
+    }
     const uint64_t total_slots = static_cast<uint64_t>(leaves) * ix->leaf_slots;
     write_leaves_kernel<<<static_cast<uint32_t>((total_slots + 255) / 256), 256, 0, s>>>(
-        sc.ord[cur][0], d_points, ix->dims, ix->leaf_slots, leaves, sc.off[tab], sc.size[tab], ix->leaf_stride,
+        leaf_order, d_points, ix->dims, ix->leaf_slots, leaves, sc.off[tab], sc.size[tab], ix->leaf_stride,
         ix->leaf_id_at, ix->leaf.as<float>());
     KNN_LAUNCHED();
     KNN_TRY_CUDA(cudaStreamSynchronize(s));  // scratch is freed on return
