@@ -70,7 +70,8 @@ __global__ void init_root_kernel(uint32_t* off, uint32_t* size, uint32_t n, uint
 // the leaves: its segment of every order is read once, as local indices (16 bits) into its points, and
 // every further level partitions the orders in shared memory.  A level over all n points in global
 // memory took six launches and about 195 us at 4.19 M 3-d points, most of it streaming and gathering ids;
-// twelve of its 22 levels run here instead (see kd_build for the figures).  Bound by the barriers of two block scans a level.
+// twelve of its 22 levels run here instead, in 470 us.
+// Bound by the barriers of two block scans a level.
 constexpr uint32_t kSubItems = 8;      // positions per thread
 constexpr uint32_t kSubCap = 4096;     // most points of a subtree
 
