@@ -1438,6 +1438,17 @@ __global__ void tc_place_kernel(const uint32_t* __restrict__ keys, const uint32_
     row_of[static_cast<size_t>(cell_tile[c]) * kTileN + (i - cell_start[c])] = vals[i];
 }
 
+// Landmark norms for the queries' assignment: +inf for cells of fewer than k points.  A query assigned to
+// such a cell starts without a bound, and a home range that leaves its own cluster made the whole block's
+// query tile scan every cell (128 dims, k 100: one such query in 65,536 took the filter from 2.7 to
+// 10 ms); the nearest landmark with k points of its own gives it a bound like its neighbours'.
+__global__ void tc_eligible_kernel(const float* __restrict__ lnorm, const uint32_t* __restrict__ cell_start, uint32_t cells,
+                                   uint32_t rows, uint32_t k, float* __restrict__ out) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= rows) return;
+    out[c] = c < cells && cell_start[c + 1] - cell_start[c] < k ? INFINITY : lnorm[c];
+}
+
 // Home range of each query tile: the cells of its (cell-sorted) queries, widened by whole
 // neighbouring cells until they hold at least `min_points` points; written as first tile, end
 // tile, first cell, last cell.
@@ -2424,6 +2435,8 @@ int tc_prepare(knn_index* ix, cudaStream_t s) {
             cell_tile[c + 1] = cell_tile[c] + ceil_div(cell_start[c + 1], kTileN);
             cell_start[c + 1] += cell_start[c];
         }
+        T.max_cell = 0;
+        for (uint32_t c = 0; c < cells; ++c) T.max_cell = std::max(T.max_cell, cell_start[c + 1] - cell_start[c]);
         const uint32_t prows = cell_tile[cells] * kTileN;
         KNN_TRY(T.cell_start.alloc((cells + 1) * 4ull));
         KNN_TRY(T.cell_tile.alloc((cells + 1) * 4ull));
@@ -2546,7 +2559,7 @@ int bf_tc_query(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, cudaSt
                                             qimg_bytes, qrows * 4ull, qtiles * 16ull,
                                             static_cast<size_t>(nq) * cap * 4, static_cast<size_t>(nq) * cap * 4,
                                             nq * 4ull, nq * 4ull, nq * 4ull, nq * 4ull, nq * 4ull,
-                                            exh_slots(nq) * a.k * 8, 256})));
+                                            exh_slots(nq) * a.k * 8, 256, kMaxCells * 4ull})));
     Carver c(ix->tc.ws.ptr);
     uint32_t* k0 = c.take<uint32_t>(nq);
     uint32_t* v0 = c.take<uint32_t>(nq);
@@ -2564,6 +2577,7 @@ int bf_tc_query(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, cudaSt
     float* seed = c.take<float>(nq);
     float* retry_r2 = c.take<float>(nq);
     uint64_t* xkeys = c.take<uint64_t>(exh_slots(nq) * a.k);
+    float* eligible = c.take<float>(kMaxCells);  // landmark layout: at most that many, whole tiles
     uint32_t* small = c.take<uint32_t>(64);  // [0] retry count, [1] error flag, [2] filter tile counter
     KNN_TRY_CUDA(cudaMemsetAsync(small, 0, 64 * sizeof(uint32_t), s));
 
@@ -2577,10 +2591,17 @@ int bf_tc_query(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, cudaSt
                                                             nullptr, nullptr, qrows, nullptr);
         KNN_LAUNCHED();
         if (H != 1 && H != 2) return fail(KNN_ERR_UNSUPPORTED, "landmark layout at %u dims", ix->dims);
+        const uint32_t lrows = ceil_div(T.cells, kTileN) * kTileN;
+        const float* lnorm = T.lnorm.as<float>();
+        if (T.max_cell >= a.k) {
+            tc_eligible_kernel<<<ceil_div(lrows, 256), 256, 0, s>>>(lnorm, T.cell_start.as<uint32_t>(), T.cells, lrows, a.k, eligible);
+            KNN_LAUNCHED();
+            lnorm = eligible;
+        }
         auto kern = H == 1 ? tc_assign_mma_kernel<1> : tc_assign_mma_kernel<2>;
         const size_t smem = assign_mma_smem(H);
         KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        kern<<<qtiles, 128, smem, s>>>(qimg, T.limg.as<uint8_t>(), T.lnorm.as<float>(), ceil_div(T.cells, kTileN),
+        kern<<<qtiles, 128, smem, s>>>(qimg, T.limg.as<uint8_t>(), lnorm, ceil_div(T.cells, kTileN),
                                        T.cells, T.f16 ? idesc_f16(kTileM, kTileN) : idesc_bf16(kTileM, kTileN), nq,
                                        a.order, a.count_dev, a.queries, ix->dims, T.land.as<float>(), T.ps,
                                        T.cell_far.as<float>(), T.cell_start.as<uint32_t>(), a.k, k0, v0, seed,

@@ -318,6 +318,7 @@ struct knn_index {
         bool tree = false;
         uint32_t bd = 0;
         uint32_t cells = 0, ptiles = 0, ctiles = 0, ps = 0;
+        uint32_t max_cell = 0;  // landmark layout: points of the largest cell
         bool f16 = true;
         float scale = 1.0f;   // power of two applied before rounding to FP16
         bool ready = false;   // built
