@@ -159,19 +159,22 @@ __global__ void __launch_bounds__(256) ball_knn_warp_kernel(const BallParams p) 
 // 32, on 262,144 points near a 4-d subspace of 16 dims: 4.2 ms (a thread per query with its stack and
 // top-k in local memory: 15.6; 4,000 uniform 32-d queries, k 64, on 30,000: 3.4 and 177).  Bound by the
 // L2 reads of balls and slots, about 10,000 rows of 80 bytes per query there.
-template <int DP>
+template <int DP, int NQ>
 struct BallWarpView {
     static constexpr bool kKeys = true;
     static constexpr bool kShared = DP > 32;  // wide queries are read from shared memory (broadcast)
     float q[kShared ? 1 : DP];
     const float4* sq;
     const float* ball;
-    uint32_t ball_stride;
+    uint32_t ball_stride, quads;  // quads: groups of four dimensions in use (NQ where known at compile time)
     float margin;
     __device__ __forceinline__ float dist2_to(const float* row, float* last) const {
         if constexpr (kShared) {
             *last = row[DP];
-            return dist2_shared<DP>(sq, reinterpret_cast<const float4*>(row));
+            return dist2_shared(sq, reinterpret_cast<const float4*>(row), quads);
+        } else if constexpr (DP == 16 || DP == 32) {
+            *last = row[DP];
+            return dist2_vec4<4 * NQ>(reinterpret_cast<const float(&)[4 * NQ]>(q), reinterpret_cast<const float4*>(row));
         } else {
             return centre_dist<DP>(q, row, last);
         }
@@ -197,10 +200,10 @@ struct BallWarpSmem {
 };
 
 // One warp's search of query qi within r2; its row goes to the query's result slots.
-template <int DP, int KR, bool SEEDED>
+template <int DP, int NQ, int KR, bool SEEDED>
 __device__ __forceinline__ void ball_warp_query(const BallParams& p, uint32_t qi, float r2, BallWarpSmem<DP>& sm) {
     const uint32_t lane = threadIdx.x & 31u;
-    BallWarpView<DP> view;
+    BallWarpView<DP, NQ> view;
     if constexpr (DP > 32) {
         stage_query<DP>(p.queries, p.dims, qi, lane, sm.q);
         view.sq = sm.q;
@@ -210,6 +213,7 @@ __device__ __forceinline__ void ball_warp_query(const BallParams& p, uint32_t qi
     view.ball = p.ball;
     view.ball_stride = p.ball_stride;
     view.margin = p.margin;
+    view.quads = (p.dims + 3) / 4;
     const WarpTree t{p.leaf, p.leaf_stride, p.leaf_slots << (p.node_depth - p.stop_depth), p.stop_depth};
     WarpTopK<KR> top;
     LocalCounters lc;
@@ -217,9 +221,9 @@ __device__ __forceinline__ void ball_warp_query(const BallParams& p, uint32_t qi
     top.init(p.k, r2, lane);
     if constexpr (SEEDED) {
         const float r = p.seeds[qi] * p.seed_scale;
-        missed = warp_search<BallWarpView<DP>, KR, true>(view, t, sm.rows, top, lc, r < r2 ? r : r2, r2);
+        missed = warp_search<BallWarpView<DP, NQ>, KR, true>(view, t, sm.rows, top, lc, r < r2 ? r : r2, r2);
     } else {
-        warp_search<BallWarpView<DP>, KR, false>(view, t, sm.rows, top, lc, r2, r2);
+        warp_search<BallWarpView<DP, NQ>, KR, false>(view, t, sm.rows, top, lc, r2, r2);
     }
     top.emit(p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
     if (p.counters && lane == 0) {
@@ -228,13 +232,13 @@ __device__ __forceinline__ void ball_warp_query(const BallParams& p, uint32_t qi
     }
 }
 
-template <int DP, int KR, bool SEEDED>
+template <int DP, int NQ, int KR, bool SEEDED>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) ball_warp_query_kernel(const BallParams p) {
     __shared__ BallWarpSmem<DP> sm[kWarpsPerBlock];
     const uint32_t w = threadIdx.x >> 5, t = blockIdx.x * kWarpsPerBlock + w;
     if (t >= (p.count_dev ? *p.count_dev : p.nq)) return;  // no block-wide barriers
     const uint32_t qi = p.order ? p.order[t] : t;
-    ball_warp_query<DP, KR, SEEDED>(p, qi, p.radii ? p.radii[qi] : p.max_d2, sm[w]);
+    ball_warp_query<DP, NQ, KR, SEEDED>(p, qi, p.radii ? p.radii[qi] : p.max_d2, sm[w]);
 }
 
 // Sort key of a query: the node reached after `levels` steps towards the nearer child centre.
@@ -358,10 +362,13 @@ int ball_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan,
     const BallParams p = ball_params(ix, a, order, std::max(plan.leaf_scan, ball_warp_bucket(ix->dims)));
     const uint32_t grid = ceil_div(a.count, kWarpsPerBlock), threads = 32 * kWarpsPerBlock;
     void (*kern)(const BallParams) = nullptr;
-    if (p.seeds)
-        kern = a.k <= 32 ? ball_warp_query_kernel<DP, 1, true> : a.k <= 64 ? ball_warp_query_kernel<DP, 2, true> : ball_warp_query_kernel<DP, 4, true>;
-    else
-        kern = a.k <= 32 ? ball_warp_query_kernel<DP, 1, false> : a.k <= 64 ? ball_warp_query_kernel<DP, 2, false> : ball_warp_query_kernel<DP, 4, false>;
+    with_quads<DP>(ix->dims, [&](auto nq) {
+        constexpr int NQ = decltype(nq)::value;
+        if (p.seeds)
+            kern = a.k <= 32 ? ball_warp_query_kernel<DP, NQ, 1, true> : a.k <= 64 ? ball_warp_query_kernel<DP, NQ, 2, true> : ball_warp_query_kernel<DP, NQ, 4, true>;
+        else
+            kern = a.k <= 32 ? ball_warp_query_kernel<DP, NQ, 1, false> : a.k <= 64 ? ball_warp_query_kernel<DP, NQ, 2, false> : ball_warp_query_kernel<DP, NQ, 4, false>;
+    });
     if (plan.timing) KNN_TRY(ix->timing.begin(s));
     kern<<<grid, threads, 0, s>>>(p);
     KNN_LAUNCHED();
@@ -476,7 +483,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) ball_batch_warp_kernel(co
         const BallParams& p = sets[si].p;
         const uint32_t t = g - sets[si].query_offset;
         const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
-        ball_warp_query<DP, KR, false>(p, qi, p.max_d2, sm[threadIdx.x >> 5]);
+        ball_warp_query<DP, warp_quads(DP, DP), KR, false>(p, qi, p.max_d2, sm[threadIdx.x >> 5]);
         __syncwarp();
     }
 }

@@ -666,22 +666,26 @@ __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGrou
 // space between clusters).  10,000 uniform 11-d queries within a radius on 500,000 points: 2.0 ms
 // (28 and 145 ms).  Bound by the instructions of the top-k insertions and box tests at C2's shape,
 // by L2 reads of boxes and slots in more dimensions.
-template <int DP>
+template <int DP, int NQ>
 struct KdWarpView {
     static constexpr bool kKeys = false;      // the nearest box first
     static constexpr bool kShared = DP > 32;  // wide queries are read from shared memory (broadcast)
     float q[kShared ? 1 : DP];
     const float4* sq;
     const float* box;
-    uint32_t box_stride;
+    uint32_t box_stride, quads;  // quads: groups of four dimensions in use, NQ at most where that is known
+                                 // at compile time (the padding beyond adds exactly 0)
     __device__ __forceinline__ void test(uint32_t node, float* bound, uint32_t*) const {
         const float* b = box + static_cast<size_t>(node) * box_stride;
-        if constexpr (kShared) {
+        if constexpr (DP == 16 || DP == 32) {
+            const float4* lo4 = reinterpret_cast<const float4*>(b);
+            *bound = box_bound<4 * NQ>(reinterpret_cast<const float(&)[4 * NQ]>(q), lo4, lo4 + DP / 4, 0.0f);
+        } else if constexpr (kShared) {
             const float4* lo4 = reinterpret_cast<const float4*>(b);
             const float4* hi4 = reinterpret_cast<const float4*>(b + DP);
             float acc = 0.0f;
 #pragma unroll 4
-            for (int v = 0; v < DP / 4; ++v) {
+            for (uint32_t v = 0; v < quads; ++v) {
                 const float4 a = sq[v];
                 const float qq[4] = {a.x, a.y, a.z, a.w};
                 acc = box_bound<4>(qq, lo4 + v, hi4 + v, acc);
@@ -694,7 +698,10 @@ struct KdWarpView {
     __device__ __forceinline__ float dist(const float* slot, int32_t* id) const {
         if constexpr (kShared) {
             *id = __float_as_int(slot[DP]);
-            return dist2_shared<DP>(sq, reinterpret_cast<const float4*>(slot));
+            return dist2_shared(sq, reinterpret_cast<const float4*>(slot), quads);
+        } else if constexpr (DP == 16 || DP == 32) {
+            *id = __float_as_int(slot[DP]);
+            return dist2_vec4<4 * NQ>(reinterpret_cast<const float(&)[4 * NQ]>(q), reinterpret_cast<const float4*>(slot));
         } else {
             return slot_dist<DP>(q, slot, id);
         }
@@ -708,10 +715,10 @@ struct KdWarpSmem {
 };
 
 // One warp's search of query qi within r2; its row goes to the query's result slots.
-template <int DP, int KR, bool SEEDED>
+template <int DP, int NQ, int KR, bool SEEDED>
 __device__ __forceinline__ void kd_warp_query(const KdParams& p, uint32_t qi, float r2, KdWarpSmem<DP>& sm) {
     const uint32_t lane = threadIdx.x & 31u;
-    KdWarpView<DP> view;
+    KdWarpView<DP, NQ> view;
     if constexpr (DP > 32) {
         stage_query<DP>(p.queries, p.dims, qi, lane, sm.q);
         view.sq = sm.q;
@@ -720,6 +727,7 @@ __device__ __forceinline__ void kd_warp_query(const KdParams& p, uint32_t qi, fl
     }
     view.box = p.box;
     view.box_stride = p.box_stride;
+    view.quads = (p.dims + 3) / 4;
     const WarpTree t{p.leaf, p.leaf_stride, p.leaf_slots << (p.node_depth - p.stop_depth), p.stop_depth};
     WarpTopK<KR> top;
     LocalCounters lc;
@@ -727,9 +735,9 @@ __device__ __forceinline__ void kd_warp_query(const KdParams& p, uint32_t qi, fl
     top.init(p.k, r2, lane);
     if constexpr (SEEDED) {
         const float r = p.seeds[qi] * p.seed_scale;
-        missed = warp_search<KdWarpView<DP>, KR, true>(view, t, sm.rows, top, lc, r < r2 ? r : r2, r2);
+        missed = warp_search<KdWarpView<DP, NQ>, KR, true>(view, t, sm.rows, top, lc, r < r2 ? r : r2, r2);
     } else {
-        warp_search<KdWarpView<DP>, KR, false>(view, t, sm.rows, top, lc, r2, r2);
+        warp_search<KdWarpView<DP, NQ>, KR, false>(view, t, sm.rows, top, lc, r2, r2);
     }
     top.emit(p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
     if (p.counters && lane == 0) {
@@ -738,13 +746,13 @@ __device__ __forceinline__ void kd_warp_query(const KdParams& p, uint32_t qi, fl
     }
 }
 
-template <int DP, int KR, bool SEEDED>
+template <int DP, int NQ, int KR, bool SEEDED>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) kd_warp_query_kernel(const KdParams p) {
     __shared__ KdWarpSmem<DP> sm[kWarpsPerBlock];
     const uint32_t w = threadIdx.x >> 5, t = blockIdx.x * kWarpsPerBlock + w;
     if (t >= (p.count_dev ? *p.count_dev : p.nq)) return;  // no block-wide barriers
     const uint32_t qi = p.order ? p.order[t] : t;
-    kd_warp_query<DP, KR, SEEDED>(p, qi, p.radii ? p.radii[qi] : p.max_d2, sm[w]);
+    kd_warp_query<DP, NQ, KR, SEEDED>(p, qi, p.radii ? p.radii[qi] : p.max_d2, sm[w]);
 }
 
 // The group search's leftovers, each within its radius in `seeds`; warps stride over the list.
@@ -754,7 +762,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) kd_leftover_kernel(const 
     const uint32_t w = threadIdx.x >> 5, n = *gp.fb_count;
     for (uint32_t t = blockIdx.x * kWarpsPerBlock + w; t < n; t += gridDim.x * kWarpsPerBlock) {
         const uint32_t qi = gp.fb_list[t];
-        kd_warp_query<DP, 1, false>(gp.p, qi, gp.seeds[qi], sm[w]);
+        kd_warp_query<DP, warp_quads(DP, DP), 1, false>(gp.p, qi, gp.seeds[qi], sm[w]);
         __syncwarp();
     }
 }
@@ -945,10 +953,13 @@ int kd_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, c
     const KdParams p = kd_box_params(ix, a, order, std::max(plan.leaf_scan, kd_warp_bucket(ix->dims)));
     const uint32_t grid = ceil_div(a.count, kWarpsPerBlock), threads = 32 * kWarpsPerBlock;
     void (*kern)(const KdParams) = nullptr;
-    if (p.seeds)
-        kern = a.k <= 32 ? kd_warp_query_kernel<DP, 1, true> : a.k <= 64 ? kd_warp_query_kernel<DP, 2, true> : kd_warp_query_kernel<DP, 4, true>;
-    else
-        kern = a.k <= 32 ? kd_warp_query_kernel<DP, 1, false> : a.k <= 64 ? kd_warp_query_kernel<DP, 2, false> : kd_warp_query_kernel<DP, 4, false>;
+    with_quads<DP>(ix->dims, [&](auto nq) {
+        constexpr int NQ = decltype(nq)::value;
+        if (p.seeds)
+            kern = a.k <= 32 ? kd_warp_query_kernel<DP, NQ, 1, true> : a.k <= 64 ? kd_warp_query_kernel<DP, NQ, 2, true> : kd_warp_query_kernel<DP, NQ, 4, true>;
+        else
+            kern = a.k <= 32 ? kd_warp_query_kernel<DP, NQ, 1, false> : a.k <= 64 ? kd_warp_query_kernel<DP, NQ, 2, false> : kd_warp_query_kernel<DP, NQ, 4, false>;
+    });
     if (plan.timing) KNN_TRY(ix->timing.begin(s));
     kern<<<grid, threads, 0, s>>>(p);
     KNN_LAUNCHED();
@@ -1062,7 +1073,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) kd_batch_warp_kernel(cons
         const KdParams& p = sets[si].p;
         const uint32_t t = g - sets[si].query_offset;
         const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
-        kd_warp_query<DP, KR, false>(p, qi, p.max_d2, sm[threadIdx.x >> 5]);
+        kd_warp_query<DP, warp_quads(DP, DP), KR, false>(p, qi, p.max_d2, sm[threadIdx.x >> 5]);
         __syncwarp();
     }
 }

@@ -124,25 +124,24 @@ __device__ __forceinline__ void stage_query(const float* __restrict__ queries, u
     __syncwarp();
 }
 
-// dist2_vec4 with the query in shared memory: the same sequential fused sum.
-template <int DP>
-__device__ __forceinline__ float dist2_shared(const float4* sq, const float4* __restrict__ p4) {
+// dist2_vec4 over the first `quads` groups of four dimensions (those in use: the padding beyond adds
+// exactly 0), with the query in shared memory: the same sequential fused sum.
+__device__ __forceinline__ float dist2_quad(const float4& a, const float4& x, float acc) {
+    float t = __fsub_rn(a.x, x.x);
+    acc = __fmaf_rn(t, t, acc);
+    t = __fsub_rn(a.y, x.y);
+    acc = __fmaf_rn(t, t, acc);
+    t = __fsub_rn(a.z, x.z);
+    acc = __fmaf_rn(t, t, acc);
+    t = __fsub_rn(a.w, x.w);
+    return __fmaf_rn(t, t, acc);
+}
+__device__ __forceinline__ float dist2_shared(const float4* sq, const float4* __restrict__ p4, uint32_t quads) {
     float acc = 0.0f;
 #pragma unroll 8
-    for (int v = 0; v < DP / 4; ++v) {
-        const float4 a = sq[v], x = p4[v];
-        float t = __fsub_rn(a.x, x.x);
-        acc = __fmaf_rn(t, t, acc);
-        t = __fsub_rn(a.y, x.y);
-        acc = __fmaf_rn(t, t, acc);
-        t = __fsub_rn(a.z, x.z);
-        acc = __fmaf_rn(t, t, acc);
-        t = __fsub_rn(a.w, x.w);
-        acc = __fmaf_rn(t, t, acc);
-    }
+    for (uint32_t v = 0; v < quads; ++v) acc = dist2_quad(sq[v], p4[v], acc);
     return acc;
 }
-
 // Per-thread counters flushed once per thread (instrumented runs only).
 struct LocalCounters {
     uint32_t nodes = 0, leaves = 0, points = 0;
