@@ -509,13 +509,18 @@ int model_gradients(const float* d_prm, uint32_t dims, const float* d_x, const f
 // ---- inference on the tensor cores ----------------------------------------------------------------
 // Seeded radii for a query batch (the query path, and the training margin, so that the margin is
 // measured on the same predictions): per 128-query tile, each thread builds its query's features
-// (scaled coordinates, sin/cos of the Fourier projections), rounds them to FP16 and writes them to
-// shared memory as the A operand (K-major, 128-byte swizzle); the hidden layers are tcgen05 GEMMs
-// against W1 (64 x F) and W2 (64 x 64), packed to FP16 in shared memory once per block, with FP32
-// accumulation in TMEM (columns 0-63 and 64-127); bias, ReLU and the output layer run in the
-// epilogue.  The prediction only seeds a radius that the fallback rounds correct, so the 16-bit
-// rounding changes no answer.  Blocks loop over tiles; every wait is bounded and a timeout leaves
-// the caller's radius (the unseeded search) for the rest of the block's rows.
+// (sin/cos of the Fourier projections, then the scaled coordinates), rounds them to FP16 and writes
+// them to shared memory as the A operand (K-major, 128-byte swizzle); the hidden layers are tcgen05
+// GEMMs against W1 (64 x F, its columns in the same order) and W2 (64 x 64), packed to FP16 in shared
+// memory once per block, with FP32 accumulation in TMEM (columns 0-63 and 64-127); bias, ReLU and the
+// output layer run in the epilogue.  Bound by the issue of the features' instructions, so an operand
+// row is written 16 bytes at a time: sines and cosines come first because their chunks of eight then
+// start at multiples of eight for every dims (one conversion, one address and one conflict-free
+// store per chunk instead of per element), and the coordinates are padded with zeros only up to the
+// K step in use.  1,048,576 queries of 3 dims: 99 us (element stores and 128 zero-padded features:
+// 198).  The prediction only seeds a radius that the fallback rounds correct, so the 16-bit rounding
+// changes no answer.  Blocks loop over tiles; every wait is bounded and a timeout leaves the caller's
+// radius (the unseeded search) for the rest of the block's rows.
 constexpr uint32_t kMlpRows = 128;
 constexpr uint32_t kMlpFeatMax = 128;  // features per row this kernel takes (dims <= 64)
 
@@ -523,9 +528,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// FP16 element (row, k) of a K-major 128-byte-swizzled image with `rows` rows.
-__device__ __forceinline__ void put_half(uint8_t* img, uint32_t rows, uint32_t row, uint32_t k, float v) {
-    *reinterpret_cast<__half*>(img + tc::sw_offset(128, rows, row, k)) = __float2half_rn(fminf(fmaxf(v, -65504.0f), 65504.0f));
+// Eight FP16 elements (row, 8 c .. 8 c + 7) of a K-major 128-byte-swizzled image with `rows` rows.
+__device__ __forceinline__ void put_halves(uint8_t* img, uint32_t rows, uint32_t row, uint32_t c, const float (&v)[8]) {
+    __half2 h[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+        h[i] = __floats2half2_rn(fminf(fmaxf(v[2 * i], -65504.0f), 65504.0f), fminf(fmaxf(v[2 * i + 1], -65504.0f), 65504.0f));
+    uint4 w;
+    memcpy(&w, h, sizeof(w));
+    *reinterpret_cast<uint4*>(img + tc::sw_offset(128, rows, row, 8 * c)) = w;
 }
 
 __device__ __forceinline__ uint64_t mlp_desc(uint32_t base, uint32_t rows, uint32_t ks) {
@@ -542,22 +553,36 @@ __global__ void __launch_bounds__(kMlpRows, 1) mlp_infer_tc_kernel(const float* 
     const uint32_t raw_a = smem_addr(smem_raw);
     uint8_t* smem = smem_raw + (((raw_a + 1023u) & ~1023u) - raw_a);
     uint8_t* sA1 = smem;                        // [128 rows][128 features] FP16, two 64-element blocks
+    uint8_t* sA2 = sA1;                         // [128 rows][64 hidden], once the first layer has read sA1
     uint8_t* sW1 = sA1 + kMlpRows * 256;        // [64 hidden][128 features]
-    uint8_t* sA2 = sW1 + kHidden * 256;         // [128 rows][64 hidden], one block
-    uint8_t* sW2 = sA2 + kMlpRows * 128;        // [64][64]
+    uint8_t* sW2 = sW1 + kHidden * 256;         // [64][64]
     float* sb = reinterpret_cast<float*>(sW2 + kHidden * 128);  // b1[64], b2[64], w3[64]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sb + 3 * kHidden);
+    float* sP = sb + 3 * kHidden;                               // [32 projections][DP]
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sP + kFourier * DP);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const ModelLayout L(dims);
     const uint32_t t = threadIdx.x, warp = t / 32, lane = t % 32;
     // Weights to FP16 images (zero beyond the features), biases and the output layer.
-    for (uint32_t e = t; e < kHidden * kMlpFeatMax; e += kMlpRows) {
-        const uint32_t n = e / kMlpFeatMax, f = e % kMlpFeatMax;
-        put_half(sW1, kHidden, n, f, f < L.feats ? prm[L.w1 + n * L.feats + f] : 0.0f);
+    const uint32_t k1 = (L.feats + 15) / 16;
+    for (uint32_t e = t; e < kHidden * 2 * k1; e += kMlpRows) {
+        const uint32_t n = e / (2 * k1), c = e % (2 * k1);
+        float v[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+            const uint32_t f = 8 * c + i;
+            v[i] = f < L.feats ? prm[L.w1 + n * L.feats + (f < 2 * kFourier ? f + dims : f - 2 * kFourier)] : 0.0f;
+        }
+        put_halves(sW1, kHidden, n, c, v);
     }
-    for (uint32_t e = t; e < kHidden * kHidden; e += kMlpRows)
-        put_half(sW2, kHidden, e / kHidden, e % kHidden, prm[L.w2 + e]);
+    for (uint32_t e = t; e < kHidden * kHidden / 8; e += kMlpRows) {
+        float v[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) v[i] = prm[L.w2 + 8 * e + i];
+        put_halves(sW2, kHidden, e / (kHidden / 8), e % (kHidden / 8), v);
+    }
+    for (uint32_t e = t; e < kFourier * DP; e += kMlpRows)
+        sP[e] = e % DP < dims ? prm[L.proj + (e % DP) * kFourier + e / DP] : 0.0f;
     for (uint32_t e = t; e < kHidden; e += kMlpRows) {
         sb[e] = prm[L.b1 + e];
         sb[kHidden + e] = prm[L.b2 + e];
@@ -575,7 +600,6 @@ __global__ void __launch_bounds__(kMlpRows, 1) mlp_infer_tc_kernel(const float* 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t idesc = idesc_f16(kMlpRows, kHidden);
-    const uint32_t k1 = (L.feats + 15) / 16;
     const float b3 = prm[L.b3], margin = prm[L.margin];
     uint32_t phase = 0, commits = 0;  // commits: thread 0's count
     for (uint32_t tile = blockIdx.x; tile * kMlpRows < count; tile += gridDim.x) {
@@ -587,20 +611,35 @@ __global__ void __launch_bounds__(kMlpRows, 1) mlp_infer_tc_kernel(const float* 
         for (int d = 0; d < DP; ++d)
             z[d] = (live && static_cast<uint32_t>(d) < dims)
                        ? (x[static_cast<size_t>(q) * dims + d] - prm[L.lo + d]) * prm[L.inv_range + d] : 0.0f;
+        // (z and the projections are zero beyond dims, which adds nothing to a sum)
+#pragma unroll 1
+        for (uint32_t c = 0; c < kFourier / 8; ++c) {
+            float sv[8], cv[8];
 #pragma unroll
-        for (int d = 0; d < DP; ++d)
-            if (static_cast<uint32_t>(d) < dims) put_half(sA1, kMlpRows, t, d, z[d]);
-        for (uint32_t f = 0; f < kFourier; ++f) {
-            float a = 0.0f;
+            for (uint32_t i = 0; i < 8; ++i) {
+                const float4* p = reinterpret_cast<const float4*>(sP + (8 * c + i) * DP);
+                float a = 0.0f;
 #pragma unroll
-            for (int d = 0; d < DP; ++d)
-                if (static_cast<uint32_t>(d) < dims) a = fmaf(z[d], prm[L.proj + d * kFourier + f], a);
-            float sv, cv;
-            sincospif(2.0f * a, &sv, &cv);
-            put_half(sA1, kMlpRows, t, dims + f, sv);
-            put_half(sA1, kMlpRows, t, dims + kFourier + f, cv);
+                for (int d = 0; d < DP; d += 4) {
+                    const float4 w = p[d / 4];
+                    a = fmaf(z[d], w.x, a);
+                    a = fmaf(z[d + 1], w.y, a);
+                    a = fmaf(z[d + 2], w.z, a);
+                    a = fmaf(z[d + 3], w.w, a);
+                }
+                sincospif(2.0f * a, &sv[i], &cv[i]);
+            }
+            put_halves(sA1, kMlpRows, t, c, sv);
+            put_halves(sA1, kMlpRows, t, kFourier / 8 + c, cv);
         }
-        for (uint32_t f = L.feats; f < kMlpFeatMax; ++f) put_half(sA1, kMlpRows, t, f, 0.0f);
+        constexpr uint32_t kChunks = (DP + 7) / 8;
+#pragma unroll
+        for (uint32_t c = 0; c < (kChunks + 1) / 2 * 2; ++c) {
+            float v[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) v[i] = 8 * c + i < DP ? z[8 * c + i < DP ? 8 * c + i : 0] : 0.0f;
+            if (kFourier / 4 + c < 2 * k1) put_halves(sA1, kMlpRows, t, kFourier / 4 + c, v);
+        }
         fence_proxy_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -614,24 +653,24 @@ __global__ void __launch_bounds__(kMlpRows, 1) mlp_infer_tc_kernel(const float* 
         }
         bool ok = !*abort && mbar_wait(bar, phase, abort);
         phase ^= 1;
-        float h[kHidden];
         if (__all_sync(0xFFFFFFFFu, ok)) {
             tc_fence_after();
             float v[32];
-            tmem_ld32(tmem + ((warp * 32u) << 16), v);
 #pragma unroll
-            for (uint32_t i = 0; i < 32; ++i) h[i] = fmaxf(v[i] + sb[i], 0.0f);
-            tmem_ld32(tmem + ((warp * 32u) << 16) + 32, v);
+            for (uint32_t c = 0; c < 2; ++c) {
+                tmem_ld32(tmem + ((warp * 32u) << 16) + 32 * c, v);
 #pragma unroll
-            for (uint32_t i = 0; i < 32; ++i) h[32 + i] = fmaxf(v[i] + sb[32 + i], 0.0f);
+                for (uint32_t i = 0; i < 32; i += 8) {
+                    float h[8];
+#pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j) h[j] = fmaxf(v[i + j] + sb[32 * c + i + j], 0.0f);
+                    put_halves(sA2, kMlpRows, t, 4 * c + i / 8, h);
+                }
+            }
         } else {
-            ok = false;
+            ok = false;  // the second layer is not issued
             *abort = 1;
-#pragma unroll
-            for (uint32_t i = 0; i < kHidden; ++i) h[i] = 0.0f;
         }
-#pragma unroll
-        for (uint32_t i = 0; i < kHidden; ++i) put_half(sA2, kMlpRows, t, i, h[i]);
         fence_proxy_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -682,16 +721,18 @@ __global__ void __launch_bounds__(kMlpRows, 1) mlp_infer_tc_kernel(const float* 
     }
 }
 
-size_t mlp_tc_smem() { return 1024 + kMlpRows * 256 + kHidden * 256 + kMlpRows * 128 + kHidden * 128 + 3 * kHidden * 4 + 64; }
+size_t mlp_tc_smem(uint32_t dp) {
+    return 1024 + kMlpRows * 256 + kHidden * 256 + kHidden * 128 + (3 * kHidden + kFourier * dp) * sizeof(float) + 64;
+}
 
 int model_predict(const float* d_prm, uint32_t dims, const float* d_x, uint32_t count, float max_d2,
                   const float* user_radii, float* d_radii, float* d_raw, cudaStream_t s, bool tensor_cores) {
     const ModelLayout L(dims);
     if (tensor_cores && L.feats <= kMlpFeatMax && count > 0) {
-        const size_t smem = mlp_tc_smem();
         const uint32_t grid = std::min<uint32_t>(ceil_div(count, kMlpRows), 3u * static_cast<uint32_t>(sm_count()));
 #define KNN_INFER_TC(D_)                                                                                           \
         if (dims <= D_) {                                                                                          \
+            const size_t smem = mlp_tc_smem(D_);                                                                   \
             KNN_TRY_CUDA(cudaFuncSetAttribute(mlp_infer_tc_kernel<D_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                               static_cast<int>(smem)));                                            \
             mlp_infer_tc_kernel<D_><<<grid, kMlpRows, smem, s>>>(d_prm, dims, d_x, count, max_d2, user_radii,      \
