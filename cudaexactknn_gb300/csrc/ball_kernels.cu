@@ -156,9 +156,11 @@ __global__ void __launch_bounds__(256) ball_knn_warp_kernel(const BallParams p) 
 
 // One query per warp (warp_search.cuh) over the balls: a node's bound is its ball's, the visit order
 // the distance to the ball's border (overlapping balls have equal bounds of zero).  65,536 queries, k
-// 32, on 262,144 points near a 4-d subspace of 16 dims: 4.2 ms (a thread per query with its stack and
+// 32, on 262,144 points near a 4-d subspace of 16 dims: 3.7 ms (a thread per query with its stack and
 // top-k in local memory: 15.6; 4,000 uniform 32-d queries, k 64, on 30,000: 3.4 and 177).  Bound by the
-// L2 reads of balls and slots, about 10,000 rows of 80 bytes per query there.
+// L1 reads of balls and slots, about 10,000 rows of 80 bytes per query there: each lane reads its own
+// row, a line per lane and 16 bytes.  (Rows staged through shared memory by coalesced asynchronous
+// copies: 5.3 ms, as the staging takes the room in which L1 keeps the rows.)
 template <int DP, int NQ>
 struct BallWarpView {
     static constexpr bool kKeys = true;

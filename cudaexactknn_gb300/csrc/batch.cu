@@ -4,11 +4,12 @@
 // many small sets pays a launch and a device-wide sync per set.
 //
 // Here the items are grouped into classes of equal (tree, padded dims, k capacity).  Each class
-// runs as one persistent kernel whose blocks take work blocks (blockDim queries of one set) from a
-// shared counter, so small and large sets share the GPU within a single launch; the queries of a
-// class are first sorted together by (set, leaf they descend to) for locality.  The classes are
-// the parallel branches of one captured CUDA graph, replayed with one cudaGraphLaunch per run.
-// Plans (leaf bucket size, block size, per-thread or warp-coherent traversal) come from the
+// runs as one persistent kernel whose warps take queries (warp per query) or whose blocks take work
+// blocks (blockDim queries of one set) from a shared counter, so small and large sets share the GPU
+// within a single launch; where it pays, the queries of a class are first sorted together by (set,
+// leaf they descend to) for locality.  The classes are the parallel branches of one captured CUDA
+// graph, replayed with one cudaGraphLaunch per run.
+// Plans (leaf bucket size, block size, warp-per-query or warp-coherent traversal) come from the
 // autotuner, run on each class's largest set; with autotuning, a class of dims >= 16 whose largest
 // set answers faster through the tensor-core filter runs its items through the filter instead, one
 // after another on a branch of their own.
@@ -195,7 +196,8 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
             // faster per query on the class's largest set.  Both are first timed on a sample (the
             // filter on 8,192 queries, the tree's default search on 1,024: a whole set of
             // 32-dimensional uniform points takes seconds per tree search); a filter four times
-            // faster than that settles it, otherwise the tree is autotuned and compared again.
+            // faster than that settles it, otherwise the tree is autotuned and compared again (on more of
+            // a larger set: see finalist_count).
             bool tc_ok = it.index->dims >= 16;
             for (uint32_t i : c.items) tc_ok = tc_ok && knn::tc_supported(items[i].index->dims, items[i].k);
             float tc_per_q = 0.0f;
@@ -218,11 +220,20 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
                 if (tc_ok) {
                     knn::QueryArgs at = a;
                     at.count = std::min<uint32_t>(a.count, 8192u);
-                    float t_tree = 0.0f;
+                    float t_tree = 0.0f, t_tc = tc_per_q * at.count;
                     if ((rc = time_query([&] { return knn::query_structure(it.index, at, c.plan, s); }, s, &t_tree)) !=
                         KNN_OK)
                         break;
-                    c.tc = tc_per_q < t_tree / at.count;
+                    if (const uint32_t n = knn::finalist_count(a.count, at.count, std::max(t_tree, t_tc))) {
+                        knn::QueryPlan tp;
+                        tp.bf16 = true;
+                        at.count = n;
+                        if ((rc = time_query([&] { return knn::bf_tc_query(it.index, at, tp, s); }, s, &t_tc)) != KNN_OK) break;
+                        if ((rc = time_query([&] { return knn::query_structure(it.index, at, c.plan, s); }, s, &t_tree)) !=
+                            KNN_OK)
+                            break;
+                    }
+                    c.tc = t_tc < t_tree;
                 }
             }
         }

@@ -382,8 +382,8 @@ struct BfShape {
 // points.  Up to 4 dims the warps of a block share a group's points first: they share the bound and
 // need no second kernel.  Beyond, a block's warps take different queries wherever there are
 // enough of them, so that each staged tile serves 64, and a lane takes four rows for every read of
-// a query (shared memory returns 128 bytes a clock, broadcast or not: 128 dims, 2,048 queries on
-// 100,000 points, k 10).
+// a query (shared memory returns 128 bytes a clock, broadcast or not): 2,048 queries of 128 dims on
+// 100,000 points, k 10: 2.3 ms (3.4 with the block's warps on the same queries, one row a lane).
 template <int DP, int KR>
 BfShape bf_shape(uint32_t n, uint32_t count, uint64_t max_splits, uint32_t per_sm = 0) {
     const uint32_t query_groups = ceil_div(count, bf_queries(KR));

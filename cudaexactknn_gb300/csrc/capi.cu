@@ -154,7 +154,7 @@ int seeded_query(knn_index* ix, const knn::QueryArgs& a, const knn::QueryPlan& p
     if (ix->structure == KNN_KD_TREE && !plan.warp) KNN_TRY(knn::kd_boxes_ready(ix, s, &warp_query));
     if (warp_query) {
         // The warp-per-query search starts each query from its seed and, where that held fewer than k
-        // points, searches it again within the caller's radius, all in one launch.  The seeds may be
+        // points, goes on within the caller's radius, all in one launch.  The seeds may be
         // widened by a factor exp(widen * margin / 2) that the autotuner picks (traversal 2).
         KNN_TRY(ix->seed_ws.reserve(n * sizeof(float)));
         float* radii = ix->seed_ws.as<float>();
@@ -215,16 +215,18 @@ int k_slot(uint32_t k) {
 }
 
 // Picks the fastest plan for this index and k by timing candidates on up to 32768 of the
-// caller's queries (8192 for brute force; CUDA events, best of two runs after a warm-up), in
-// three stages: traversal (thread or warp) x leaf bucket size, or the tensor-core filter; then
-// block size; then tracker/stack storage.  Results are exact for every candidate.
+// caller's queries (131,072 for k-d trees, 8192 for brute force; CUDA events, best of two runs after a
+// warm-up): the tensor-core filter (against the best of the others once more on the whole batch); for trees the learned seeds' widening and bucket sizes, then
+// traversal (a warp per query, or warp-coherent) x leaf bucket size, and for the warp-coherent one
+// block size and tracker/stack storage; for brute force the warps that share a query's points.
+// Results are exact for every candidate.
 int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t s, knn::QueryPlan* out,
              float* best_ms, uint32_t* tried, bool allow_tc = true) {
     const knn::Range range("autotune");
     knn::QueryArgs t = a;
     // Brute force costs n distances per query; a smaller sample keeps tuning short.  k-d trees
-    // take up to 131,072 queries: the warp-group search needs enough warps to fill the GPU before
-    // its time per query means what it will mean on a large batch.
+    // take up to 131,072 queries: their searches are fast enough that fewer time the launch more
+    // than the search.
     t.count = std::min<uint32_t>(a.count, ix->structure == KNN_BRUTE_FORCE ? 8192u
                                           : ix->structure == KNN_KD_TREE ? 131072u : 32768u);
     t.counters = nullptr;
@@ -257,9 +259,9 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
         t.count = std::max(1024u, std::min(t.count, fit & ~127u));
     }
     // k-d trees: the batch's first queries are a sparser set than the batch (fewer queries per
-    // region of space), which misjudges the warp-group search, whose cost depends on how close a
-    // warp's queries are.  The sample is instead every s-th run of 32 queries of the batch's
-    // locality order (s = count / sample), gathered into scratch: each run is a warp's group as
+    // region of space), which misjudges searches whose cost depends on how close neighbouring
+    // queries are.  The sample is instead every s-th run of 32 queries of the batch's locality order
+    // (s = count / sample), gathered into scratch: each run is a warp's queries (warp-coherent) as
     // the real pass has it, and the runs cover the batch's whole extent.  Its rows are written to
     // the first rows of the caller's result buffers, which the real pass then overwrites.
     if (ix->structure == KNN_KD_TREE && a.count > t.count && !a.order && !a.count_dev) do {
@@ -286,6 +288,8 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
     knn::QueryPlan best;
     best.block = 128;
     float best_t = 1e30f;
+    knn::QueryPlan finalist[2];  // the fastest of the structure's own searches, and the filter
+    float finalist_t[2] = {1e30f, 1e30f};
     auto time_plan = [&](const knn::QueryPlan& p, float* ms) -> int {
         float best_rep = 1e30f;
         for (int rep = 0; rep < 3; ++rep) {
@@ -297,8 +301,9 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             KNN_TRY_CUDA(cudaEventElapsedTime(&v, e0, e1));
             if (rep > 0) best_rep = std::min(best_rep, v);  // the first run warms caches and workspaces
             // A candidate whose first run already takes 4x the best plan's time cannot win: its
-            // warm runs are skipped (in 32-dimensional trees a run can take seconds).
-            if (rep == 0 && v > 4.0f * best_t) {
+            // warm runs are skipped (in 32-dimensional trees a run can take seconds).  The filter's
+            // first run also lays the index out, so its second one tells.
+            if (rep == (p.bf16 ? 1 : 0) && v > 4.0f * best_t) {
                 best_rep = v;
                 break;
             }
@@ -315,6 +320,10 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
         if (v < best_t) {
             best_t = v;
             best = p;
+        }
+        if (v < finalist_t[p.bf16]) {
+            finalist_t[p.bf16] = v;
+            finalist[p.bf16] = p;
         }
         return KNN_OK;
     };
@@ -339,7 +348,7 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
         if (learned && ix->structure != KNN_BRUTE_FORCE) {
             // And without them: a warp's search finds a radius nearly as good in its first bucket, so
             // where the model is not cheap against the search the seeds do not pay for it (4.19 M
-            // clustered 3-d points, 1,048,576 queries: 1.83 ms without, 2.0 with).
+            // clustered 3-d points, 1,048,576 queries: 1.76 ms without, 2.04 with).
             knn::QueryPlan p;
             p.block = 128;
             p.unseeded = true;
@@ -402,6 +411,25 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
             if ((rc = consider(p)) != KNN_OK) break;
         }
     } while (false);
+    // The filter's time per query falls with the batch (a tile of points serves every query near it),
+    // the trees' does not, so where both were timed on a sample they meet again on the batch.
+    const float slower = std::max(finalist_t[0], finalist_t[1]);
+    const uint32_t final_count = rc == KNN_OK && slower < 1e30f ? knn::finalist_count(a.count, t.count, slower) : 0;
+    if (final_count) {
+        t = a;
+        t.counters = nullptr;
+        t.count = final_count;
+        const knn::QueryPlan pair[2] = {finalist[0], finalist[1]}, on_sample = best;
+        const float sample_t = best_t;
+        best_t = 1e30f;
+        for (const auto& p : pair)
+            if ((rc = consider(p)) != KNN_OK) break;
+        if (rc == KNN_ERR_OUT_OF_MEMORY) {  // no room for a pass this size: the sample decides
+            rc = KNN_OK;
+            best = on_sample;
+            best_t = sample_t;
+        }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc != KNN_OK) return rc;

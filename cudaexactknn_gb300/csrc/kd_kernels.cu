@@ -660,10 +660,10 @@ __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGrou
 }
 
 // One query per warp (warp_search.cuh) against the tight node boxes: the default search, and the
-// group search's leftovers.  1,048,576 queries, k 16, on 4.19 M clustered 3-d points: 1.83 ms, 8.5
+// group search's leftovers.  1,048,576 queries, k 16, on 4.19 M clustered 3-d points: 1.76 ms, 8.5
 // boxes of 32 tested and 7.5 buckets of 32 slots scanned per query; a thread per query took 3.2 ms
 // over the same boxes and 38 to 60 ms with splitting planes only (their bound prunes little in the
-// space between clusters).  10,000 uniform 11-d queries within a radius on 500,000 points: 2.0 ms
+// space between clusters).  10,000 uniform 11-d queries within a radius on 500,000 points: 1.8 ms
 // (28 and 145 ms).  Bound by the instructions of the top-k insertions and box tests at C2's shape,
 // by L2 reads of boxes and slots in more dimensions.
 template <int DP, int NQ>
@@ -943,9 +943,9 @@ int kd_boxes(knn_index* ix, cudaStream_t s, bool* ready) {
     return rc == KNN_ERR_OUT_OF_MEMORY ? KNN_OK : rc;
 }
 
-// Bucket slots at least (plans may ask for more).  A warp scans 32 slots at once, and the fewer, larger buckets of 32 are
-// the cheapest in few dimensions (4.19 M 3-d points: 1.83 ms, 1.99 with 8); in more the boxes of
-// smaller ones prune more (11 dims: 1.92 ms with 16, 2.3 with 32).
+// Bucket slots at least (plans may ask for more).  A warp scans 32 slots at once, and the fewer, larger
+// buckets of 32 are the cheapest in few dimensions (4.19 M 3-d points: 1.76 ms, 8% more with 8); in more
+// the boxes of smaller ones prune more (11 dims: 1.8 ms with 16, a fifth more with 32).
 inline uint32_t kd_warp_bucket(uint32_t dims) { return dims <= 8 ? 32u : 16u; }
 
 template <uint32_t DP>

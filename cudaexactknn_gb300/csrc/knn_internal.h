@@ -122,6 +122,17 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(ptr); }
 };
 
+// Queries on which the tensor-core filter and a structure's own search are timed against each other
+// once more, after both took at most `slower_ms` on a sample: the batch, or what the slower of them does
+// in 64 ms; 0 where that is less than twice the sample.  (1,048,576 points near a 4-d subspace of 16
+// dims, 262,144 queries, k 32: the ball tree was chosen on 32,768 queries and takes 26 ms on the
+// batch, the filter 15.)
+inline uint32_t finalist_count(uint32_t count, uint32_t sample, float slower_ms) {
+    const double fit = static_cast<double>(sample) * (64.0 / (slower_ms > 1e-3f ? slower_ms : 1e-3f));
+    const uint32_t n = fit < count ? static_cast<uint32_t>(fit) : count;
+    return n / 2 >= sample ? n : 0;
+}
+
 // Bump allocator over one device buffer (256-byte aligned carve-outs).
 struct Carver {
     char* base;
