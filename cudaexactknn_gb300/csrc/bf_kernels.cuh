@@ -81,18 +81,6 @@ struct BfSmem {
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
     return (static_cast<uint64_t>(__float_as_uint(b)) << 32) | __float_as_uint(a);
 }
-// Both halves by sub.rn / fma.rn, each rounded as the scalar instruction rounds it.
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t sqr_add2(uint64_t t, uint64_t acc) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(t), "l"(acc));
-    return d;
-}
-
 // The bounds of a query group, as they stand (other warps lower them).
 template <uint32_t Q>
 __device__ __forceinline__ void bf_bounds(const uint4* at, uint32_t (&out)[Q]) {

@@ -1326,88 +1326,76 @@ __global__ void tc_pack_kernel(const float* __restrict__ src, uint32_t src_strid
     if (ids) ids[r] = valid ? (src_ids ? src_ids[sr] : sr) : kNone;
 }
 
-// Nearest landmark (float distance, lowest index on ties) of each row; rows past the live count
-// get key `cells`.  keys/vals are indexed by row; vals = the source row.  With `cell_far` (per
-// cell: float squared distance from the landmark to its farthest point) and `cell_start`, also
-// writes seed[source row]: an upper bound on the float distance from the row to its k-th
-// nearest point, (|x - l| + r)^2 over the landmark's own cell when that holds >= k points, else
-// +inf (rounded up, margins g for the float distances and 2^-120 for subnormal ones).
+// Nearest landmark (float distance in any summation order, lowest index on ties) of each row: keys =
+// its index, vals = the row.  A warp has 32 rows; its four groups of eight lanes take a quarter of the
+// dimensions each, of four rows a lane, so that one read of a landmark from shared memory (16 bytes a
+// lane, 512 a warp whether they differ or not) feeds four rows, two dimensions per packed instruction.
+// The quarters are then summed across the groups, each lane ending with its own row.  1,048,576 rows
+// of 128 dims, an average of three rounds' landmarks: 10.5 ms, 12.1 with a row per lane and all its
+// dimensions, which was bound by those reads; the packed arithmetic of 8 warps per SM (183
+// registers) bounds it now.
 template <int DP>
 __global__ void __launch_bounds__(128) tc_assign_kernel(const float* __restrict__ src, uint32_t stride, uint32_t dims,
-                                                        uint32_t rows, const uint32_t* __restrict__ order,
-                                                        const uint32_t* __restrict__ live_count,
-                                                        const float* __restrict__ land, uint32_t ps, uint32_t cells,
-                                                        uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                                        const float* __restrict__ cell_far,
-                                                        const uint32_t* __restrict__ cell_start, uint32_t k,
-                                                        float* __restrict__ seed) {
-    constexpr uint32_t kChunk = 64;
-    __shared__ float sl[kChunk * DP];
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = r < rows && r < (live_count ? *live_count : rows);
-    const uint32_t row = live ? (order ? order[r] : r) : 0u;
-    float q[DP];
+                                                        uint32_t rows, const float* __restrict__ land, uint32_t ps,
+                                                        uint32_t cells, uint32_t* __restrict__ keys,
+                                                        uint32_t* __restrict__ vals) {
+    constexpr uint32_t kChunk = 64, kRows = 4, kQuarter = DP / 4;
+    __shared__ float4 sl[kChunk * DP / 4];
+    const uint32_t lane = threadIdx.x & 31u, part = lane >> 3, first = blockIdx.x * 128 + (threadIdx.x & ~31u);
+    uint64_t q[kRows][kQuarter / 2];
 #pragma unroll
-    for (int d = 0; d < DP; ++d) q[d] = (live && static_cast<uint32_t>(d) < dims) ? src[static_cast<size_t>(row) * stride + d] : 0.0f;
+    for (uint32_t r = 0; r < kRows; ++r) {
+        const uint32_t row = first + (lane & 7u) + 8 * r;
+        const float* x = src + static_cast<size_t>(min(row, rows - 1)) * stride;
+#pragma unroll
+        for (uint32_t d = 0; d < kQuarter; d += 2) {
+            const uint32_t at = part * kQuarter + d;
+            const float a = at < dims ? x[at] : 0.0f, b = at + 1 < dims ? x[at + 1] : 0.0f;
+            q[r][d / 2] = static_cast<uint64_t>(__float_as_uint(b)) << 32 | __float_as_uint(a);
+        }
+    }
     float best = INFINITY;
     uint32_t bi = 0;
     for (uint32_t c0 = 0; c0 < cells; c0 += kChunk) {
         __syncthreads();
-        for (uint32_t e = threadIdx.x; e < kChunk * DP; e += blockDim.x) {
-            const uint32_t j = e / DP, d = e % DP;
-            sl[e] = c0 + j < cells ? land[static_cast<size_t>(c0 + j) * ps + d] : 0.0f;
+        for (uint32_t e = threadIdx.x; e < kChunk * DP / 4; e += 128) {
+            const uint32_t j = c0 + e / (DP / 4);
+            sl[e] = j < cells ? reinterpret_cast<const float4*>(land + static_cast<size_t>(j) * ps)[e % (DP / 4)]
+                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
         __syncthreads();
         const uint32_t jn = min(kChunk, cells - c0);
-        // Two landmarks at a time, four partial sums each (the assignment may pick any landmark,
-        // and the seed's error margin holds for any summation order).
-        auto consider = [&](float acc, uint32_t j) {
-            if (acc < best) {
-                best = acc;
-                bi = c0 + j;
-            }
-        };
-        uint32_t j = 0;
-        for (; j + 1 < jn; j += 2) {
-            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f, b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f;
+        for (uint32_t j = 0; j < jn; ++j) {
+            const ulonglong2* l = reinterpret_cast<const ulonglong2*>(sl + j * (DP / 4) + part * (kQuarter / 4));
+            uint64_t acc[kRows] = {0, 0, 0, 0};
 #pragma unroll
-            for (int d = 0; d < DP; ++d) {
-                const float t = __fsub_rn(q[d], sl[j * DP + d]), u = __fsub_rn(q[d], sl[(j + 1) * DP + d]);
-                switch (d & 3) {
-                    case 0: a0 = __fmaf_rn(t, t, a0); b0 = __fmaf_rn(u, u, b0); break;
-                    case 1: a1 = __fmaf_rn(t, t, a1); b1 = __fmaf_rn(u, u, b1); break;
-                    case 2: a2 = __fmaf_rn(t, t, a2); b2 = __fmaf_rn(u, u, b2); break;
-                    default: a3 = __fmaf_rn(t, t, a3); b3 = __fmaf_rn(u, u, b3); break;
+            for (uint32_t d = 0; d < kQuarter / 4; ++d) {
+                const ulonglong2 v = l[d];
+#pragma unroll
+                for (uint32_t r = 0; r < kRows; ++r) {
+                    acc[r] = sqr_add2(sub2(q[r][2 * d], v.x), acc[r]);
+                    acc[r] = sqr_add2(sub2(q[r][2 * d + 1], v.y), acc[r]);
                 }
             }
-            consider((a0 + a1) + (a2 + a3), j);
-            consider((b0 + b1) + (b2 + b3), j + 1);
-        }
-        if (j < jn) {
-            float acc = 0.0f;
+            float a[kRows];
 #pragma unroll
-            for (int d = 0; d < DP; ++d) {
-                const float t = __fsub_rn(q[d], sl[j * DP + d]);
-                acc = __fmaf_rn(t, t, acc);
+            for (uint32_t r = 0; r < kRows; ++r)
+                a[r] = __uint_as_float(static_cast<uint32_t>(acc[r])) + __uint_as_float(static_cast<uint32_t>(acc[r] >> 32));
+            // Group p ends with rows 8 p ..: halves by bit 1 of the group, then by bit 0.
+            const bool hi = lane & 16u, lo = lane & 8u;
+            const float b0 = (hi ? a[2] : a[0]) + __shfl_xor_sync(0xFFFFFFFFu, hi ? a[0] : a[2], 16);
+            const float b1 = (hi ? a[3] : a[1]) + __shfl_xor_sync(0xFFFFFFFFu, hi ? a[1] : a[3], 16);
+            const float d2 = (lo ? b1 : b0) + __shfl_xor_sync(0xFFFFFFFFu, lo ? b0 : b1, 8);
+            if (d2 < best) {
+                best = d2;
+                bi = c0 + j;
             }
-            consider(acc, j);
         }
     }
-    if (r < rows) {
-        keys[r] = live ? bi : cells;
-        vals[r] = row;
-        if (seed && live) {
-            float t = INFINITY;
-            if (best <= FLT_MAX && cell_start[bi + 1] - cell_start[bi] >= k) {
-                const float g = rel_margin(dims);
-                const float inv = __frcp_ru(__fsub_rd(1.0f, g));  // >= 1 / (1 - g)
-                const float a = __fsqrt_ru(__fmul_ru(best, inv));  // >= exact |x - l|
-                const float b = __fsqrt_ru(__fmul_ru(cell_far[bi], inv));
-                // Plus 2^-120 for float distances whose terms fall in the subnormal range.
-                t = __fadd_ru(__fmul_ru(__fmul_ru(__fadd_ru(a, b), __fadd_ru(a, b)), __fadd_ru(1.0f, g)), 0x1p-120f);
-            }
-            seed[row] = t;
-        }
+    const uint32_t row = first + lane;
+    if (row < rows) {
+        keys[row] = bi;
+        vals[row] = row;
     }
 }
 
@@ -2059,22 +2047,14 @@ __global__ void __launch_bounds__(128, 1) tc_assign_mma_kernel(
 
 size_t assign_mma_smem(uint32_t H) { return 1024 + a_bytes(H) + 2 * b_bytes(H) + 2 * kTileN * 4 + 64; }
 
-int launch_assign(uint32_t dp, const float* src, uint32_t stride, uint32_t dims, uint32_t rows, const uint32_t* order,
-                  const uint32_t* live_count, const float* land, uint32_t ps, uint32_t cells, uint32_t* keys,
-                  uint32_t* vals, cudaStream_t s, const float* cell_far = nullptr, const uint32_t* cell_start = nullptr,
-                  uint32_t k = 0, float* seed = nullptr) {
+int launch_assign(uint32_t dp, const float* src, uint32_t stride, uint32_t dims, uint32_t rows, const float* land,
+                  uint32_t ps, uint32_t cells, uint32_t* keys, uint32_t* vals, cudaStream_t s) {
     const uint32_t grid = ceil_div(rows, 128);
-#define KNN_ASSIGN(D_)                                                                                         \
-    case D_:                                                                                                   \
-        tc_assign_kernel<D_><<<grid, 128, 0, s>>>(src, stride, dims, rows, order, live_count, land, ps, cells, \
-                                                   keys, vals, cell_far, cell_start, k, seed);                 \
-        break;
-    switch (dp) {
-        KNN_ASSIGN(1) KNN_ASSIGN(2) KNN_ASSIGN(3) KNN_ASSIGN(4) KNN_ASSIGN(8) KNN_ASSIGN(16) KNN_ASSIGN(32)
-        KNN_ASSIGN(64) KNN_ASSIGN(128)
-        default: return fail(KNN_ERR_UNSUPPORTED, "dims");
+    switch (dp) {  // the landmark layout's dims
+        case 64: tc_assign_kernel<64><<<grid, 128, 0, s>>>(src, stride, dims, rows, land, ps, cells, keys, vals); break;
+        case 128: tc_assign_kernel<128><<<grid, 128, 0, s>>>(src, stride, dims, rows, land, ps, cells, keys, vals); break;
+        default: return fail(KNN_ERR_UNSUPPORTED, "landmark layout of %u dims", dp);
     }
-#undef KNN_ASSIGN
     KNN_LAUNCHED();
     return KNN_OK;
 }
@@ -2346,7 +2326,7 @@ int tc_prepare(knn_index* ix, cudaStream_t s) {
             tc_gather_rows_kernel<<<ceil_div(cells * ps, 256), 256, 0, s>>>(src, stride, dims, lr, cells, ps,
                                                                            T.land.as<float>());
             KNN_LAUNCHED();
-            KNN_TRY(launch_assign(ix->dp, src, stride, dims, n, nullptr, nullptr, T.land.as<float>(), ps, cells, k0, v0, s));
+            KNN_TRY(launch_assign(ix->dp, src, stride, dims, n, T.land.as<float>(), ps, cells, k0, v0, s));
             KNN_TRY_CUDA(cudaStreamSynchronize(s));  // lrows is reused
             return KNN_OK;
         };

@@ -329,4 +329,16 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
     return pos;
 }
 
+// Two packed floats, both halves by sub.rn / fma.rn, each rounded as the scalar instruction rounds it.
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t sqr_add2(uint64_t t, uint64_t acc) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(t), "l"(acc));
+    return d;
+}
+
 }  // namespace knn
