@@ -867,27 +867,6 @@ __global__ void kd_box_up_kernel(float* __restrict__ box, uint32_t depth, uint32
     }
 }
 
-template <uint32_t DP>
-int kd_box_build_dp(knn_index* ix, cudaStream_t s) {
-    constexpr uint32_t QS = box_qs(DP), T = box_up_nodes(QS);
-    uint32_t depth = ix->kd_box_depth;
-    const size_t nodes = (static_cast<size_t>(2) << depth) - 1;
-    ix->kd_box_stride = 2 * QS;
-    KNN_TRY(ix->kd_box.alloc(nodes * ix->kd_box_stride * sizeof(float)));
-    kd_box_bottom_kernel<DP><<<ceil_div(1u << depth, 128), 128, 0, s>>>(
-        ix->leaf.as<float>(), ix->leaf_stride, depth, ix->node_depth, ix->node_count, ix->leaf_slots,
-        ix->kd_box.as<float>(), ix->kd_box_stride);
-    KNN_LAUNCHED();
-    while (depth) {
-        uint32_t levels = 0;
-        while (levels < depth && (2u << levels) <= T) ++levels;
-        kd_box_up_kernel<QS><<<ceil_div(1u << depth, T), T, 0, s>>>(ix->kd_box.as<float>(), depth, levels);
-        KNN_LAUNCHED();
-        depth -= levels;
-    }
-    return KNN_OK;
-}
-
 template <int DP, int KMAX>
 static int launch_kd_group(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
                            float* seeds, uint32_t* fb_list, uint32_t* fb_count, cudaStream_t s) {
@@ -921,12 +900,34 @@ static int launch_kd_group(knn_index* ix, const QueryArgs& a, const QueryPlan& p
 }
 
 // Builds the node boxes on first use, down to subtrees of at most 4 slots (16 slots beyond 16 dims,
-// where a box is as large as several slots).
+// where a box is as large as several slots).  The index holds them only once the device has finished
+// them: batch graphs, training and queries captured on other streams read them without waiting for the
+// stream of the query that built them, and a build that failed leaves none.  They are built on the
+// index's second stream, so that the host waits for the build alone, not for what the caller's stream
+// still has to do (the tree is complete since its creation).
 template <uint32_t DP>
-int kd_box_ensure(knn_index* ix, cudaStream_t s) {
+int kd_box_ensure(knn_index* ix) {
     if (ix->kd_box.ptr) return KNN_OK;
-    ix->kd_box_depth = scan_depth_for(ix->node_depth, ix->leaf_slots, DP <= 16 ? 4 : 16);
-    return kd_box_build_dp<DP>(ix, s);
+    constexpr uint32_t QS = box_qs(DP), T = box_up_nodes(QS), stride = 2 * QS;
+    const uint32_t bottom = scan_depth_for(ix->node_depth, ix->leaf_slots, DP <= 16 ? 4 : 16);
+    DevBuf buf;
+    KNN_TRY(buf.alloc(((static_cast<size_t>(2) << bottom) - 1) * stride * sizeof(float)));
+    KNN_TRY(ix->side.ensure());
+    const cudaStream_t s = ix->side.stream;
+    float* box = buf.as<float>();
+    kd_box_bottom_kernel<DP><<<ceil_div(1u << bottom, 128), 128, 0, s>>>(
+        ix->leaf.as<float>(), ix->leaf_stride, bottom, ix->node_depth, ix->node_count, ix->leaf_slots, box, stride);
+    KNN_LAUNCHED();
+    for (uint32_t depth = bottom, levels = 0; depth; depth -= levels) {
+        for (levels = 0; levels < depth && (2u << levels) <= T; ++levels) {}
+        kd_box_up_kernel<QS><<<ceil_div(1u << depth, T), T, 0, s>>>(box, depth, levels);
+        KNN_LAUNCHED();
+    }
+    KNN_TRY_CUDA(cudaStreamSynchronize(s));
+    ix->kd_box_depth = bottom;
+    ix->kd_box_stride = stride;
+    ix->kd_box.swap(buf);
+    return KNN_OK;
 }
 
 // The boxes for a search that can do without them: *ready is false where they are missing and cannot
@@ -938,7 +939,7 @@ int kd_boxes(knn_index* ix, cudaStream_t s, bool* ready) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     KNN_TRY_CUDA(cudaStreamIsCapturing(s, &cs));
     if (cs != cudaStreamCaptureStatusNone) return KNN_OK;
-    const int rc = kd_box_ensure<DP>(ix, s);
+    const int rc = kd_box_ensure<DP>(ix);
     *ready = rc == KNN_OK;
     return rc == KNN_ERR_OUT_OF_MEMORY ? KNN_OK : rc;
 }
@@ -975,7 +976,7 @@ int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, 
         return fail(KNN_ERR_INVALID_ARGUMENT, "group search: dims above 16");
     } else {
         if (a.k > 32) return fail(KNN_ERR_INVALID_ARGUMENT, "group search: k above 32");
-        KNN_TRY(kd_box_ensure<DP>(ix, s));
+        KNN_TRY(kd_box_ensure<DP>(ix));
         const size_t n = a.count;
         KNN_TRY(ix->group_ws.reserve(carve_bytes({n * 4, n * 4, 256})));
         Carver c(ix->group_ws.ptr);

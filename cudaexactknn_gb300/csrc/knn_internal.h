@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <initializer_list>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "../../include/cudaexactknn.h"
@@ -115,6 +116,10 @@ struct DevBuf {
         }
         bytes = n;
         return KNN_OK;
+    }
+    void swap(DevBuf& o) {
+        std::swap(ptr, o.ptr);
+        std::swap(bytes, o.bytes);
     }
     // Grow-only: keeps the current allocation when it is large enough.
     int reserve(size_t n) { return n <= bytes ? KNN_OK : alloc(n); }
@@ -251,8 +256,9 @@ struct StreamOrder {
     }
 };
 
-// A second stream of the index for work that can run beside the caller's stream within one
-// query (the radius model's seeds beside the locality sort), joined back through events.
+// A second stream of the index: for work that can run beside the caller's stream within one
+// query (the radius model's seeds beside the locality sort), joined back through events, and for the
+// k-d node boxes.
 struct SideStream {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -338,7 +344,7 @@ struct knn_index {
 
     // k-d tree: split value per internal node (implicit heap, children 2i+1, 2i+2).
     knn::DevBuf split;
-    // k-d tree (built on first use): the tight bounding box of the points under every node down to
+    // k-d tree (built on first use, complete on the device once held here): the tight bounding box of the points under every node down to
     // depth kd_box_depth (subtrees of at most 4 slots, 16 beyond 16 dims), per node lo[q], hi[q] with
     // q = max(4, padded dims) floats each; and the warp-group search's scratch.
     knn::DevBuf kd_box;
@@ -363,7 +369,7 @@ struct knn_index {
     knn::DevBuf workspace;
     knn::DevBuf staging;   // device copies of host queries/results (knn_query_host)
     knn::HostIo host_io;   // knn_query_host's copy streams
-    knn::SideStream side;  // the radius model's stream within a learned-radius query
+    knn::SideStream side;  // the radius model's stream within a learned-radius query; the k-d boxes' build
     knn::StreamOrder order_guard;
     knn::DevBuf counters;  // DevCounters
     knn::QueryTiming timing;
