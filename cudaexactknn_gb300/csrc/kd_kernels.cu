@@ -927,6 +927,7 @@ int kd_box_ensure(knn_index* ix) {
     ix->kd_box_depth = bottom;
     ix->kd_box_stride = stride;
     ix->kd_box.swap(buf);
+    ix->device_bytes += ix->kd_box.bytes;
     return KNN_OK;
 }
 

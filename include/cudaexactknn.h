@@ -150,7 +150,8 @@ typedef struct knn_index_info {
     uint32_t node_depth;  /* internal node levels */
     uint32_t leaf_slots;  /* 2^depth_skips */
     uint32_t node_count;  /* internal nodes, 2^node_depth - 1 */
-    uint64_t device_bytes;
+    uint64_t device_bytes; /* the index, and what its first queries built for it and keep: a k-d
+                              tree's node boxes, the tensor-core filter's layout */
     float build_ms;       /* device time of the construction, CUDA events */
     uint32_t radius_model;/* 1 when a learned radius model is attached */
 } knn_index_info;

@@ -112,3 +112,16 @@ def test_training_beside_the_first_query():
         torch.cuda.synchronize()
         ix.close()
     np.testing.assert_array_equal(models[0].view(np.uint32), models[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("dims,opts", [(3, {}), (3, {"traversal": 2}), (12, {}), (40, {})])
+def test_device_bytes_count_the_boxes(dims, opts):
+    pts, qs, want = _case(dims, n=5000, q=50)
+    ix = gu.make_index("kd", pts)
+    before = ix.info().device_bytes
+    gu.assert_rows_equal(*gu.run(ix, qs, 10, **opts), *want)
+    after = ix.info().device_bytes
+    assert after >= before + 2 * 4 * dims * (5000 // 32)  # two corners per 32 slots at least
+    gu.assert_rows_equal(*gu.run(ix, qs, 10, **opts), *want)
+    assert ix.info().device_bytes == after  # built once
+    ix.close()
