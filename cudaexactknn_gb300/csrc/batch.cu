@@ -251,8 +251,8 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
             continue;
         }
         if (!c.plan.warp) {
-            // A warp per query; k-d trees over each index's node boxes, built now (capture cannot
-            // allocate), or the per-thread search where there is no memory for them.
+            // A warp per query; k-d trees over each index's node boxes, or the per-thread search where
+            // there is no memory for them.
             c.plan.box = true;
             for (uint32_t i : c.items) {
                 if (c.structure != KNN_KD_TREE) break;

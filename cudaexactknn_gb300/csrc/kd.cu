@@ -20,7 +20,7 @@ int kd_query_dp(knn_index*, const QueryArgs&, const QueryPlan&, cudaStream_t);
 template <uint32_t DP>
 int kd_order_dp(knn_index*, const QueryArgs&, cudaStream_t, const uint32_t**, uint32_t);
 template <uint32_t DP>
-int kd_boxes(knn_index*, cudaStream_t, bool*);
+int kd_box_build_dp(const knn_index*, uint32_t, knn_index::KdBoxes*, cudaStream_t);
 
 namespace {
 
@@ -210,6 +210,28 @@ __global__ void __launch_bounds__(kSubCap / kSubItems) kd_subtree_kernel(const S
     }
 }
 
+int kd_box_build(const knn_index* ix, uint32_t bucket, knn_index::KdBoxes* boxes, cudaStream_t s) {
+    switch (ix->dp) {
+        case 1: return kd_box_build_dp<1>(ix, bucket, boxes, s);
+        case 2: return kd_box_build_dp<2>(ix, bucket, boxes, s);
+        case 3: return kd_box_build_dp<3>(ix, bucket, boxes, s);
+        case 4: return kd_box_build_dp<4>(ix, bucket, boxes, s);
+        case 8: return kd_box_build_dp<8>(ix, bucket, boxes, s);
+        case 16: return kd_box_build_dp<16>(ix, bucket, boxes, s);
+        case 32: return kd_box_build_dp<32>(ix, bucket, boxes, s);
+        case 64: return kd_box_build_dp<64>(ix, bucket, boxes, s);
+        case 128: return kd_box_build_dp<128>(ix, bucket, boxes, s);
+        default: return fail(KNN_ERR_UNSUPPORTED, "dims %u", ix->dims);
+    }
+}
+
+// The index takes boxes that the device has finished.
+void kd_box_hold(knn_index* ix, knn_index::KdBoxes& held, knn_index::KdBoxes& boxes) {
+    held.depth = boxes.depth;
+    held.buf.swap(boxes.buf);
+    ix->device_bytes += held.buf.bytes;
+}
+
 }  // namespace
 
 // Leaf slot stride (floats) and position of the index within a slot.
@@ -303,7 +325,13 @@ int kd_build(knn_index* ix, const float* d_points, uint32_t, cudaStream_t s) {
         leaf_order, d_points, ix->dims, ix->leaf_slots, leaves, sc.off[tab], sc.size[tab], ix->leaf_stride,
         ix->leaf_id_at, ix->leaf.as<float>());
     KNN_LAUNCHED();
+    // The node boxes are part of the tree: whatever searches it later, on any stream, finds them finished.
+    // Without memory for them the index is made all the same (the first query tries again).
+    knn_index::KdBoxes boxes;
+    const int rc = kd_box_build(ix, 0, &boxes, s);
+    if (rc != KNN_OK && rc != KNN_ERR_OUT_OF_MEMORY) return rc;
     KNN_TRY_CUDA(cudaStreamSynchronize(s));  // scratch is freed on return
+    if (rc == KNN_OK) kd_box_hold(ix, ix->kd_box, boxes);
     return KNN_OK;
 }
 
@@ -322,19 +350,27 @@ int kd_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t
     }
 }
 
+// Boxes built after the index was made.  It holds them only once the device has finished them: batch
+// graphs, training and captured queries read them without waiting for the stream of the query that
+// built them, and a build that failed leaves none.
+int kd_box_ensure(knn_index* ix, knn_index::KdBoxes& held, uint32_t bucket, cudaStream_t s) {
+    if (held.buf.ptr) return KNN_OK;
+    knn_index::KdBoxes boxes;
+    KNN_TRY(kd_box_build(ix, bucket, &boxes, s));
+    KNN_TRY_CUDA(cudaStreamSynchronize(s));
+    kd_box_hold(ix, held, boxes);
+    return KNN_OK;
+}
+
 int kd_boxes_ready(knn_index* ix, cudaStream_t s, bool* ready) {
-    switch (ix->dp) {
-        case 1: return kd_boxes<1>(ix, s, ready);
-        case 2: return kd_boxes<2>(ix, s, ready);
-        case 3: return kd_boxes<3>(ix, s, ready);
-        case 4: return kd_boxes<4>(ix, s, ready);
-        case 8: return kd_boxes<8>(ix, s, ready);
-        case 16: return kd_boxes<16>(ix, s, ready);
-        case 32: return kd_boxes<32>(ix, s, ready);
-        case 64: return kd_boxes<64>(ix, s, ready);
-        case 128: return kd_boxes<128>(ix, s, ready);
-        default: return fail(KNN_ERR_UNSUPPORTED, "dims %u", ix->dims);
-    }
+    *ready = ix->kd_box.buf.ptr != nullptr;
+    if (*ready) return KNN_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    KNN_TRY_CUDA(cudaStreamIsCapturing(s, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return KNN_OK;
+    const int rc = kd_box_ensure(ix, ix->kd_box, 0, s);
+    *ready = rc == KNN_OK;
+    return rc == KNN_ERR_OUT_OF_MEMORY ? KNN_OK : rc;
 }
 
 int kd_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order, uint32_t max_levels) {

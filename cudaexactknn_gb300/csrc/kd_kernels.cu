@@ -11,8 +11,8 @@
 //     point whose key could enter the top-k is skipped, ties included;
 //   * k-th key cached in a register; tracker/stack storage chosen by the plan.
 //
-// That per-thread search is what the engine runs where the tight node boxes are not to be had (a
-// query captured into a graph before any query built them, or no memory left for them).  Otherwise
+// That per-thread search is what the engine runs where the tight node boxes are not to be had (no
+// memory for them when the index was made, nor since).  Otherwise
 // each query gets a warp (kd_warp_query_kernel, warp_search.cuh), bounded by the boxes.
 
 #include <algorithm>
@@ -256,12 +256,16 @@ inline KdParams kd_params(const knn_index* ix, const QueryArgs& a, const uint32_
     return p;
 }
 
-// The same for a search over the node boxes.
-inline KdParams kd_box_params(const knn_index* ix, const QueryArgs& a, const uint32_t* order, uint32_t bucket) {
+// Floats per coordinate set of a node box.
+__host__ __device__ constexpr int box_qs(int dp) { return dp < 4 ? 4 : dp; }
+
+// The same for a search over node boxes.
+inline KdParams kd_box_params(const knn_index* ix, const knn_index::KdBoxes& boxes, const QueryArgs& a,
+                              const uint32_t* order, uint32_t bucket) {
     KdParams p = kd_params(ix, a, order, bucket);
-    p.stop_depth = std::min(p.stop_depth, ix->kd_box_depth);
-    p.box = ix->kd_box.as<float>();
-    p.box_stride = ix->kd_box_stride;
+    p.stop_depth = std::min(p.stop_depth, boxes.depth);
+    p.box = boxes.buf.as<float>();
+    p.box_stride = 2 * box_qs(static_cast<int>(ix->dp));
     return p;
 }
 
@@ -329,9 +333,6 @@ template <uint32_t DP>
 int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s);
 
 template <uint32_t DP>
-int kd_boxes(knn_index* ix, cudaStream_t s, bool* ready);
-
-template <uint32_t DP>
 int kd_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s);
 
 template <uint32_t DP>
@@ -344,7 +345,7 @@ int kd_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStrea
         const uint32_t block = p.block ? p.block : 128;
         const bool fits = tracker_smem_bytes(p.sh_nn, k_class(a.k), block) + stack_smem_bytes(p.sh_stack, block) <= kMaxBlockSmem;
         bool ready = false;
-        if (fits || p.box) KNN_TRY(kd_boxes<DP>(ix, s, &ready));
+        if (fits || p.box) KNN_TRY(kd_boxes_ready(ix, s, &ready));
         if (ready) {
             // Neighbouring queries share the boxes and slots they read only through the caches: an
             // order pays once the index outgrows L2 (16 M clustered 3-d points, 2 M queries: 3.74 ms
@@ -388,7 +389,6 @@ constexpr uint32_t kGroupStack = 96;  // node stack (at most 7 net entries per s
 constexpr uint32_t kGroupRounds = 6;  // radius growth rounds before a query is left over
 
 __host__ __device__ constexpr uint32_t group_cap(int kmax) { return kmax <= 8 ? 32u : (kmax <= 16 ? 48u : 80u); }
-__host__ __device__ constexpr int box_qs(int dp) { return dp < 4 ? 4 : dp; }
 
 template <int DP, int KMAX>
 struct GroupWarpSmem {
@@ -796,36 +796,74 @@ __global__ void __launch_bounds__(128) kd_self_seed_kernel(const KdParams p, uin
     seeds[qi] = tr.radius();  // the caller's radius while fewer than k points were offered
 }
 
-// Tight boxes of the nodes down to `depth` (per node lo[QS], hi[QS]; padding slots excluded).
+// Tight boxes of the nodes at `depth` (per node lo[QS], hi[QS]; padding slots excluded).  Up to 16 dims
+// min(32, slots) lanes share a node, a slot each at a time, and fold their corners by shuffles; beyond,
+// a warp goes through a node's slots with its lanes over the dimensions.  Either way neighbouring lanes
+// read neighbouring memory and no thread has more than a 32nd of a large node's slots or dimensions.
 template <int DP>
-__global__ void kd_box_bottom_kernel(const float* __restrict__ leaf, uint32_t leaf_stride, uint32_t depth,
-                                     uint32_t node_depth, uint32_t node_count, uint32_t leaf_slots,
-                                     float* __restrict__ box, uint32_t box_stride) {
+__global__ void __launch_bounds__(128) kd_box_bottom_kernel(const float* __restrict__ leaf, uint32_t leaf_stride,
+                                                            uint32_t depth, uint32_t slots, float* __restrict__ box) {
     constexpr int QS = box_qs(DP);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (1u << depth)) return;
-    const uint32_t node = (1u << depth) - 1u + i;
-    float lo[QS], hi[QS];
+    const uint32_t lanes = DP > 16 ? 32u : min(slots, 32u);  // powers of two
+    const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint32_t l = threadIdx.x & (lanes - 1u);
+    const uint64_t i = t / lanes;
+    const bool live = i < (1u << depth);
+    const float* slot = leaf + static_cast<size_t>(live ? i : 0) * slots * leaf_stride;
+    float* out = box + ((static_cast<size_t>(1) << depth) - 1 + i) * (2 * QS);
+    if constexpr (DP > 16) {
+        constexpr int N = DP / 32;
+        float lo[N], hi[N];
 #pragma unroll
-    for (int d = 0; d < QS; ++d) {
-        lo[d] = d < DP ? INFINITY : 0.0f;
-        hi[d] = d < DP ? -INFINITY : 0.0f;
-    }
-    const SlotRange sr = subtree_slots(node, depth, node_depth, node_count, leaf_slots);
-    const float* slot = leaf + sr.first * leaf_stride;
-    for (uint32_t s = 0; s < sr.count; ++s, slot += leaf_stride) {
-        if (__float_as_int(slot[DP]) < 0) continue;  // padding
+        for (int j = 0; j < N; ++j) {
+            lo[j] = INFINITY;
+            hi[j] = -INFINITY;
+        }
+        if (!live) return;
+#pragma unroll 4
+        for (uint32_t s = 0; s < slots; ++s, slot += leaf_stride) {
+            const bool point = __float_as_int(slot[DP]) >= 0;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const float x = slot[32 * j + l];
+                lo[j] = point ? fminf(lo[j], x) : lo[j];
+                hi[j] = point ? fmaxf(hi[j], x) : hi[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            out[32 * j + l] = lo[j];
+            out[QS + 32 * j + l] = hi[j];
+        }
+    } else {
+        float lo[DP], hi[DP];
 #pragma unroll
         for (int d = 0; d < DP; ++d) {
-            lo[d] = fminf(lo[d], slot[d]);
-            hi[d] = fmaxf(hi[d], slot[d]);
+            lo[d] = INFINITY;
+            hi[d] = -INFINITY;
         }
-    }
-    float* out = box + static_cast<size_t>(node) * box_stride;
+        for (uint32_t s = l; live && s < slots; s += lanes) {
+            const float* x = slot + static_cast<size_t>(s) * leaf_stride;
+            if (__float_as_int(x[DP]) < 0) continue;  // padding
 #pragma unroll
-    for (int d = 0; d < QS; ++d) {
-        out[d] = lo[d];
-        out[QS + d] = hi[d];
+            for (int d = 0; d < DP; ++d) {
+                lo[d] = fminf(lo[d], x[d]);
+                hi[d] = fmaxf(hi[d], x[d]);
+            }
+        }
+        for (uint32_t m = lanes / 2; m; m /= 2) {
+#pragma unroll
+            for (int d = 0; d < DP; ++d) {
+                lo[d] = fminf(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], m));
+                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], m));
+            }
+        }
+        if (!live || l) return;
+#pragma unroll
+        for (int d = 0; d < QS; ++d) {
+            out[d] = d < DP ? lo[d < DP ? d : 0] : 0.0f;
+            out[QS + d] = d < DP ? hi[d < DP ? d : 0] : 0.0f;
+        }
     }
 }
 
@@ -868,10 +906,10 @@ __global__ void kd_box_up_kernel(float* __restrict__ box, uint32_t depth, uint32
 }
 
 template <int DP, int KMAX>
-static int launch_kd_group(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
-                           float* seeds, uint32_t* fb_list, uint32_t* fb_count, cudaStream_t s) {
+static int launch_kd_group(knn_index* ix, const knn_index::KdBoxes& boxes, const QueryArgs& a, const QueryPlan& plan,
+                           const uint32_t* order, float* seeds, uint32_t* fb_list, uint32_t* fb_count, cudaStream_t s) {
     KdGroupParams gp{};
-    gp.p = kd_box_params(ix, a, order, plan.leaf_scan ? plan.leaf_scan : 8u);
+    gp.p = kd_box_params(ix, boxes, a, order, plan.leaf_scan ? plan.leaf_scan : 8u);
     gp.seeds = seeds;
     gp.fb_list = fb_list;
     gp.fb_count = fb_count;
@@ -899,60 +937,38 @@ static int launch_kd_group(knn_index* ix, const QueryArgs& a, const QueryPlan& p
     return KNN_OK;
 }
 
-// Builds the node boxes on first use, down to subtrees of at most 4 slots (16 slots beyond 16 dims,
-// where a box is as large as several slots).  The index holds them only once the device has finished
-// them: batch graphs, training and queries captured on other streams read them without waiting for the
-// stream of the query that built them, and a build that failed leaves none.  They are built on the
-// index's second stream, so that the host waits for the build alone, not for what the caller's stream
-// still has to do (the tree is complete since its creation).
+// Bucket slots at least (plans may ask for more).  A warp scans 32 slots at once, and the fewer, larger
+// buckets of 32 are the cheapest in few dimensions (4.19 M 3-d points: 1.76 ms, 8% more with 8); in more
+// the boxes of smaller ones prune more (11 dims: 1.8 ms with 16, a fifth more with 32).
+inline uint32_t kd_warp_bucket(uint32_t dims) { return dims <= 8 ? 32u : 16u; }
+
+// Enqueues the build of the node boxes down to subtrees of at most `bucket` slots (0: the default
+// search's) into boxes of their own.
 template <uint32_t DP>
-int kd_box_ensure(knn_index* ix) {
-    if (ix->kd_box.ptr) return KNN_OK;
-    constexpr uint32_t QS = box_qs(DP), T = box_up_nodes(QS), stride = 2 * QS;
-    const uint32_t bottom = scan_depth_for(ix->node_depth, ix->leaf_slots, DP <= 16 ? 4 : 16);
-    DevBuf buf;
-    KNN_TRY(buf.alloc(((static_cast<size_t>(2) << bottom) - 1) * stride * sizeof(float)));
-    KNN_TRY(ix->side.ensure());
-    const cudaStream_t s = ix->side.stream;
-    float* box = buf.as<float>();
-    kd_box_bottom_kernel<DP><<<ceil_div(1u << bottom, 128), 128, 0, s>>>(
-        ix->leaf.as<float>(), ix->leaf_stride, bottom, ix->node_depth, ix->node_count, ix->leaf_slots, box, stride);
+int kd_box_build_dp(const knn_index* ix, uint32_t bucket, knn_index::KdBoxes* boxes, cudaStream_t s) {
+    constexpr uint32_t QS = box_qs(DP), T = box_up_nodes(QS);
+    boxes->depth = scan_depth_for(ix->node_depth, ix->leaf_slots, bucket ? bucket : kd_warp_bucket(ix->dims));
+    // Leaves beyond 256 slots are read in parts, levels below the tree's that only this build knows: two
+    // leaves of 65,536 slots and 40 dims would take two warps 7 ms.
+    uint32_t bottom = boxes->depth, slots = ix->leaf_slots << (ix->node_depth - bottom);
+    for (; slots > 256; slots /= 2) ++bottom;
+    KNN_TRY(boxes->buf.alloc(((static_cast<size_t>(2) << bottom) - 1) * 2 * QS * sizeof(float)));
+    float* box = boxes->buf.as<float>();
+    const uint64_t threads = static_cast<uint64_t>(DP > 16 ? 32u : std::min(slots, 32u)) << bottom;
+    kd_box_bottom_kernel<DP><<<static_cast<uint32_t>((threads + 127) / 128), 128, 0, s>>>(
+        ix->leaf.as<float>(), ix->leaf_stride, bottom, slots, box);
     KNN_LAUNCHED();
     for (uint32_t depth = bottom, levels = 0; depth; depth -= levels) {
         for (levels = 0; levels < depth && (2u << levels) <= T; ++levels) {}
         kd_box_up_kernel<QS><<<ceil_div(1u << depth, T), T, 0, s>>>(box, depth, levels);
         KNN_LAUNCHED();
     }
-    KNN_TRY_CUDA(cudaStreamSynchronize(s));
-    ix->kd_box_depth = bottom;
-    ix->kd_box_stride = stride;
-    ix->kd_box.swap(buf);
-    ix->device_bytes += ix->kd_box.bytes;
     return KNN_OK;
 }
 
-// The boxes for a search that can do without them: *ready is false where they are missing and cannot
-// be built now (the stream is being captured, or no memory is left for them).
-template <uint32_t DP>
-int kd_boxes(knn_index* ix, cudaStream_t s, bool* ready) {
-    *ready = ix->kd_box.ptr != nullptr;
-    if (*ready) return KNN_OK;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    KNN_TRY_CUDA(cudaStreamIsCapturing(s, &cs));
-    if (cs != cudaStreamCaptureStatusNone) return KNN_OK;
-    const int rc = kd_box_ensure<DP>(ix);
-    *ready = rc == KNN_OK;
-    return rc == KNN_ERR_OUT_OF_MEMORY ? KNN_OK : rc;
-}
-
-// Bucket slots at least (plans may ask for more).  A warp scans 32 slots at once, and the fewer, larger
-// buckets of 32 are the cheapest in few dimensions (4.19 M 3-d points: 1.76 ms, 8% more with 8); in more
-// the boxes of smaller ones prune more (11 dims: 1.8 ms with 16, a fifth more with 32).
-inline uint32_t kd_warp_bucket(uint32_t dims) { return dims <= 8 ? 32u : 16u; }
-
 template <uint32_t DP>
 int kd_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s) {
-    const KdParams p = kd_box_params(ix, a, order, std::max(plan.leaf_scan, kd_warp_bucket(ix->dims)));
+    const KdParams p = kd_box_params(ix, ix->kd_box, a, order, std::max(plan.leaf_scan, kd_warp_bucket(ix->dims)));
     const uint32_t grid = ceil_div(a.count, kWarpsPerBlock), threads = 32 * kWarpsPerBlock;
     void (*kern)(const KdParams) = nullptr;
     with_quads<DP>(ix->dims, [&](auto nq) {
@@ -969,7 +985,7 @@ int kd_warp_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, c
     return KNN_OK;
 }
 
-// Warp-group search (plan.group) from each query's own subtree: boxes built on first use, the group
+// Warp-group search (plan.group) from each query's own subtree: its boxes built on first use, the group
 // kernel in the batch's locality order, then the leftovers.
 template <uint32_t DP>
 int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s) {
@@ -977,7 +993,10 @@ int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, 
         return fail(KNN_ERR_INVALID_ARGUMENT, "group search: dims above 16");
     } else {
         if (a.k > 32) return fail(KNN_ERR_INVALID_ARGUMENT, "group search: k above 32");
-        KNN_TRY(kd_box_ensure<DP>(ix));
+        // Boxes of subtrees of 4 slots, as its plans may scan; a tree whose leaves are as large as the
+        // default search's buckets has one set of boxes for both.
+        knn_index::KdBoxes& boxes = ix->leaf_slots >= kd_warp_bucket(ix->dims) ? ix->kd_box : ix->kd_fine_box;
+        KNN_TRY(kd_box_ensure(ix, boxes, 4, s));
         const size_t n = a.count;
         KNN_TRY(ix->group_ws.reserve(carve_bytes({n * 4, n * 4, 256})));
         Carver c(ix->group_ws.ptr);
@@ -985,15 +1004,15 @@ int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, 
         uint32_t* fb_list = c.take<uint32_t>(n);
         uint32_t* fb_count = c.take<uint32_t>(1);
         switch (k_class(a.k)) {
-            case 8: return launch_kd_group<DP, 8>(ix, a, plan, order, seeds, fb_list, fb_count, s);
-            case 16: return launch_kd_group<DP, 16>(ix, a, plan, order, seeds, fb_list, fb_count, s);
-            default: return launch_kd_group<DP, 32>(ix, a, plan, order, seeds, fb_list, fb_count, s);
+            case 8: return launch_kd_group<DP, 8>(ix, boxes, a, plan, order, seeds, fb_list, fb_count, s);
+            case 16: return launch_kd_group<DP, 16>(ix, boxes, a, plan, order, seeds, fb_list, fb_count, s);
+            default: return launch_kd_group<DP, 32>(ix, boxes, a, plan, order, seeds, fb_list, fb_count, s);
         }
     }
 }
 
 template int kd_query_dp<KNN_DP>(knn_index*, const QueryArgs&, const QueryPlan&, cudaStream_t);
-template int kd_boxes<KNN_DP>(knn_index*, cudaStream_t, bool*);
+template int kd_box_build_dp<KNN_DP>(const knn_index*, uint32_t, knn_index::KdBoxes*, cudaStream_t);
 template int kd_order_dp<KNN_DP>(knn_index*, const QueryArgs&, cudaStream_t, const uint32_t**, uint32_t);
 
 
@@ -1123,8 +1142,8 @@ size_t kd_batch_set_bytes() { return sizeof(KdBatchSet); }
 void kd_batch_set_fill(void* out, const knn_index* ix, const QueryArgs& a, const QueryPlan& plan,
                         const uint32_t* order, uint32_t order_base, uint32_t first_block, uint32_t query_offset) {
     KdBatchSet bs{};
-    // (A class of warp-per-query searches has every index's boxes built before the batch is captured.)
-    bs.p = plan.box ? kd_box_params(ix, a, order, std::max(plan.leaf_scan, kd_warp_bucket(ix->dims)))
+    // (A class of warp-per-query searches has every index's boxes.)
+    bs.p = plan.box ? kd_box_params(ix, ix->kd_box, a, order, std::max(plan.leaf_scan, kd_warp_bucket(ix->dims)))
                     : kd_params(ix, a, order, plan.leaf_scan);
     bs.p.order_base = order_base;
     bs.first_block = first_block;

@@ -256,9 +256,8 @@ struct StreamOrder {
     }
 };
 
-// A second stream of the index: for work that can run beside the caller's stream within one
-// query (the radius model's seeds beside the locality sort), joined back through events, and for the
-// k-d node boxes.
+// A second stream of the index for work that can run beside the caller's stream within one
+// query (the radius model's seeds beside the locality sort), joined back through events.
 struct SideStream {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -344,11 +343,14 @@ struct knn_index {
 
     // k-d tree: split value per internal node (implicit heap, children 2i+1, 2i+2).
     knn::DevBuf split;
-    // k-d tree (built on first use, complete on the device once held here): the tight bounding box of the points under every node down to
-    // depth kd_box_depth (subtrees of at most 4 slots, 16 beyond 16 dims), per node lo[q], hi[q] with
-    // q = max(4, padded dims) floats each; and the warp-group search's scratch.
-    knn::DevBuf kd_box;
-    uint32_t kd_box_depth = 0, kd_box_stride = 0;
+    // k-d tree: the tight bounding box of the points under every node down to `depth`, per node lo[q],
+    // hi[q] with q = max(4, padded dims) floats each; complete on the device once held here.  kd_box
+    // reaches the default search's buckets and is built with the tree, kd_fine_box the warp-group
+    // search's smaller ones, on its first query.  And that search's scratch.
+    struct KdBoxes {
+        knn::DevBuf buf;
+        uint32_t depth = 0;
+    } kd_box, kd_fine_box;
     knn::DevBuf group_ws;
 
     // Trees: leaf slots, 2^node_depth leaves x leaf_slots slots; a slot is `leaf_stride` floats:
@@ -369,7 +371,7 @@ struct knn_index {
     knn::DevBuf workspace;
     knn::DevBuf staging;   // device copies of host queries/results (knn_query_host)
     knn::HostIo host_io;   // knn_query_host's copy streams
-    knn::SideStream side;  // the radius model's stream within a learned-radius query; the k-d boxes' build
+    knn::SideStream side;  // the radius model's stream within a learned-radius query
     knn::StreamOrder order_guard;
     knn::DevBuf counters;  // DevCounters
     knn::QueryTiming timing;
@@ -461,8 +463,10 @@ int tc_selftest(uint32_t dims, float* max_rel_err, uint32_t* bad);
 int kd_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order, uint32_t max_levels = 24);
 int ball_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order);
 int kd_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s);
-// Whether queries can search the k-d node boxes (built here if missing): not where the stream is being
-// captured before they were built, nor where no memory is left for them.
+// The k-d node boxes down to subtrees of `bucket` slots (0: the default search's), built if `held` has none.
+int kd_box_ensure(knn_index* ix, knn_index::KdBoxes& held, uint32_t bucket, cudaStream_t s);
+// Whether queries can search the node boxes.  They come with the index; where there was no memory for
+// them they are built here, unless the stream is being captured or there still is none.
 int kd_boxes_ready(knn_index* ix, cudaStream_t s, bool* ready);
 int ball_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s);
 

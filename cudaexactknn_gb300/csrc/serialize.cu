@@ -213,6 +213,13 @@ int knn_index_deserialize(const void* host_buf, size_t size, void* stream, knn_i
         ix->model_margin = m;
     }
     ix->device_bytes = h.bytes[0] + h.bytes[1] + h.bytes[2] + h.bytes[3];
+    if (ix->structure == KNN_KD_TREE && ix->n) {  // the node boxes are not part of the blob
+        bool ready = false;
+        if ((rc = knn::kd_boxes_ready(ix, s, &ready)) != KNN_OK) {
+            delete ix;
+            return rc;
+        }
+    }
     *out = ix;
     return KNN_OK;
 }

@@ -111,11 +111,11 @@ typedef struct knn_query_opts {
                                leaf (0 = the engine's choice, or the tree's own leaves; the
                                warp-per-query search takes values below its own choice as that) */
     uint32_t traversal;     /* trees: 0 = one depth-first search per query (the reference's scheme);
-                               k-d trees run it with a warp per query, bounded by tight node boxes
-                               that the first query builds (a thread per query, bounded by the
-                               splitting planes, where they cannot be built: inside a stream
-                               capture, or out of memory; the storage options above apply to that
-                               search and to traversal 1), ball trees always, over their balls;
+                               k-d trees run it with a warp per query, bounded by the tight node
+                               boxes that come with the tree (a thread per query, bounded by the
+                               splitting planes, where there is no memory for them; the storage
+                               options above apply to that search and to traversal 1), ball trees
+                               always, over their balls;
                                1 = warp-coherent search (a warp's queries walk together);
                                k-d trees of at most 16 dims, k <= 32: 2 = warp-group search (a
                                warp's 32 queries walk the tree once against the node boxes from
@@ -150,8 +150,8 @@ typedef struct knn_index_info {
     uint32_t node_depth;  /* internal node levels */
     uint32_t leaf_slots;  /* 2^depth_skips */
     uint32_t node_count;  /* internal nodes, 2^node_depth - 1 */
-    uint64_t device_bytes; /* the index, and what its first queries built for it and keep: a k-d
-                              tree's node boxes, the tensor-core filter's layout */
+    uint64_t device_bytes; /* the index, and what queries built for it and keep: the tensor-core
+                              filter's layout, the k-d warp-group search's node boxes */
     float build_ms;       /* device time of the construction, CUDA events */
     uint32_t radius_model;/* 1 when a learned radius model is attached */
 } knn_index_info;

@@ -1,6 +1,6 @@
-"""The k-d tree's node boxes, built by the first query that searches them, are complete before anything
-else reads them: batch graphs, training and captured queries run on streams that do not wait for the
-stream of the query that built them."""
+"""The k-d tree's node boxes come with the tree, reach the buckets that are searched, and are complete
+before anything reads them: batch graphs, training and captured queries run on streams that do not wait
+for the stream of the index's first query."""
 
 import numpy as np
 import pytest
@@ -114,14 +114,40 @@ def test_training_beside_the_first_query():
     np.testing.assert_array_equal(models[0].view(np.uint32), models[1].view(np.uint32))
 
 
-@pytest.mark.parametrize("dims,opts", [(3, {}), (3, {"traversal": 2}), (12, {}), (40, {})])
-def test_device_bytes_count_the_boxes(dims, opts):
-    pts, qs, want = _case(dims, n=5000, q=50)
-    ix = gu.make_index("kd", pts)
-    before = ix.info().device_bytes
-    gu.assert_rows_equal(*gu.run(ix, qs, 10, **opts), *want)
-    after = ix.info().device_bytes
-    assert after >= before + 2 * 4 * dims * (5000 // 32)  # two corners per 32 slots at least
-    gu.assert_rows_equal(*gu.run(ix, qs, 10, **opts), *want)
-    assert ix.info().device_bytes == after  # built once
+@pytest.mark.parametrize("dims", [3, 12, 40])
+def test_boxes_reach_the_buckets_that_are_searched(dims):
+    """An index holds its tree and the boxes of subtrees of 32 slots (16 beyond 8 dims), no deeper, from its
+    creation or from its saved form on; the warp-group search's smaller ones come with that search's first
+    query.  device_bytes counts all of them."""
+    from cudaexactknn_gb300 import knn
+    pts, qs, want = _case(dims, n=60000, q=50)
+    made = gu.make_index("kd", pts)
+    info = made.info()
+    row = 4 if dims < 4 else {12: 16, 40: 64}[dims]
+    tree = 4 * info.node_count + 4 * (info.node_count + 1) * info.leaf_slots * (4 if dims < 4 else row + 4)
+    box = ((2 << (info.node_depth - (5 if dims <= 8 else 4))) - 1) * 2 * 4 * row
+    for ix in (made, knn.load_index(made.serialize())):
+        assert ix.info().device_bytes == tree + box
+        gu.assert_rows_equal(*gu.run(ix, qs, 10), *want)
+        assert ix.info().device_bytes == tree + box
+        if dims <= 16:
+            for _ in range(2):
+                gu.assert_rows_equal(*gu.run(ix, qs, 10, traversal=2), *want)
+                assert ix.info().device_bytes > tree + 3 * box
+            gu.assert_rows_equal(*gu.run(ix, qs, 10), *want)
+        ix.close()
+
+
+# A node's slots over fewer lanes than a warp, one each, and several; dimensions over the lanes beyond 16.
+@pytest.mark.parametrize("dims", [1, 3, 9, 16, 17, 100])
+@pytest.mark.parametrize("n,skips", [(1, 0), (2, 1), (17, 2), (33, 5), (1000, 0), (1000, 4), (5000, 7), (3000, 30),
+                                     (513, 9), (1000, 9)])
+def test_boxes_of_every_bucket_size(dims, n, skips):
+    rng = np.random.default_rng(n + dims)
+    pts = W.uniform(rng, n, dims) - np.float32(0.5)  # both signs: padding's zeros lie inside
+    qs = (W.uniform(rng, 40, dims) - np.float32(0.5)) * np.float32(3)
+    want = oracle.bf_knn(pts, qs, 5, fma=True, threads=8)
+    ix = gu.make_index("kd", pts, skips)
+    for traversal in (0, 2, 0) if dims <= 16 else (0,):
+        gu.assert_rows_equal(*gu.run(ix, qs, 5, traversal=traversal), *want, what=f"traversal {traversal}")
     ix.close()
