@@ -2,7 +2,8 @@
 // and bf_noalloc.cu (the allocation-free entry point).
 //
 // Replaces BruteForceKernels::knnKernel / knnShKernel (src/BruteForceGpu.cuh:9-50), where one
-// thread scans all n points for its query straight from global memory.  Here a warp holds Q
+// thread scans all n points for its query straight from global memory.  Here, but for few points or
+// many queries with small k (the thread-per-query form at the end), a warp holds Q
 // queries and its lanes take 32 points at a time:
 //   * every pair's distance is the reference's sequential fused sum, two queries per packed
 //     instruction (sub/fma.rn.f32x2 round each half as the scalar instructions do);
@@ -29,6 +30,7 @@
 #include <algorithm>
 
 #include "knn_internal.h"
+#include "tracker.cuh"
 #include "warp_search.cuh"
 
 namespace knn {
@@ -414,6 +416,145 @@ int bf_launch_merge(const BfParams& p, uint32_t splits, cudaStream_t stream) {
     bf_merge_kernel<KR><<<ceil_div(p.nq, 4), 128, 0, stream>>>(p.partial, splits, p.nq, p.k, p.max_d2, p.radii, p.order,
                                                                p.count_dev, p.out_idx, p.out_dist);
     KNN_LAUNCHED();
+    return KNN_OK;
+}
+
+// ---- a thread per query ---------------------------------------------------------------------------
+// The plain form: a thread holds its query and its top-k in registers and goes through the tiles a block
+// stages, all threads reading the same point.  No lists in shared memory, no first look, no merge
+// over warps: nothing to pay per query but the insertions themselves.  bf_by_thread says where that wins.
+// `kk` of the k places can be filled (min(k, n)); the others are written as they start.
+template <int DP>
+struct BfThreadTile {
+    static constexpr uint32_t PS = (DP + 3) / 4 * 4, kRows = 8192 / PS;  // 32 KB
+    static constexpr uint32_t kChunk = 4 * kRows;                        // least points of a split
+};
+constexpr uint32_t kBfThreads = 128;
+
+template <int DP, int KMAX, bool RAW>
+__global__ void __launch_bounds__(kBfThreads) bf_thread_kernel(const BfParams p, uint32_t kk) {
+    constexpr uint32_t PS = BfThreadTile<DP>::PS, T = BfThreadTile<DP>::kRows;
+    __shared__ float4 tile[T * PS / 4];
+    const uint32_t t = blockIdx.x * kBfThreads + threadIdx.x;
+    const bool active = t < p.nq;
+    const uint32_t qi = active ? (p.order ? p.order[t] : t) : 0u;
+    float q[PS];
+#pragma unroll
+    for (uint32_t d = 0; d < PS; ++d)
+        q[d] = active && d < p.dims ? p.queries[static_cast<size_t>(qi) * p.dims + d] : 0.0f;
+    const float r2 = active && p.radii ? p.radii[qi] : p.max_d2;
+    Tracker<KMAX, false, false> tr;
+    tr.init(kk, r2, nullptr, 0);
+    const uint32_t lo = blockIdx.y * p.chunk, hi = min(p.n, lo + p.chunk);
+    for (uint32_t base = lo; base < hi; base += T) {
+        const uint32_t rows = min(T, hi - base);
+        __syncthreads();
+        if constexpr (RAW) {
+            for (uint32_t i = threadIdx.x; i < rows * PS; i += kBfThreads) {
+                const uint32_t r = i / PS, d = i % PS;
+                reinterpret_cast<float*>(tile)[i] = d < p.dims ? p.points[static_cast<size_t>(base + r) * p.dims + d] : 0.0f;
+            }
+        } else {
+            const float4* src = reinterpret_cast<const float4*>(p.points) + static_cast<size_t>(base) * (PS / 4);
+            for (uint32_t i = threadIdx.x; i < rows * (PS / 4); i += kBfThreads) tile[i] = src[i];
+        }
+        __syncthreads();
+        if (!active) continue;
+        uint32_t r = 0;
+        for (; r + 1 < rows; r += 2) {  // two chains at a time
+            const float d0 = dist2_vec4<PS>(q, tile + r * (PS / 4));
+            const float d1 = dist2_vec4<PS>(q, tile + (r + 1) * (PS / 4));
+            tr.offer(make_key(d0, static_cast<int32_t>(base + r)));
+            tr.offer(make_key(d1, static_cast<int32_t>(base + r + 1)));
+        }
+        if (r < rows) tr.offer(make_key(dist2_vec4<PS>(q, tile + r * (PS / 4)), static_cast<int32_t>(base + r)));
+    }
+    if (!active) return;
+    if (p.partial) {
+        tr.emit_keys(kk, p.partial + (static_cast<size_t>(blockIdx.y) * p.nq + t) * p.k);
+        return;
+    }
+    int32_t* idx = p.out_idx + static_cast<size_t>(qi) * p.k;
+    float* dist = p.out_dist + static_cast<size_t>(qi) * p.k;
+    tr.emit(kk, idx, dist);
+    for (uint32_t i = kk; i < p.k; ++i) {
+        idx[i] = -1;
+        dist[i] = r2;
+    }
+}
+
+// Splits of a thread per query's scan: until the blocks cover the GPU about four times, at least kChunk
+// points each.
+template <int DP, int KMAX, bool RAW>
+uint32_t bf_thread_splits(uint32_t n, uint32_t count, uint64_t max_splits) {
+    static const int per_sm = [] {
+        int v = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, bf_thread_kernel<DP, KMAX, RAW>, kBfThreads, 0) == cudaSuccess
+                   ? std::max(v, 1) : 1;
+    }();
+    const uint32_t want = ceil_div(4u * static_cast<uint32_t>(sm_count() * per_sm), ceil_div(count, kBfThreads));
+    return static_cast<uint32_t>(std::max<uint64_t>(
+        1, std::min<uint64_t>({want, ceil_div(n, BfThreadTile<DP>::kChunk), max_splits, 0xFFFFu})));
+}
+
+// Whether a thread per query answers a call faster than the warps do.  Measured over 1 to 128 dims, 4 to
+// 262,144 points, 1 to 200,000 queries, k 1 to 100; the line is where the two take the same time.
+//   * Very few points: a thread's scan is over before a warp's lists are set up (3 dims, 32 points, k 8,
+//     100,000 queries: 15 us, a warp 60).
+//   * Beyond, once the threads fill the GPU (12,288: 81 per SM; with fewer the scan's latency shows:
+//     2,048 points of 32 dims, k 8, 8,000 queries 134 us against 60 with a warp, 32,000 queries 195
+//     against 295) up to a number of points that grows with the dimensions, as the warps' staging leaves
+//     one block per SM there, and falls with k, as every insertion holds up 32 queries.
+// (For k beyond 16 the line is a multiple of k or its square: that many of the points are insertions.)
+inline bool bf_by_thread(int dp, uint32_t k, uint32_t n, uint32_t count, uint32_t splits, uint32_t chunk) {
+    if (k > 32) return n <= 16 && dp >= 64 && count >= 16384;
+    if (n <= 16) return true;
+    if (count < 64) return false;
+    if (n <= (k > 16 ? 32u : k <= 8 && dp <= 16 ? 128u : 64u)) return true;
+    const uint64_t threads = static_cast<uint64_t>(count) * splits;
+    if (threads < (count < 128 && dp >= 32 ? 8192u : dp == 128 ? 10000u : 12288u)) return false;
+    switch (dp) {
+        case 8:
+        case 16: {
+            const uint32_t most = threads < 30000 ? 1024u : dp == 8 ? 16384u : 4096u;
+            return n <= (k <= 8 ? most : k <= 16 ? 128u : k * k / 8);
+        }
+        case 32: return k <= 8 || n <= (k <= 16 ? 1024u : k * k / 4);
+        case 64: return k <= 8 || n <= (k <= 16 ? 2048u : k * k / 2);
+        case 128:
+            // (More work than this is the warps' again: the thread's registers leave two blocks per SM.)
+            return (n <= 512 || static_cast<uint64_t>(count) * ceil_div(n, chunk) <= 200000) &&
+                   n <= (k <= 8 ? 65536u : k <= 16 ? 16384u : k * k);
+        default:
+            return n <= (k <= 8 ? 256u : k <= 16 ? 64u : 2 * k) ||
+                   (static_cast<uint64_t>(n) * k <= (dp == 4 ? 2048u : 1024u) && 60ull * n * k <= threads);
+    }
+}
+
+// Launches a thread per query (and the merge, where the points are split); *ran is false where the warps
+// are to answer.  `scratch(splits)` gives the room for the splits' lists in p.partial.
+template <int DP, int KMAX, bool RAW, class Scratch>
+int bf_launch_thread(BfParams p, uint64_t max_splits, Scratch&& scratch, cudaStream_t stream, bool* ran) {
+    uint32_t splits = bf_thread_splits<DP, KMAX, RAW>(p.n, p.nq, max_splits);
+    *ran = bf_by_thread(DP, p.k, p.n, p.nq, splits, BfThreadTile<DP>::kChunk);
+    if (!*ran) return KNN_OK;
+    p.chunk = ceil_div(ceil_div(p.n, splits), BfThreadTile<DP>::kRows) * BfThreadTile<DP>::kRows;
+    splits = ceil_div(p.n, p.chunk);
+    if (splits > 1) KNN_TRY(scratch(splits, &p.partial));
+    else p.partial = nullptr;
+    bf_thread_kernel<DP, KMAX, RAW><<<dim3(ceil_div(p.nq, kBfThreads), splits), kBfThreads, 0, stream>>>(p, std::min(p.k, p.n));
+    KNN_LAUNCHED();
+    return splits > 1 ? bf_launch_merge<1>(p, splits, stream) : KNN_OK;
+}
+
+// The same by the places there are to fill.
+template <int DP, bool RAW, class Scratch>
+int bf_thread_query(const BfParams& p, uint64_t max_splits, Scratch&& scratch, cudaStream_t stream, bool* ran) {
+    const uint32_t kk = std::min(p.k, p.n);
+    *ran = false;
+    if (kk <= 8) return bf_launch_thread<DP, 8, RAW>(p, max_splits, scratch, stream, ran);
+    if (kk <= 16) return bf_launch_thread<DP, 16, RAW>(p, max_splits, scratch, stream, ran);
+    if (kk <= 32) return bf_launch_thread<DP, 32, RAW>(p, max_splits, scratch, stream, ran);
     return KNN_OK;
 }
 

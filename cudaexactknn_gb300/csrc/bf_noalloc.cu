@@ -56,9 +56,16 @@ int scratch_address(uint64_t** out) {
 }
 
 template <int DP, int KR>
-int run(const float* points, uint32_t n, uint32_t dims, const float* queries, uint32_t count, float max_d2,
-        uint32_t k, int32_t* idx, float* dist, uint64_t* scratch, cudaStream_t s) {
-    const BfShape shape = bf_shape<DP, KR>(n, count, kScratchKeys / (static_cast<uint64_t>(count) * k));
+int run(BfParams p, uint64_t max_splits, uint64_t* scratch, cudaStream_t s) {
+    const BfShape shape = bf_shape<DP, KR>(p.n, p.nq, max_splits);
+    p.partial = scratch;
+    KNN_TRY((bf_launch<DP, KR, true>(p, shape, s)));
+    return shape.splits > 1 ? bf_launch_merge<KR>(p, shape.splits, s) : KNN_OK;
+}
+
+template <int DP>
+int run_k(const float* points, uint32_t n, uint32_t dims, const float* queries, uint32_t count, float max_d2,
+          uint32_t k, int32_t* idx, float* dist, uint64_t* scratch, cudaStream_t s) {
     BfParams p{};
     p.points = points;
     p.n = n;
@@ -69,17 +76,16 @@ int run(const float* points, uint32_t n, uint32_t dims, const float* queries, ui
     p.k = k;
     p.out_idx = idx;
     p.out_dist = dist;
-    p.partial = scratch;
-    KNN_TRY((bf_launch<DP, KR, true>(p, shape, s)));
-    return shape.splits > 1 ? bf_launch_merge<KR>(p, shape.splits, s) : KNN_OK;
-}
-
-template <int DP>
-int run_k(const float* points, uint32_t n, uint32_t dims, const float* queries, uint32_t count, float max_d2,
-          uint32_t k, int32_t* idx, float* dist, uint64_t* scratch, cudaStream_t s) {
-    if (k <= 32) return run<DP, 1>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
-    if (k <= 64) return run<DP, 2>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
-    return run<DP, 4>(points, n, dims, queries, count, max_d2, k, idx, dist, scratch, s);
+    const uint64_t max_splits = kScratchKeys / (static_cast<uint64_t>(count) * k);
+    bool ran = false;
+    KNN_TRY((bf_thread_query<DP, true>(p, max_splits, [&](uint32_t, uint64_t** out) {
+        *out = scratch;
+        return static_cast<int>(KNN_OK);
+    }, s, &ran)));
+    if (ran) return KNN_OK;
+    if (k <= 32) return run<DP, 1>(p, max_splits, scratch, s);
+    if (k <= 64) return run<DP, 2>(p, max_splits, scratch, s);
+    return run<DP, 4>(p, max_splits, scratch, s);
 }
 
 }  // namespace
