@@ -74,8 +74,7 @@ struct BfSmem {
         uint32_t least[kBfWarps * Q * KR * 32];                    // the first look's minima, query by query
     };
     uint32_t count[kBfWarps][Q];                                   // keys left in a buffer at the end, and (top bit) whether its list holds any
-    uint64_t kth[kBfWarps][Q];                                     // each list's k-th key
-    uint4 bound[kBfWarps][Q >= 4 ? Q / 4 : 1];                     // per query group: distance bits
+    uint4 limit[kBfWarps][Q >= 4 ? Q / 4 : 1];                     // per warp and query: see bf_limits
     float2 q[kBfWarps][Q / 2][bf_wide(DP) ? DP : 1];            // pairs of queries, by dimension
     float4 tile[2 * bf_tile(DP) * kStride / 4];
 };
@@ -83,9 +82,13 @@ struct BfSmem {
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
     return (static_cast<uint64_t>(__float_as_uint(b)) << 32) | __float_as_uint(a);
 }
-// The bounds of a query group, as they stand (other warps lower them).
+// The distance bits that a warp's next points have to be below, as they stand (other warps lower them): one
+// more than the bound on the k-th distance that any warp of the query has found, or its own list's k-th
+// distance once that is a point's.  A warp meets its points by ascending index, so one at that distance
+// comes after all in its list: with equal distances left to the keys, data of many of them filled and
+// flushed buffers to no end (32,880 equal points, 16,237 queries: 1,661 us, a thread per query 374).
 template <uint32_t Q>
-__device__ __forceinline__ void bf_bounds(const uint4* at, uint32_t (&out)[Q]) {
+__device__ __forceinline__ void bf_limits(const uint4* at, uint32_t (&out)[Q]) {
     const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(at));
     if constexpr (Q == 2) {
         asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(out[0]), "=r"(out[1]) : "r"(a));
@@ -97,17 +100,18 @@ __device__ __forceinline__ void bf_bounds(const uint4* at, uint32_t (&out)[Q]) {
                          : "r"(a + 4 * j));
     }
 }
+__device__ __forceinline__ uint32_t bf_above(uint32_t bits) { return bits + (bits != 0xFFFFFFFFu ? 1u : 0u); }
 
 // Sorts a buffer of n <= 64 keys into a list in shared memory; returns the list's k-th key.
 template <int KR>
-__device__ __noinline__ uint64_t bf_flush(uint64_t* list, const uint64_t* buf, uint32_t n, uint32_t k, uint32_t lane, uint64_t kth) {
+__device__ __noinline__ uint64_t bf_flush(uint64_t* list, const uint64_t* buf, uint32_t n, uint32_t k, uint32_t lane) {
     WarpTopK<KR> top;
     top.k = k;
     top.lane = lane;
-    top.kth = kth;
     top.empty = false;
 #pragma unroll
     for (int j = 0; j < KR; ++j) top.v[j] = list[32 * j + lane];
+    top.refresh();
     for (uint32_t i = 0; i < n; i += 32) top.offer(i + lane < n, i + lane < n ? buf[i + lane] : ~0ull);
 #pragma unroll
     for (int j = 0; j < KR; ++j) list[32 * j + lane] = top.v[j];
@@ -136,15 +140,14 @@ __global__ void __launch_bounds__(32 * kBfWarps, R == 1 ? 3 : 2) bf_warp_kernel(
     // The group's queries in pairs, their lists and bounds.  A slot past the live list holds key 0:
     // nothing is below it.
     uint64_t qr[bf_wide(DP) ? 1 : Q / 2][bf_wide(DP) ? 1 : DP];
-    uint32_t* bounds = reinterpret_cast<uint32_t*>(sm.bound[g]);
+    auto limit_of = [&](uint32_t of_warp, uint32_t j) { return reinterpret_cast<uint32_t*>(sm.limit[of_warp]) + j; };
 #pragma unroll
     for (uint32_t j = 0; j < Q; ++j) {
         const uint32_t t = first + j;
         const uint64_t fill = t < live ? make_key(p.radii ? p.radii[query_of(t)] : p.max_d2, -1) : 0ull;
 #pragma unroll
         for (int r = 0; r < KR; ++r) sm.list[w][j][32 * r + lane] = fill;
-        if (lane == 0) sm.kth[w][j] = fill;
-        if (part == 0 && lane == 0) bounds[j] = static_cast<uint32_t>(fill >> 32);
+        if (lane == 0) *limit_of(w, j) = t < live ? bf_above(static_cast<uint32_t>(fill >> 32)) : 0u;
     }
 #pragma unroll
     for (uint32_t h = 0; h < Q / 2; ++h) {
@@ -269,28 +272,31 @@ __global__ void __launch_bounds__(32 * kBfWarps, R == 1 ? 3 : 2) bf_warp_kernel(
         __syncthreads();
         for (uint32_t e = w; e < groups * Q; e += kBfWarps) {
             WarpTopK<KR> top;
-            uint32_t* at = reinterpret_cast<uint32_t*>(sm.bound[e / Q]) + e % Q;
-            top.init(p.k, __uint_as_float(*at), lane);
+            const uint32_t within = *limit_of(e / Q, e % Q);  // (the query's radius, in every part's row)
+            if (!within) continue;
+            top.init(p.k, __uint_as_float(within - 1u), lane);
             for (uint32_t s = 0; s < per_query; s += 32)
                 top.offer(true, static_cast<uint64_t>(sm.least[e * per_query + s + lane]) << 32);
-            __syncwarp();
-            if (lane == 0) *at = static_cast<uint32_t>(top.kth >> 32);
+            if (lane < parts) *limit_of(lane * groups + e / Q, e % Q) = bf_above(static_cast<uint32_t>(top.kth >> 32));
         }
         __syncthreads();
     }
 
-    uint32_t count[Q], bound[Q], flushed = 0;  // keys in each buffer; bounds; lists that hold any (bit j)
+    uint32_t count[Q], limit[Q], flushed = 0;  // keys in each buffer; bf_limits; lists that hold any (bit j)
 #pragma unroll
     for (uint32_t j = 0; j < Q; ++j) count[j] = 0;
-    bf_bounds(sm.bound[g], bound);
+    // Lane s tells part s of a new k-th distance.  (The address is kept beyond 4 dims only: there the loop is
+    // 11% slower without, 6 dims, 65,536 points, 16,000 queries, k 32; up to 4 dims 15% slower with it.)
+    const uint32_t peer = static_cast<uint32_t>(__cvta_generic_to_shared(limit_of(lane < parts ? lane * groups + g : w, 0)));
+    bf_limits(sm.limit[w], limit);
     scan(1, [&](const uint64_t (&acc)[Q / 2], uint32_t index, bool live_point, uint32_t) {
         bool hit = false;
 #pragma unroll
-        for (uint32_t j = 0; j < Q; ++j) hit |= bits_of(acc, j) <= bound[j];
+        for (uint32_t j = 0; j < Q; ++j) hit |= bits_of(acc, j) < limit[j];
         if (!__any_sync(kFullMask, hit && live_point)) return;
 #pragma unroll
         for (uint32_t j = 0; j < Q; ++j) {
-            const bool cand = live_point && bits_of(acc, j) <= bound[j];
+            const bool cand = live_point && bits_of(acc, j) < limit[j];
             const uint32_t m = __ballot_sync(kFullMask, cand);
             if (!m) continue;
             uint64_t* buf = sm.buf[w][j];
@@ -298,18 +304,18 @@ __global__ void __launch_bounds__(32 * kBfWarps, R == 1 ? 3 : 2) bf_warp_kernel(
             count[j] += __popc(m);
             if (count[j] <= 32) continue;  // room for the next step's 32
             __syncwarp();
-            const uint64_t was = sm.kth[w][j];
-            const uint64_t now = bf_flush<KR>(sm.list[w][j], buf, count[j], p.k, lane, was);
+            const uint64_t now = bf_flush<KR>(sm.list[w][j], buf, count[j], p.k, lane);
             count[j] = 0;
             flushed |= 1u << j;
-            // (The bound is any of the parts' k-th distance: k points lie within it.)
-            if (now != was && lane == 0) {
-                sm.kth[w][j] = now;
-                atomicMin(bounds + j, static_cast<uint32_t>(now >> 32));
+            // (Its k points lie within the list's k-th distance, whichever part holds them.)
+            if (lane < parts && key_index(now) >= 0) {
+                const uint32_t to = static_cast<uint32_t>(now >> 32) + (lane == part ? 0u : 1u);
+                if constexpr (bf_wide(DP)) asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(peer + 4 * j), "r"(to) : "memory");
+                else atomicMin(limit_of(lane * groups + g, j), to);
             }
             __syncwarp();
         }
-        bf_bounds(sm.bound[g], bound);  // (read here, not at every step: shared memory returns 128 bytes a clock)
+        bf_limits(sm.limit[w], limit);  // (read here, not at every step: shared memory returns 128 bytes a clock)
     });
 #pragma unroll
     for (uint32_t j = 0; j < Q; ++j)
@@ -516,7 +522,7 @@ inline bool bf_by_thread(int dp, uint32_t k, uint32_t n, uint32_t count, uint32_
     switch (dp) {
         case 8:
         case 16: {
-            const uint32_t most = threads < 30000 ? 1024u : dp == 8 ? 16384u : 4096u;
+            const uint32_t most = threads < 30000 ? 1024u : dp == 8 ? 32768u : 4096u;
             return n <= (k <= 8 ? most : k <= 16 ? 128u : k * k / 8);
         }
         case 32: return k <= 8 || n <= (k <= 16 ? 1024u : k * k / 4);
