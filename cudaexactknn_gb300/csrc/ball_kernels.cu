@@ -3,8 +3,8 @@
 // Replaces BallTreeKernels::knnDevice and its four storage variants (src/BallTreeGpu.cuh:36-200),
 // a depth-first search per thread: at each internal node the distance to both child balls, the closer
 // one entered, the farther one pushed when it can still hold a neighbour (src/BallTreeGpu.cuh:82-92).
-// Here each query gets a warp (ball_warp_query_kernel, warp_search.cuh); traversal 1 walks 32
-// neighbouring queries together.
+// Here each query gets a warp (ball_warp_query_kernel, warp_search.cuh), or a thread where very many
+// queries have very few dims (ball_knn_kernel); traversal 1 walks 32 neighbouring queries together.
 // The reference's border distance sqrt(d2) - r (with -use_fast_math's approximate sqrt) can
 // round above a point's own float distance and prune a true neighbour; here knn::ball_bound
 // uses directed rounding and relative margins so it never exceeds the float dist2 of any point
@@ -66,6 +66,82 @@ __device__ __forceinline__ float centre_dist(const float (&q)[DP], const float* 
         *r = b[DP];
         return dist2_vec4<DP>(q, reinterpret_cast<const float4*>(b));
     }
+}
+
+// One thread's search: query slot t of the batch (its query is p.order[t] - p.order_base, or t).
+template <int DP, int KMAX>
+__device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t t) {
+    const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
+    float q[DP];
+    load_query<DP>(p.queries, p.dims, qi, q);
+    const float r2 = p.radii ? p.radii[qi] : p.max_d2;
+
+    Tracker<KMAX, false, false> tr;
+    tr.init(p.k, r2, nullptr, 0);
+    Stack<false> st;
+    st.init(nullptr, 0);
+    st.push(0, 0.0f);
+    LocalCounters lc;
+    bool overflow = false;
+
+    while (st.top) {
+        uint32_t node;
+        float bound;
+        st.pop(&node, &bound);
+        if (bound > tr.radius()) continue;
+        bool pruned = false;
+        uint32_t depth = heap_depth(node);
+        while (depth < p.stop_depth) {
+            const uint32_t l = 2 * node + 1;
+            float rl, rr;
+            const float sl = centre_dist<DP>(q, p.ball + static_cast<size_t>(l) * p.ball_stride, &rl);
+            const float sr = centre_dist<DP>(q, p.ball + static_cast<size_t>(l + 1) * p.ball_stride, &rr);
+            const float bl = ball_bound(sl, rl, p.margin);
+            const float br = ball_bound(sr, rr, p.margin);
+            ++lc.nodes;
+            // Visit order only (not a bound): the nearer border first.
+            const bool left_first = sqrtf(sl) - rl < sqrtf(sr) - rr;
+            const uint32_t close_child = left_first ? l : l + 1;
+            const float close_b = left_first ? bl : br;
+            const float far_b = left_first ? br : bl;
+            if (close_b > tr.radius()) {
+                // The farther ball's bound is at least as large in the common case, but the
+                // order above is approximate, so it is checked on its own.
+                if (far_b <= tr.radius()) {
+                    node = left_first ? l + 1 : l;
+                    ++depth;
+                    continue;
+                }
+                pruned = true;
+                break;
+            }
+            if (far_b <= tr.radius()) overflow |= !st.push(left_first ? l + 1 : l, far_b);
+            node = close_child;
+            ++depth;
+        }
+        if (pruned) continue;
+        const SlotRange r = subtree_slots(node, depth, p.node_depth, p.node_count, p.leaf_slots);
+        const float* slot = p.leaf + r.first * p.leaf_stride;
+        ++lc.leaves;
+        for (uint32_t s = 0; s < r.count; ++s, slot += p.leaf_stride) {
+            int32_t id;
+            const float d2 = slot_dist<DP>(q, slot, &id);
+            if (id < 0) continue;
+            ++lc.points;
+            tr.offer(make_key(d2, id));
+        }
+    }
+    tr.emit(p.k, p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
+    if (p.counters) {
+        lc.flush(p.counters);
+        if (overflow) atomicExch(&p.counters->error, 1);
+    }
+}
+
+template <int DP, int KMAX>
+__global__ void __launch_bounds__(128) ball_knn_kernel(const BallParams p) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < p.nq) ball_search_thread<DP, KMAX>(p, t);
 }
 
 // Warp-coherent variant (see kd_knn_warp_kernel): the warp's queries walk the tree together,
@@ -292,6 +368,32 @@ inline BallParams ball_params(const knn_index* ix, const QueryArgs& a, const uin
     return p;
 }
 
+// Whether a batch's queries get a thread each, in locality order, instead of a warp each (kd_by_thread says
+// when that pays; a ball's bound is the same either way, so queries far from the points cost a thread no
+// more than a warp).  1,000,000 queries, a warp and a thread each, us: 30,000 1-d points, k 1, 656 and 186;
+// 30,000 3-d points, k 8, 1,594 and 1,429; 1,000,000 uniform 3-d points, k 1, 1,524 and 979, clustered ones
+// 6,150 and 7,700; on the clustered ones with k 4 7,115 and 11,834, so from k 3 on the line also asks for
+// four queries a point.
+constexpr bool kBallThreadDims(int dp) { return dp <= 4; }
+inline bool ball_by_thread(int dp, uint32_t n, const QueryArgs& a, const QueryPlan& p) {
+    if (!p.reorder || a.order || a.count_dev || a.seeds || a.k > 16) return false;
+    const uint64_t q = a.count;
+    if (dp == 1) return q >= (a.k <= 8 ? 250000u : 500000u);
+    if (dp <= 3 && a.k <= 2) return q >= 500000;
+    return a.k <= 8 && q >= 1000000 && q >= 4ull * n;
+}
+
+template <int DP>
+int launch_ball_thread(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order, cudaStream_t s) {
+    const BallParams p = ball_params(ix, a, order, plan.leaf_scan);
+    auto kern = a.k <= 8 ? ball_knn_kernel<DP, 8> : ball_knn_kernel<DP, 16>;
+    if (plan.timing) KNN_TRY(ix->timing.begin(s));
+    kern<<<ceil_div(a.count, 128), 128, 0, s>>>(p);
+    KNN_LAUNCHED();
+    if (plan.timing) KNN_TRY(ix->timing.end(s));
+    return KNN_OK;
+}
+
 // Warp-coherent search (traversal 1).
 template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
 static int launch_ball(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, const uint32_t* order,
@@ -336,8 +438,7 @@ int ball_order_dp(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint3
     const uint32_t levels = std::min<uint32_t>(ix->node_depth, 24);
     if (levels == 0) return KNN_OK;
     const size_t nq = a.count;
-    const size_t need = carve_bytes({nq * 4, nq * 4, nq * 4, nq * 4, radix_sort_temp_bytes(a.count)});
-    KNN_TRY(ix->workspace.reserve(need));
+    KNN_TRY(ix->workspace.reserve(order_bytes(a.count)));
     Carver c(ix->workspace.ptr);
     uint32_t* keys = c.take<uint32_t>(nq);
     uint32_t* vals = c.take<uint32_t>(nq);
@@ -387,6 +488,14 @@ int ball_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStr
         const size_t storage = tracker_smem_bytes(p.sh_nn, k_class(a.k), block) + stack_smem_bytes(p.sh_stack, block);
         if (storage > kMaxBlockSmem)
             return fail(KNN_ERR_CUDA, "storage options: %zu bytes of shared memory per block of %u", storage, block);
+        if constexpr (kBallThreadDims(DP)) {
+            if (ball_by_thread(DP, ix->n, a, p)) {
+                bool room = false;
+                KNN_TRY(order_room(ix, a.count, s, &room));
+                if (room) KNN_TRY(ball_order_dp<DP>(ix, a, s, &order));
+                if (order) return launch_ball_thread<DP>(ix, a, p, order, s);
+            }
+        }
         // Neighbouring queries share the rows they read through the caches: an order pays where rows are
         // wide (the search then lives on L2 reads; 16 dims, 65,536 queries on 262,144 points: 4.14 ms
         // sorted, 4.39 not) or the index outgrows L2, and costs otherwise (3 dims, 25,000 queries on

@@ -12,8 +12,8 @@
 //   * k-th key cached in a register; tracker/stack storage chosen by the plan.
 //
 // That per-thread search is what the engine runs where the tight node boxes are not to be had (no
-// memory for them when the index was made, nor since).  Otherwise
-// each query gets a warp (kd_warp_query_kernel, warp_search.cuh), bounded by the boxes.
+// memory for them when the index was made, nor since), and for very many queries of very few dims
+// (kd_by_thread; with the boxes as a second bound).  Otherwise each query gets a warp (kd_warp_query_kernel, warp_search.cuh), bounded by the boxes.
 
 #include <algorithm>
 #include <cstring>
@@ -44,8 +44,9 @@ struct KdParams {
     uint32_t order_base;  // subtracted from order entries (batched orders hold batch-wide ids)
     float max_d2;
     const float* radii;
-    const float* box;     // tight node boxes (warp-per-query search), per node lo[], hi[]
+    const float* box;     // tight node boxes, per node lo[], hi[], down to depth box_depth, or null
     uint32_t box_stride;  // floats per box
+    uint32_t box_depth;
     const float* seeds;   // warp-per-query search: per query radius to start from (x seed_scale), or null
     float seed_scale;
     uint32_t k;
@@ -53,6 +54,53 @@ struct KdParams {
     float* out_dist;
     DevCounters* counters;
 };
+
+// Floats per coordinate set of a node box.
+__host__ __device__ constexpr int box_qs(int dp) { return dp < 4 ? 4 : dp; }
+
+// Lower bound on the float dist2 from q to any point of the box (lo, hi): per dimension the gap
+// o = max(fl(lo - q), fl(q - hi), 0), then the same fused sum as dist2 in dimension order.  For a
+// point p of the box, |fl(q - p)| >= o (p lies beyond lo or hi, and rounding is monotone), and
+// fma(t, t, acc) is non-decreasing in |t| and acc >= 0, so the bound never exceeds dist2(q, p).
+// An empty box (lo = +inf, hi = -inf) gives +inf.
+template <int DP>
+__device__ __forceinline__ float box_bound(const float (&q)[DP], const float4* __restrict__ lo4,
+                                           const float4* __restrict__ hi4, float acc) {
+#pragma unroll
+    for (int v = 0; v < (DP + 3) / 4; ++v) {
+        const float4 lo = __ldg(lo4 + v), hi = __ldg(hi4 + v);
+        const float l[4] = {lo.x, lo.y, lo.z, lo.w};
+        const float h[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (4 * v + c < DP) {
+                const float o = fmaxf(fmaxf(__fsub_rn(l[c], q[4 * v + c]), __fsub_rn(q[4 * v + c], h[c])), 0.0f);
+                acc = __fmaf_rn(o, o, acc);
+            }
+        }
+    }
+    return acc;
+}
+
+template <int DP>
+__device__ __forceinline__ float box_bound(const float (&q)[DP], const float* __restrict__ box) {
+    return box_bound<DP>(q, reinterpret_cast<const float4*>(box), reinterpret_cast<const float4*>(box + box_qs(DP)), 0.0f);
+}
+
+// Whether a batch's queries get a thread each, in locality order, instead of a warp each: in very few
+// dims, for few neighbours, where the queries are so many that neighbouring threads walk the same path
+// (a warp's search has some 500 instructions even then).  The sort and the divergence of fewer queries
+// cost more, the more so for queries far from the points.  1,000,000 queries, a warp and a thread each, us:
+// 30,000 1-d points, k 1, 470 and 142; 30,000 2-d points, k 4, 571 and 386; 2,000 3-d points, k 1, 557 and
+// 386; but 1,000,000 2-d points, k 8, 745 and 750, and 400,000 queries far from them, k 1, 414 and 1,492.
+constexpr bool kd_by_thread_dims(int dp) { return dp <= 3; }
+inline bool kd_by_thread(int dp, uint32_t n, const QueryArgs& a, const QueryPlan& p) {
+    if (!kd_by_thread_dims(dp) || !p.reorder || a.order || a.count_dev || a.seeds || a.k > 16) return false;
+    const uint64_t q = a.count;
+    if (dp == 1) return q >= (a.k <= 8 ? 250000u : 500000u);
+    if (dp == 2) return a.k <= 4 && q >= 800000 && q >= 4ull * n;
+    return a.k <= 2 && q >= 1000000 && q >= 128ull * n;
+}
 
 // One thread's search: query slot t of the batch (its query is p.order[t] - p.order_base, or t).
 template <int DP, int KMAX, bool HEAP, bool SHNN, bool SHST>
@@ -85,8 +133,13 @@ __device__ __forceinline__ void kd_search_thread(const KdParams& p, uint32_t t, 
             const uint32_t l = 2 * node + 1;
             const uint32_t close_child = diff < 0.0f ? l : l + 1;
             const uint32_t far_child = diff < 0.0f ? l + 1 : l;
-            const float b = __fmul_rn(diff, diff);
-            if (b <= tr.radius()) overflow |= !st.push(far_child, b);
+            float b = __fmul_rn(diff, diff);
+            if (b <= tr.radius()) {
+                // (The plane alone says little to a query far from the points.)
+                if constexpr (kd_by_thread_dims(DP))
+                    if (depth < p.box_depth) b = fmaxf(b, box_bound<DP>(q, p.box + static_cast<size_t>(far_child) * p.box_stride));
+                if (b <= tr.radius()) overflow |= !st.push(far_child, b);
+            }
             node = close_child;
             ++depth;
             ++lc.nodes;
@@ -256,9 +309,6 @@ inline KdParams kd_params(const knn_index* ix, const QueryArgs& a, const uint32_
     return p;
 }
 
-// Floats per coordinate set of a node box.
-__host__ __device__ constexpr int box_qs(int dp) { return dp < 4 ? 4 : dp; }
-
 // The same for a search over node boxes.
 inline KdParams kd_box_params(const knn_index* ix, const knn_index::KdBoxes& boxes, const QueryArgs& a,
                               const uint32_t* order, uint32_t bucket) {
@@ -266,6 +316,7 @@ inline KdParams kd_box_params(const knn_index* ix, const knn_index::KdBoxes& box
     p.stop_depth = std::min(p.stop_depth, boxes.depth);
     p.box = boxes.buf.as<float>();
     p.box_stride = 2 * box_qs(static_cast<int>(ix->dp));
+    p.box_depth = boxes.depth;
     return p;
 }
 
@@ -277,7 +328,12 @@ static int launch_kd(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, c
     auto kern = plan.warp ? kd_knn_warp_kernel<DP, KMAX, HEAP, SHNN, SHST> : kd_knn_kernel<DP, KMAX, HEAP, SHNN, SHST>;
     if (smem > 48 * 1024)
         KNN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    const KdParams p = kd_params(ix, a, order, plan.leaf_scan);
+    KdParams p = kd_params(ix, a, order, plan.leaf_scan);
+    if (ix->kd_box.buf.ptr) {
+        p.box = ix->kd_box.buf.as<float>();
+        p.box_stride = 2 * box_qs(DP);
+        p.box_depth = ix->kd_box.depth;
+    }
     if (plan.timing) KNN_TRY(ix->timing.begin(s));
     kern<<<ceil_div(a.count, block), block, smem, s>>>(p);
     KNN_LAUNCHED();
@@ -312,8 +368,7 @@ int kd_order_dp(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_
     const uint32_t levels = std::min<uint32_t>(ix->node_depth, std::min<uint32_t>(max_levels, 24));
     if (levels == 0) return KNN_OK;
     const size_t nq = a.count;
-    const size_t need = carve_bytes({nq * 4, nq * 4, nq * 4, nq * 4, radix_sort_temp_bytes(a.count)});
-    KNN_TRY(ix->workspace.reserve(need));
+    KNN_TRY(ix->workspace.reserve(order_bytes(a.count)));
     Carver c(ix->workspace.ptr);
     uint32_t* keys = c.take<uint32_t>(nq);
     uint32_t* vals = c.take<uint32_t>(nq);
@@ -347,6 +402,12 @@ int kd_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStrea
         bool ready = false;
         if (fits || p.box) KNN_TRY(kd_boxes_ready(ix, s, &ready));
         if (ready) {
+            if (kd_by_thread(DP, ix->n, a, p)) {
+                bool room = false;
+                KNN_TRY(order_room(ix, a.count, s, &room));
+                if (room) KNN_TRY(kd_order_dp<DP>(ix, a, s, &order, 24));
+                if (order) return a.k <= 8 ? launch_kd_variant<DP, 8>(ix, a, p, order, s) : launch_kd_variant<DP, 16>(ix, a, p, order, s);
+            }
             // Neighbouring queries share the boxes and slots they read only through the caches: an
             // order pays once the index outgrows L2 (16 M clustered 3-d points, 2 M queries: 3.74 ms
             // sorted, 3.96 unsorted; 40 M and 4 M: 7.59 and 8.48) and costs before (4.19 M and 1 M:
@@ -411,35 +472,6 @@ struct KdGroupParams {
     uint32_t* fb_count;
     uint32_t* group_counter; // next group of 32 queries (zero before the launch)
 };
-
-// Lower bound on the float dist2 from q to any point of the box (lo, hi): per dimension the gap
-// o = max(fl(lo - q), fl(q - hi), 0), then the same fused sum as dist2 in dimension order.  For a
-// point p of the box, |fl(q - p)| >= o (p lies beyond lo or hi, and rounding is monotone), and
-// fma(t, t, acc) is non-decreasing in |t| and acc >= 0, so the bound never exceeds dist2(q, p).
-// An empty box (lo = +inf, hi = -inf) gives +inf.
-template <int DP>
-__device__ __forceinline__ float box_bound(const float (&q)[DP], const float4* __restrict__ lo4,
-                                           const float4* __restrict__ hi4, float acc) {
-#pragma unroll
-    for (int v = 0; v < (DP + 3) / 4; ++v) {
-        const float4 lo = __ldg(lo4 + v), hi = __ldg(hi4 + v);
-        const float l[4] = {lo.x, lo.y, lo.z, lo.w};
-        const float h[4] = {hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (4 * v + c < DP) {
-                const float o = fmaxf(fmaxf(__fsub_rn(l[c], q[4 * v + c]), __fsub_rn(q[4 * v + c], h[c])), 0.0f);
-                acc = __fmaf_rn(o, o, acc);
-            }
-        }
-    }
-    return acc;
-}
-
-template <int DP>
-__device__ __forceinline__ float box_bound(const float (&q)[DP], const float* __restrict__ box) {
-    return box_bound<DP>(q, reinterpret_cast<const float4*>(box), reinterpret_cast<const float4*>(box + box_qs(DP)), 0.0f);
-}
 
 template <int DP, int KMAX>
 __global__ void __launch_bounds__(kGroupWarps * 32) kd_group_kernel(const KdGroupParams gp) {

@@ -51,6 +51,24 @@ inline uint32_t scan_depth_for(uint32_t node_depth, uint32_t leaf_slots, uint32_
     return node_depth - levels;
 }
 
+// Scratch of a batch's locality order (kd_order, ball_order).
+inline size_t order_bytes(uint32_t count) {
+    const size_t nq = count;
+    return carve_bytes({nq * 4, nq * 4, nq * 4, nq * 4, radix_sort_temp_bytes(count)});
+}
+// Whether there is room for it, for a search that can do without: not where the stream is being captured
+// and the workspace would have to grow, nor where no memory is left.
+inline int order_room(knn_index* ix, uint32_t count, cudaStream_t s, bool* room) {
+    *room = ix->workspace.bytes >= order_bytes(count);
+    if (*room) return KNN_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    KNN_TRY_CUDA(cudaStreamIsCapturing(s, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return KNN_OK;
+    const int rc = ix->workspace.reserve(order_bytes(count));
+    *room = rc == KNN_OK;
+    return rc == KNN_ERR_OUT_OF_MEMORY ? KNN_OK : rc;
+}
+
 // Index of the point in a leaf slot, without its coordinates.
 template <int DP>
 __device__ __forceinline__ int32_t slot_id(const float* __restrict__ slot) {
