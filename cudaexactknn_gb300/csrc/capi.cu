@@ -773,6 +773,7 @@ int knn_radius_model_import(knn_index* index, const float* h_params, uint32_t co
     index->has_model = true;
     index->model_k = k;
     index->model_margin = h_params[n - 1];  // the margin is the model's last parameter
+    index->forget_learned_plans();
     return KNN_OK;
 }
 

@@ -391,6 +391,11 @@ struct knn_index {
         float ms = 0.0f;
         uint32_t candidates = 0;
     } tuned[5][2];
+    // A new radius model: plans tuned with the old one (its seeds, how far to widen them, or to leave
+    // them) say nothing about it.
+    void forget_learned_plans() {
+        for (auto& t : tuned) t[1].valid = false;
+    }
 };
 
 namespace knn {
