@@ -709,7 +709,7 @@ int knn_tuned_plan(const knn_index* index, uint32_t k, uint32_t learned_radius, 
     out->shmem_stack = slot.plan.sh_stack;
     out->leaf_scan = slot.plan.leaf_scan;
     out->traversal = slot.plan.group ? 2u : slot.plan.box ? 3u : (slot.plan.warp ? 1u : 0u);
-    out->flags = slot.plan.bf16 ? KNN_QF_BF16_FILTER : 0u;
+    out->flags = slot.plan.bf16 ? KNN_QF_BF16_FILTER : learned_radius && !slot.plan.unseeded ? KNN_QF_LEARNED_RADIUS : 0u;
     out->reserved = slot.candidates;
     if (ms) *ms = slot.ms;
     return KNN_OK;

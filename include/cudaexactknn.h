@@ -277,7 +277,11 @@ KNN_API int knn_last_query_timing(knn_index* index, float* total_ms, float* kern
 
 /* The plan KNN_QF_AUTOTUNE chose for this index and k (block size, tracking, storage, leaf
  * bucket, traversal), with the tuning sample's time in *ms and the number of candidates timed
- * in out->reserved.  Autotuning runs on the first KNN_QF_AUTOTUNE query per k class. */
+ * in out->reserved.  out->flags holds KNN_QF_BF16_FILTER where the filter was chosen, and, of a
+ * learned-radius query's plan, KNN_QF_LEARNED_RADIUS where it starts from the model's seeds (without
+ * it the tuner found them slower than none).  How far the seeds are widened, and how many warps share
+ * a brute-force query's points, are the tuner's own.  Autotuning runs on the first KNN_QF_AUTOTUNE
+ * query per k class; a new radius model starts it anew for learned-radius queries. */
 KNN_API int knn_tuned_plan(const knn_index* index, uint32_t k, uint32_t learned_radius, knn_query_opts* out,
                            float* ms);
 

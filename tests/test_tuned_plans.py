@@ -47,3 +47,20 @@ def test_a_new_model_is_tuned_anew(structure):
     assert _plan(ix, 10, 1) is None and _plan(ix, 10, 0) is not None
     tune()
     ix.close()
+
+
+@pytest.mark.parametrize("structure", ["kd", "ball", "bf"])
+def test_a_plan_says_whether_it_uses_the_seeds(structure):
+    """With seeds that hold nothing, a plan that uses them counts every query as short; one that does not, none."""
+    from cudaexactknn_gb300 import _lib, knn
+    ix, qs, want = _learned_index(structure, 3)
+    params = ix.export_radius_model()
+    params[-1] -= 30
+    ix.import_radius_model(params, 10)
+    learned = _lib.QF_AUTOTUNE | _lib.QF_LEARNED_RADIUS
+    gu.assert_rows_equal(*gu.run(ix, qs, 10, flags=learned), *want)
+    gu.assert_rows_equal(*gu.run(ix, qs, 10, flags=_lib.QF_AUTOTUNE), *want)
+    short = ix.stats(knn.Query(gu.to_dev(qs), len(qs), float("inf")), 10, flags=learned).fallback_queries
+    assert bool(_plan(ix, 10, 1).flags & _lib.QF_LEARNED_RADIUS) == (short > len(qs) // 2)
+    assert not _plan(ix, 10, 0).flags & _lib.QF_LEARNED_RADIUS
+    ix.close()
