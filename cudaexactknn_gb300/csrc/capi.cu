@@ -312,11 +312,13 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
         ++n_tried;
         return KNN_OK;
     };
+    float last_t = 0.0f;  // the last candidate's time
     auto consider = [&](const knn::QueryPlan& p) -> int {
         float v = 0.0f;
         const int r = time_plan(p, &v);
         if (r == KNN_ERR_INVALID_ARGUMENT) return KNN_OK;  // a launch shape that does not fit: skip
         if (r != KNN_OK) return r;
+        last_t = v;
         if (v < best_t) {
             best_t = v;
             best = p;
@@ -363,8 +365,13 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
         }
         if (ix->structure != KNN_BRUTE_FORCE) {
             for (bool warp : {false, true}) {
+                bool far_off = false;
                 for (uint32_t leaf : {0u, 4u, 8u, 16u, 32u, 64u}) {
                     if (leaf && leaf <= ix->leaf_slots) continue;
+                    if (far_off) {  // settled by the traversal's first candidate
+                        ++n_tried;
+                        continue;
+                    }
                     knn::QueryPlan p = best;
                     p.bf16 = false;
                     p.group = p.unseeded = false;
@@ -372,6 +379,10 @@ int autotune(knn_index* ix, const knn::QueryArgs& a, bool learned, cudaStream_t 
                     p.warp = warp;
                     p.leaf_scan = leaf;
                     if ((rc = consider(p)) != KNN_OK) break;
+                    // A bucket size changes a traversal's time a few times over at most.  (The sample is
+                    // sized by the default search; the warp-coherent one can take a hundred times
+                    // as long, and a run of each of its buckets was most of the tuning.)
+                    if (leaf == 0) far_off = last_t > 16.0f * best_t;
                 }
                 if (rc != KNN_OK) break;
             }

@@ -277,7 +277,7 @@ KNN_API int knn_last_query_timing(knn_index* index, float* total_ms, float* kern
 
 /* The plan KNN_QF_AUTOTUNE chose for this index and k (block size, tracking, storage, leaf
  * bucket, traversal), with the tuning sample's time in *ms and the number of candidates timed
- * in out->reserved.  out->flags holds KNN_QF_BF16_FILTER where the filter was chosen, and, of a
+ * (or settled by the time of one like them) in out->reserved.  out->flags holds KNN_QF_BF16_FILTER where the filter was chosen, and, of a
  * learned-radius query's plan, KNN_QF_LEARNED_RADIUS where it starts from the model's seeds (without
  * it the tuner found them slower than none).  How far the seeds are widened, and how many warps share
  * a brute-force query's points, are the tuner's own.  Autotuning runs on the first KNN_QF_AUTOTUNE
