@@ -221,6 +221,7 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
                     knn::QueryArgs at = a;
                     at.count = std::min<uint32_t>(a.count, 8192u);
                     float t_tree = 0.0f, t_tc = tc_per_q * at.count;
+                    bool room = true;
                     if ((rc = time_query([&] { return knn::query_structure(it.index, at, c.plan, s); }, s, &t_tree)) !=
                         KNN_OK)
                         break;
@@ -228,12 +229,16 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
                         knn::QueryPlan tp;
                         tp.bf16 = true;
                         at.count = n;
-                        if ((rc = time_query([&] { return knn::bf_tc_query(it.index, at, tp, s); }, s, &t_tc)) != KNN_OK) break;
-                        if ((rc = time_query([&] { return knn::query_structure(it.index, at, c.plan, s); }, s, &t_tree)) !=
-                            KNN_OK)
-                            break;
+                        rc = time_query([&] { return knn::bf_tc_query(it.index, at, tp, s); }, s, &t_tc);
+                        if (rc == KNN_ERR_OUT_OF_MEMORY) {  // no room for the filter on a batch this size
+                            rc = KNN_OK;
+                            room = false;
+                        } else if (rc == KNN_OK) {
+                            rc = time_query([&] { return knn::query_structure(it.index, at, c.plan, s); }, s, &t_tree);
+                        }
+                        if (rc != KNN_OK) break;
                     }
-                    c.tc = t_tc < t_tree;
+                    c.tc = room && t_tc < t_tree;
                 }
             }
         }
@@ -243,12 +248,16 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
             tp.bf16 = true;
             for (uint32_t i : c.items)
                 if ((rc = knn::bf_tc_query(items[i].index, item_args(items[i]), tp, s)) != KNN_OK) break;
+            if (rc == KNN_ERR_OUT_OF_MEMORY) {  // the trees answer with what they have
+                rc = KNN_OK;
+                c.tc = false;
+            }
             if (rc != KNN_OK) break;
             if (cudaStreamSynchronize(s) != cudaSuccess) {
                 rc = fail(KNN_ERR_CUDA, "stream synchronize");
                 break;
             }
-            continue;
+            if (c.tc) continue;
         }
         if (!c.plan.warp) {
             // A warp per query; k-d trees over each index's node boxes, or the per-thread search where
