@@ -363,9 +363,9 @@ static int launch_kd_variant(knn_index* ix, const QueryArgs& a, const QueryPlan&
 // descent steps (stable radix sort on the path bits).  The order lives in the index workspace
 // until the next query.
 template <uint32_t DP>
-int kd_order_dp(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order, uint32_t max_levels) {
+int kd_order_dp(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order) {
     *order = nullptr;
-    const uint32_t levels = std::min<uint32_t>(ix->node_depth, std::min<uint32_t>(max_levels, 24));
+    const uint32_t levels = std::min<uint32_t>(ix->node_depth, 24);
     if (levels == 0) return KNN_OK;
     const size_t nq = a.count;
     KNN_TRY(ix->workspace.reserve(order_bytes(a.count)));
@@ -405,7 +405,7 @@ int kd_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStrea
             if (kd_by_thread(DP, ix->n, a, p)) {
                 bool room = false;
                 KNN_TRY(order_room(ix, a.count, s, &room));
-                if (room) KNN_TRY(kd_order_dp<DP>(ix, a, s, &order, 24));
+                if (room) KNN_TRY(kd_order_dp<DP>(ix, a, s, &order));
                 if (order) return a.k <= 8 ? launch_kd_variant<DP, 8>(ix, a, p, order, s) : launch_kd_variant<DP, 16>(ix, a, p, order, s);
             }
             // Neighbouring queries share the boxes and slots they read only through the caches: an
@@ -413,11 +413,11 @@ int kd_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStrea
             // sorted, 3.96 unsorted; 40 M and 4 M: 7.59 and 8.48) and costs before (4.19 M and 1 M:
             // 1.92 and 1.83).
             if (!order && p.reorder && a.count >= kWarpOrderMin && ix->leaf.bytes > kL2Bytes)
-                KNN_TRY(kd_order_dp<DP>(ix, a, s, &order, 24));
+                KNN_TRY(kd_order_dp<DP>(ix, a, s, &order));
             return kd_warp_query_dp<DP>(ix, a, p, order, s);
         }
     }
-    if (!order && p.reorder && a.count >= 4096) KNN_TRY(kd_order_dp<DP>(ix, a, s, &order, 24));
+    if (!order && p.reorder && a.count >= 4096) KNN_TRY(kd_order_dp<DP>(ix, a, s, &order));
     if (p.group && !a.count_dev) return kd_group_query_dp<DP>(ix, a, p, order, s);
     switch (k_class(a.k)) {
         case 8: return launch_kd_variant<DP, 8>(ix, a, p, order, s);
@@ -1045,7 +1045,7 @@ int kd_group_query_dp(knn_index* ix, const QueryArgs& a, const QueryPlan& plan, 
 
 template int kd_query_dp<KNN_DP>(knn_index*, const QueryArgs&, const QueryPlan&, cudaStream_t);
 template int kd_box_build_dp<KNN_DP>(const knn_index*, uint32_t, knn_index::KdBoxes*, cudaStream_t);
-template int kd_order_dp<KNN_DP>(knn_index*, const QueryArgs&, cudaStream_t, const uint32_t**, uint32_t);
+template int kd_order_dp<KNN_DP>(knn_index*, const QueryArgs&, cudaStream_t, const uint32_t**);
 
 
 // ---- batches of independent sets (one persistent kernel per class of sets) -----------------------

@@ -464,8 +464,8 @@ int tc_prepare(knn_index* ix, cudaStream_t s);
 int bf_tc_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s);
 int tc_selftest(uint32_t dims, float* max_rel_err, uint32_t* bad);
 // Locality order of a query batch for the trees (kd_order / ball_order), in the index workspace.
-// k-d: queries sorted by the node they reach after min(max_levels, 24, tree depth) descent steps.
-int kd_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order, uint32_t max_levels = 24);
+// k-d: queries sorted by the node they reach after min(24, tree depth) descent steps.
+int kd_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order);
 int ball_order(knn_index* ix, const QueryArgs& a, cudaStream_t s, const uint32_t** order);
 int kd_query(knn_index* ix, const QueryArgs& a, const QueryPlan& p, cudaStream_t s);
 // The k-d node boxes down to subtrees of `bucket` slots (0: the default search's), built if `held` has none.

@@ -67,11 +67,9 @@ struct Tracker {
             mem.emit(k, idx, dist);
     }
 
-    __device__ __forceinline__ void emit_keys(uint32_t k, uint64_t* out) {
-        if constexpr (kReg)
-            reg.emit_keys(k, out);
-        else
-            mem.emit_keys(k, out);
+    __device__ __forceinline__ void emit_keys(uint32_t k, uint64_t* out) const {
+        static_assert(kReg, "keys are written by the register form");
+        reg.emit_keys(k, out);
     }
 };
 

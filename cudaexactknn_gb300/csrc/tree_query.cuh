@@ -69,12 +69,6 @@ inline int order_room(knn_index* ix, uint32_t count, cudaStream_t s, bool* room)
     return rc == KNN_ERR_OUT_OF_MEMORY ? KNN_OK : rc;
 }
 
-// Index of the point in a leaf slot, without its coordinates.
-template <int DP>
-__device__ __forceinline__ int32_t slot_id(const float* __restrict__ slot) {
-    return __float_as_int(slot[DP]);
-}
-
 // Depth-first stack of (node, bound) entries: registers/local memory, or shared memory laid
 // out entry-major (entry e of thread t at e*block + t) so a warp's pushes hit distinct banks.
 template <bool SHARED>

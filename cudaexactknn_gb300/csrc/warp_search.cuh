@@ -73,12 +73,6 @@ __device__ __forceinline__ uint64_t warp_bitonic_merge64(uint64_t v, uint32_t la
     return v;
 }
 
-// The 32 smallest of two ascending 32-key sequences (one key per lane each), ascending.
-__device__ __forceinline__ uint64_t warp_merge_low64(uint64_t a, uint64_t b, uint32_t lane) {
-    const uint64_t rb = shfl64(b, 31 - lane);
-    return warp_bitonic_merge64(a < rb ? a : rb, lane);  // a bitonic sequence holding the 32 smallest
-}
-
 // The k smallest keys seen, ascending over (register, lane): rank r is register r / 32 of lane r % 32.
 // KR = 1 takes k <= 32, 2 k in (32, 64], 4 k in (64, 128].
 template <int KR>
