@@ -70,7 +70,7 @@ __device__ __forceinline__ float centre_dist(const float (&q)[DP], const float* 
 
 // One thread's search: query slot t of the batch (its query is p.order[t] - p.order_base, or t).
 template <int DP, int KMAX>
-__device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t t) {
+__device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t t, uint2* sh_stack) {
     const uint32_t qi = p.order ? p.order[t] - p.order_base : t;
     float q[DP];
     load_query<DP>(p.queries, p.dims, qi, q);
@@ -78,8 +78,7 @@ __device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t
 
     Tracker<KMAX, false, false> tr;
     tr.init(p.k, r2, nullptr, 0);
-    Stack<false> st;
-    st.init(nullptr, 0);
+    LevelStack st{sh_stack + threadIdx.x, blockDim.x, p.stop_depth + 1, 0};
     st.push(0, 0.0f);
     LocalCounters lc;
     bool overflow = false;
@@ -89,9 +88,11 @@ __device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t
         float bound;
         st.pop(&node, &bound);
         if (bound > tr.radius()) continue;
-        bool pruned = false;
         uint32_t depth = heap_depth(node);
-        while (depth < p.stop_depth) {
+        bool within = true;
+        // (One condition and no early exit: with one, the compiler had a warp's threads go on apart for
+        // 1.5 times the instructions.)
+        while (within && depth < p.stop_depth) {
             const uint32_t l = 2 * node + 1;
             float rl, rr;
             const float sl = centre_dist<DP>(q, p.ball + static_cast<size_t>(l) * p.ball_stride, &rl);
@@ -99,36 +100,24 @@ __device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t
             const float bl = ball_bound(sl, rl, p.margin);
             const float br = ball_bound(sr, rr, p.margin);
             ++lc.nodes;
-            // Visit order only (not a bound): the nearer border first.
             const bool left_first = sqrtf(sl) - rl < sqrtf(sr) - rr;
-            const uint32_t close_child = left_first ? l : l + 1;
-            const float close_b = left_first ? bl : br;
-            const float far_b = left_first ? br : bl;
-            if (close_b > tr.radius()) {
-                // The farther ball's bound is at least as large in the common case, but the
-                // order above is approximate, so it is checked on its own.
-                if (far_b <= tr.radius()) {
-                    node = left_first ? l + 1 : l;
-                    ++depth;
-                    continue;
-                }
-                pruned = true;
-                break;
-            }
-            if (far_b <= tr.radius()) overflow |= !st.push(left_first ? l + 1 : l, far_b);
-            node = close_child;
+            const float close_b = left_first ? bl : br, far_b = left_first ? br : bl;
+            const bool close_in = close_b <= tr.radius(), far_in = far_b <= tr.radius();
+            const uint32_t close_child = left_first ? l : l + 1, far_child = left_first ? l + 1 : l;
+            if (close_in && far_in) overflow |= !st.push(far_child, far_b);
+            node = close_in ? close_child : far_child;
+            within = close_in || far_in;
             ++depth;
         }
-        if (pruned) continue;
+        if (!within) continue;
         const SlotRange r = subtree_slots(node, depth, p.node_depth, p.node_count, p.leaf_slots);
         const float* slot = p.leaf + r.first * p.leaf_stride;
         ++lc.leaves;
         for (uint32_t s = 0; s < r.count; ++s, slot += p.leaf_stride) {
             int32_t id;
             const float d2 = slot_dist<DP>(q, slot, &id);
-            if (id < 0) continue;
-            ++lc.points;
-            tr.offer(make_key(d2, id));
+            lc.points += id >= 0 ? 1u : 0u;
+            tr.offer(id >= 0 ? make_key(d2, id) : ~0ull);
         }
     }
     tr.emit(p.k, p.out_idx + static_cast<size_t>(qi) * p.k, p.out_dist + static_cast<size_t>(qi) * p.k);
@@ -140,8 +129,9 @@ __device__ __forceinline__ void ball_search_thread(const BallParams& p, uint32_t
 
 template <int DP, int KMAX>
 __global__ void __launch_bounds__(128) ball_knn_kernel(const BallParams p) {
+    extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < p.nq) ball_search_thread<DP, KMAX>(p, t);
+    if (t < p.nq) ball_search_thread<DP, KMAX>(p, t, reinterpret_cast<uint2*>(smem));
 }
 
 // Warp-coherent variant (see kd_knn_warp_kernel): the warp's queries walk the tree together,
@@ -371,16 +361,18 @@ inline BallParams ball_params(const knn_index* ix, const QueryArgs& a, const uin
 // Whether a batch's queries get a thread each, in locality order, instead of a warp each (kd_by_thread says
 // when that pays; a ball's bound is the same either way, so queries far from the points cost a thread no
 // more than a warp).  1,000,000 queries, a warp and a thread each, us: 30,000 1-d points, k 1, 656 and 186;
-// 30,000 3-d points, k 8, 1,594 and 1,429; 1,000,000 uniform 3-d points, k 1, 1,524 and 979, clustered ones
-// 6,150 and 7,700; on the clustered ones with k 4 7,115 and 11,834, so from k 3 on the line also asks for
-// four queries a point.
+// 20,000 3-d points, k 8, 1,702 and 1,197; 300 4-d points, k 16, 1,527 and 1,617, 600 3-d ones 1,477 and 1,258;
+// 1,000,000 uniform 3-d points, k 1, 1,524 and 970, clustered ones 6,150 and 6,700, with k 4 7,115 and 8,600: from
+// k 3 on the line also asks for many queries a point.
 constexpr bool kBallThreadDims(int dp) { return dp <= 4; }
 inline bool ball_by_thread(int dp, uint32_t n, const QueryArgs& a, const QueryPlan& p) {
     if (!p.reorder || a.order || a.count_dev || a.seeds || a.k > 16) return false;
     const uint64_t q = a.count;
+    if (n <= 64 && a.k <= 4) return q >= 200000;
     if (dp == 1) return q >= (a.k <= 8 ? 250000u : 500000u);
     if (dp <= 3 && a.k <= 2) return q >= 500000;
-    return a.k <= 8 && q >= 1000000 && q >= 4ull * n;
+    if (a.k <= 8) return dp <= 3 ? q >= 400000 && q >= 8ull * n : q >= 1000000 && q >= 8ull * n;
+    return q >= 1000000 && q >= (dp <= 3 ? 32ull : 128ull) * n;
 }
 
 template <int DP>
@@ -388,7 +380,7 @@ int launch_ball_thread(knn_index* ix, const QueryArgs& a, const QueryPlan& plan,
     const BallParams p = ball_params(ix, a, order, plan.leaf_scan);
     auto kern = a.k <= 8 ? ball_knn_kernel<DP, 8> : ball_knn_kernel<DP, 16>;
     if (plan.timing) KNN_TRY(ix->timing.begin(s));
-    kern<<<ceil_div(a.count, 128), 128, 0, s>>>(p);
+    kern<<<ceil_div(a.count, 128), 128, (p.stop_depth + 1) * 128 * sizeof(uint2), s>>>(p);
     KNN_LAUNCHED();
     if (plan.timing) KNN_TRY(ix->timing.end(s));
     return KNN_OK;

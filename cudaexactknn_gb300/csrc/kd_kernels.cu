@@ -93,10 +93,15 @@ __device__ __forceinline__ float box_bound(const float (&q)[DP], const float* __
 // cost more, the more so for queries far from the points.  1,000,000 queries, a warp and a thread each, us:
 // 30,000 1-d points, k 1, 470 and 142; 30,000 2-d points, k 4, 571 and 386; 2,000 3-d points, k 1, 557 and
 // 386; but 1,000,000 2-d points, k 8, 745 and 750, and 400,000 queries far from them, k 1, 414 and 1,492.
+// And on trees so small that a search reads most of them: 200,000 queries, 300 50-d points, k 10, 2,295 and
+// 1,479; 20 3-d points, k 1, 1.5 times a thread's time.
 constexpr bool kd_by_thread_dims(int dp) { return dp <= 3; }
 inline bool kd_by_thread(int dp, uint32_t n, const QueryArgs& a, const QueryPlan& p) {
-    if (!kd_by_thread_dims(dp) || !p.reorder || a.order || a.count_dev || a.seeds || a.k > 16) return false;
+    if (!p.reorder || a.order || a.count_dev || a.seeds || a.k > 16) return false;
     const uint64_t q = a.count;
+    if (n <= 64 && q >= (dp <= 4 && a.k <= 4 ? 200000u : 1000000u)) return true;
+    if (dp >= 32 && n <= 320 && q >= 200000) return true;
+    if (!kd_by_thread_dims(dp)) return false;
     if (dp == 1) return q >= (a.k <= 8 ? 250000u : 500000u);
     if (dp == 2) return a.k <= 4 && q >= 800000 && q >= 4ull * n;
     return a.k <= 2 && q >= 1000000 && q >= 128ull * n;

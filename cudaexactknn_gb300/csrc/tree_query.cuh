@@ -114,6 +114,25 @@ struct Stack {
     }
 };
 
+// The same in shared memory with no more room than the tree has levels (at most 33 KB for 128 threads), so that the
+// blocks of a search without other shared memory still fill an SM.
+struct LevelStack {
+    uint2* at;  // this thread's first entry; the next ones `stride` apart
+    uint32_t stride, levels, top;
+    __device__ __forceinline__ bool push(uint32_t node, float bound) {
+        if (top >= levels) return false;
+        at[top * stride] = make_uint2(node, __float_as_uint(bound));
+        ++top;
+        return true;
+    }
+    __device__ __forceinline__ void pop(uint32_t* node, float* bound) {
+        --top;
+        const uint2 e = at[top * stride];
+        *node = e.x;
+        *bound = __uint_as_float(e.y);
+    }
+};
+
 __host__ __device__ constexpr size_t stack_smem_bytes(bool shared, uint32_t block) {
     return shared ? 2ull * (kMaxTreeDepth + 1) * block * sizeof(uint32_t) : 0;
 }

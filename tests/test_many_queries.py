@@ -29,7 +29,9 @@ def _case(dims, n, count):
     ("kd", 1, 5000, 250000, (1, 8, 9), 0), ("kd", 1, 3, 500000, (9, 16), 0), ("kd", 1, 20000, 500000, (16,), 4),
     ("kd", 2, 3000, 800000, (1, 4, 5), 0), ("kd", 2, 3000, 800000, (4,), 7), ("kd", 3, 900, 1000000, (1, 2, 3), 2),
     ("ball", 1, 5000, 250000, (1, 8, 9), 1), ("ball", 1, 700, 500000, (16,), 3), ("ball", 2, 9000, 500000, (1, 2, 3), 1),
-    ("ball", 3, 9000, 500000, (2,), 5), ("ball", 4, 9000, 1000000, (1, 8, 9), 1), ("ball", 2, 1, 1000000, (8,), 1)])
+    ("ball", 3, 9000, 500000, (2,), 5), ("ball", 4, 9000, 1000000, (1, 8, 9), 1), ("ball", 2, 1, 1000000, (8,), 1),
+    ("kd", 24, 320, 200000, (1, 16, 17), 0), ("kd", 100, 320, 200000, (5,), 3), ("kd", 4, 64, 200000, (4, 5), 1), ("kd", 12, 64, 1000000, (16,), 0),
+    ("ball", 3, 64, 200000, (4, 5), 1), ("ball", 4, 1024, 1000000, (16,), 2)])
 def test_rows(structure, dims, n, count, ks, skips):
     pts, qs, rows = _case(dims, n, count)
     dq = gu.to_dev(qs)
