@@ -533,6 +533,8 @@ def measure(D, w, key, steps, warmup, plain_steps, world, rank, cpu=True):
     prof = profile_summary(kernel_name, key)
     roofline = {"bound": roof_bound, "achieved": achieved, "peak": peak, "unit": roof_unit, "frac": achieved / peak,
                 "traffic": prof.get("dram_bytes_per_launch"),
+                # (Bytes of every visit, most of them served by L1 and L2: the tree searches are bound by
+                # instruction issue, see traffic and l2_gbs.)
                 "peak_source": f"{peak_kind} " + ("bf16_tflops" if roof_bound == "tensor" else "hbm_gbs"),
                 "kernel": kernel_name, "kernel_ms": kernel_ms,
                 "kernel_span": "sum of the CUDA-event spans of every search kernel of the pass "
@@ -585,7 +587,7 @@ def measure(D, w, key, steps, warmup, plain_steps, world, rank, cpu=True):
 def measure_c5(D, scale, steps, warmup, plain_steps, world, rank, cpu=True):
     """Uneven batch: 64 independent sets in one CUDA-graph launch against one plain batchKnn per
     set (each ending in a device synchronisation, as the reference's does), both over every
-    query of every set.  The plain form takes ~35 s per step (its 32-dimensional ball trees visit
+    query of every set.  The plain form takes ~8 s per step (its 32-dimensional ball trees visit
     most of their nodes), so it is timed over `plain_steps` steps after a warm-up on 64 queries
     per set."""
     import torch

@@ -183,8 +183,8 @@ int batch_create(const knn_batch_item* items, uint32_t count, uint32_t flags, vo
     }
     int rc = KNN_OK;
     for (auto& c : b->classes) {
-        // Plan: the autotuned plan of the class's largest set, or per-thread search with the
-        // tree's own leaves.
+        // Plan: the autotuned plan of the class's largest set, or a warp per query with the engine's own
+        // bucket sizes.
         uint32_t largest = c.items[0];
         for (uint32_t i : c.items)
             if (items[i].count > items[largest].count) largest = i;

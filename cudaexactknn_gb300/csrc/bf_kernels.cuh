@@ -7,8 +7,9 @@
 // queries and its lanes take 32 points at a time:
 //   * every pair's distance is the reference's sequential fused sum, two queries per packed
 //     instruction (sub/fma.rn.f32x2 round each half as the scalar instructions do);
-//   * a first look at every kBfSample-th step of 32 points keeps only the least distance per lane
-//     (and, for k > 32, per turn of KR); the k-th smallest of those is the distance of a point with
+//   * a first look at every eighth tile of points (every fourth below 32 tiles, all of them below 8)
+//     keeps only the least distance per lane (and, for k > 32, per turn of KR); the k-th smallest of
+//     those is the distance of a point with
 //     k - 1 others at or below it, an upper bound on the query's k-th distance.  The scan proper
 //     then appends the few points within the bound to a buffer, and only a full buffer (or the end)
 //     is sorted into the k smallest keys.  A list per thread, as
@@ -20,11 +21,11 @@
 //     the bound and merge their lists in shared memory) and over blocks (merged by a second kernel).
 // Keys, ties and results equal the reference's brute force bit for bit.
 //
-// Measured (before: 2-chain loop per thread, list in registers or local memory): 65,536 3-d points,
-// 4,096 queries, k 8: 255 us (455; 1,335 with heap tracking); 4,096 points, 16 queries: 41 us with its
-// launches (200, one block); 128 dims, 2,048 queries on 100,000 points, k 10: 2.3 ms (2.7), 256 queries
-// on 262,144, k 100: 1.64 ms (46.6).  Bound by issue at 3.4 warps per scheduler (registers), at 60% the
-// scan, the rest first look, appends and merges.
+// Measured (before: a thread per query at all sizes, list in registers or local memory): 65,536 3-d points,
+// 4,096 queries, k 8: 268 us (455; 1,335 with heap tracking); 4,096 points, 16 queries: 46 us with its
+// launches (200, one block); 128 dims, 256 queries on 262,144 points, k 100: 1.64 ms (46.6).  At the first
+// of these 54% of the issue slots are used, with 5 warps per scheduler; the largest stall is the barrier
+// between staged tiles.
 #pragma once
 
 #include <algorithm>
@@ -54,7 +55,7 @@ struct BfParams {
 };
 
 constexpr uint32_t kBfWarps = 8;   // warps per block
-constexpr uint32_t kBfSample = 8;  // every how many steps (tiles) the first look takes
+constexpr uint32_t kBfSample = 8;  // every how many tiles the first look takes one, of many
 
 // Queries per warp, by top-k registers.
 __host__ __device__ constexpr uint32_t bf_queries(int kr) { return kr == 1 ? 8u : kr == 2 ? 4u : 2u; }

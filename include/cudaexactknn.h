@@ -78,8 +78,8 @@ typedef enum knn_structure {
 /* Query flags. */
 #define KNN_QF_SYNC 1u           /* synchronise the stream before returning */
 #define KNN_QF_AUTOTUNE 2u       /* engine picks block size, tracking, storage and leaf size */
-#define KNN_QF_LEARNED_RADIUS 4u /* seed each query's radius from the trained model; queries
-                                    with fewer than k hits are re-run unbounded */
+#define KNN_QF_LEARNED_RADIUS 4u /* seed each query's radius from the trained model; a query with
+                                    fewer than k hits goes on within the caller's radius */
 #define KNN_QF_BF16_FILTER 8u    /* any index, dims >= 16: 16-bit (FP16, or BF16 for values beyond
                                     FP16's range) tcgen05 filter with rigorous bounds + exact FP32
                                     rescore; the same answer as the plain search */
@@ -99,7 +99,9 @@ typedef enum knn_structure {
  * Run-time form of batchKnn's template arguments (src/KdTreeGpu.cuh:392,
  * src/BruteForceGpu.cuh:74): BLOCK_SIZE, USE_HEAP_TRACKING, USE_TRACKING_SHMEM,
  * USE_STACK_SHMEM.  A zeroed struct (or NULL) means block 0 = engine default, sorted
- * insertion tracking in registers, stack in registers.
+ * insertion tracking in registers, stack in registers.  Brute force and the trees' default search
+ * keep their top-k and stack where they are fastest and take these four as checked (sizes no block
+ * can hold are refused) but unused.
  */
 typedef struct knn_query_opts {
     uint32_t block_size;
@@ -115,7 +117,8 @@ typedef struct knn_query_opts {
                                boxes that come with the tree (a thread per query, bounded by the
                                splitting planes, where there is no memory for them; the storage
                                options above apply to that search and to traversal 1), ball trees
-                               always, over their balls;
+                               over their balls; for very many queries of very few dims (or on very
+                               few points) and small k either takes a thread per query;
                                1 = warp-coherent search (a warp's queries walk together);
                                k-d trees of at most 16 dims, k <= 32: 2 = warp-group search (a
                                warp's 32 queries walk the tree once against the node boxes from
