@@ -38,6 +38,7 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
     const char* base = std::strrchr(file, '/');
     std::snprintf(g_last_error, sizeof(g_last_error), "%s: %s (%s:%d)", cudaGetErrorString(e), what,
                   base ? base + 1 : file, line);
+    cudaGetLastError();  // (reported here; left standing, the next call's launch check would report it again)
     return e == cudaErrorMemoryAllocation ? KNN_ERR_OUT_OF_MEMORY : KNN_ERR_CUDA;
 }
 
