@@ -526,8 +526,10 @@ int run_query(knn_index* ix, const knn::QueryArgs& a, const knn_query_opts* opts
     const knn::Range range("knn query");
     return knn::no_throw([&] {
         if (ix) KNN_TRY(ix->order_guard.before(s));
-        KNN_TRY(run_query_checked(ix, a, opts, s));
-        return ix ? ix->order_guard.after(s) : KNN_OK;
+        const int rc = run_query_checked(ix, a, opts, s);
+        // (A query that failed may have enqueued work on the index's scratch all the same.)
+        const int after = ix ? ix->order_guard.after(s) : KNN_OK;
+        return rc != KNN_OK ? rc : after;
     });
 }
 
